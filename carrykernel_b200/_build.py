@@ -22,6 +22,9 @@ LIB = os.path.join(PKG, "libcarry_gdn.so")
 # forces, reports and (with an extra kernel that writes a buffer late) provokes the path of set-up inputs
 # that changed under the streaming kernel's feet.  Nothing in the package loads it.
 WAIT_TEST_LIB = os.path.join(PKG, "libcarry_gdn_waittest.so")
+# Native call path of the Python surfaces (CPython extension over torch's C++ tensors; no device code)
+NATIVE = os.path.join(PKG, "_native.so")
+NATIVE_SOURCE = "host_native.cpp"
 SOURCES = ("carry_gdn_api.cu", "carry_gdn_generic.cu", "carry_gdn_tile128.cu",
            "carry_gdn_tile128_vk.cu", "carry_gdn_tile128_kv.cu", "carry_gdn_multi.cu",
            "carry_gdn_pool.cu", "carry_gdn_noef128.cu")
@@ -37,16 +40,31 @@ def _nvcc() -> str:
     raise RuntimeError("nvcc not found (set NVCC or put it on PATH)")
 
 
+def _native_command(out: str):
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    cxx = os.environ.get("CXX") or shutil.which("g++") or "g++"
+    includes = [*cpp_extension.include_paths(device_type="cuda"), sysconfig.get_paths()["include"]]
+    libdir = os.path.join(os.path.dirname(torch.__file__), "lib")
+    return [cxx, "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            *(f"-isystem{d}" for d in includes), NATIVE_SOURCE, "-o", out, f"-L{libdir}",
+            "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10"]
+
+
 def is_stale() -> bool:
-    if not os.path.exists(LIB) or not os.path.exists(WAIT_TEST_LIB):
+    products = (LIB, WAIT_TEST_LIB, NATIVE)
+    if not all(os.path.exists(p) for p in products):
         return True
-    built = min(os.path.getmtime(LIB), os.path.getmtime(WAIT_TEST_LIB))
-    deps = [os.path.join(CSRC, s) for s in SOURCES + HEADERS]
+    built = min(os.path.getmtime(p) for p in products)
+    deps = [os.path.join(CSRC, s) for s in (*SOURCES, NATIVE_SOURCE, *HEADERS)]
     return any(os.path.getmtime(d) > built for d in deps if os.path.exists(d))
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile the library if it is missing or older than its sources.
+    """Compile the library and the native call path if one is missing or older than its sources.
     Returns the path of the shared object; raises on compiler failure.  The
     ptxas resource report (registers, spills) goes to ``build/ptxas.log``."""
     if not force and not is_stale():
@@ -61,12 +79,15 @@ def build(force: bool = False, verbose: bool = False) -> str:
 
     def compile_one(job):
         src, twin = job
+        if src == NATIVE_SOURCE:
+            cmd = _native_command(NATIVE)
+            return NATIVE, cmd, subprocess.run(cmd, cwd=CSRC, capture_output=True, text=True)
         obj = os.path.join(obj_dir, src.replace(".cu", ".waittest.o" if twin else ".o"))
         cmd = [nvcc, *NVCC_FLAGS, *(("-DCARRY_TEST_WAIT_EXPIRY",) if twin else ()), "-c", "-o", obj, src]
         proc = subprocess.run(cmd, cwd=CSRC, capture_output=True, text=True)
         return obj, cmd, proc
 
-    jobs = [(s, False) for s in SOURCES] + [(s, True) for s in twin_sources]
+    jobs = [(s, False) for s in (*SOURCES, NATIVE_SOURCE)] + [(s, True) for s in twin_sources]
     with ThreadPoolExecutor(max_workers=len(jobs)) as pool:
         results = list(pool.map(compile_one, jobs))
     log = []

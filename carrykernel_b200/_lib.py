@@ -115,12 +115,23 @@ class PoolCopyArgs(C.Structure):
     ]
 
 
+class PoolCopyLayersArgs(C.Structure):
+    _fields_ = [
+        ("src", C.POINTER(Pool)), ("dst", C.POINTER(Pool)), ("layers", C.c_int32),
+        ("src_slot", C.c_int32), ("dst_slot", C.c_int32),
+    ]
+
+
 ERR_UNSUPPORTED = -5
 
 EXPORTS = ("carry_gdn_quant_step", "carry_gdn_fp32_step", "carry_gdn_packed_decode",
            "carry_gdn_packed_decode_multi", "carry_gdn_pool_store", "carry_gdn_pool_load",
-           "carry_gdn_pool_copy", "carry_gdn_strerror", "carry_gdn_abi_version",
-           "carry_gdn_last_kernel")
+           "carry_gdn_pool_copy", "carry_gdn_pool_copy_layers", "carry_gdn_write_ids", "carry_gdn_strerror",
+           "carry_gdn_abi_version", "carry_gdn_last_kernel")
+# what the native call path is given the addresses of, in the order it expects them (csrc/host_native.cpp, Table)
+_NATIVE_ENTRIES = ("carry_gdn_quant_step", "carry_gdn_fp32_step", "carry_gdn_packed_decode",
+                   "carry_gdn_packed_decode_multi", "carry_gdn_pool_store", "carry_gdn_pool_load",
+                   "carry_gdn_pool_copy", "carry_gdn_pool_copy_layers", "carry_gdn_write_ids")
 
 _lib = None
 _lock = threading.Lock()
@@ -156,13 +167,24 @@ def load_library(path: str | None = None):
         lib.carry_gdn_pool_store.argtypes = [C.POINTER(PoolStoreArgs), C.c_void_p]
         lib.carry_gdn_pool_load.argtypes = [C.POINTER(PoolLoadArgs), C.c_void_p]
         lib.carry_gdn_pool_copy.argtypes = [C.POINTER(PoolCopyArgs), C.c_void_p]
+        lib.carry_gdn_pool_copy_layers.argtypes = [C.POINTER(PoolCopyLayersArgs), C.c_void_p]
+        lib.carry_gdn_write_ids.argtypes = [C.c_void_p, C.c_void_p, C.c_int32, C.c_void_p]
         for fn in (lib.carry_gdn_quant_step, lib.carry_gdn_fp32_step, lib.carry_gdn_packed_decode,
                    lib.carry_gdn_packed_decode_multi, lib.carry_gdn_pool_store, lib.carry_gdn_pool_load,
-                   lib.carry_gdn_pool_copy):
+                   lib.carry_gdn_pool_copy, lib.carry_gdn_pool_copy_layers, lib.carry_gdn_write_ids):
             fn.restype = C.c_int
         if lib.carry_gdn_abi_version() != ABI_VERSION:
             raise CudaUnavailable(
                 f"ABI mismatch: library {lib.carry_gdn_abi_version()}, binding {ABI_VERSION}")
+        try:
+            from . import _native
+        except ImportError as exc:
+            raise CudaUnavailable(
+                f"the native call path is missing or cannot be loaded ({exc}): "
+                "build it with `python -m carrykernel_b200._build`") from exc
+        lib.native_table = _native.make_table(
+            *(C.cast(getattr(lib, name), C.c_void_p).value for name in _NATIVE_ENTRIES))
+        lib.native = _native
         _lib = lib
         return _lib
 

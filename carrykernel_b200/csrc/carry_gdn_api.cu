@@ -2,6 +2,8 @@
 // include/carry_gdn.h for the contract of every entry point.
 #include "carry_gdn_common.cuh"
 
+#include <initializer_list>
+
 namespace {
 
 thread_local int g_last_kernel = 0;
@@ -236,6 +238,36 @@ int carry_gdn_pool_copy(const CarryGdnPoolCopyArgs* a, void* stream) {
   const int rc2 = carry::launch_pool_copy(*a, static_cast<cudaStream_t>(stream));
   if (rc2 == CARRY_GDN_OK) g_last_kernel = 4;
   return rc2;
+}
+
+int carry_gdn_pool_copy_layers(const CarryGdnPoolCopyLayersArgs* a, void* stream) {
+  clear_stale_error();
+  if (!a || !a->src || !a->dst) return CARRY_GDN_ERR_NULL;
+  if (a->layers < 1) return CARRY_GDN_ERR_SHAPE;
+  for (int l = 0; l < a->layers; ++l) {
+    const CarryGdnPool &s = a->src[l], &d = a->dst[l], &r = a->src[0];
+    int rc = pool_ok(s);
+    if (rc == CARRY_GDN_OK) rc = pool_ok(d);
+    if (rc != CARRY_GDN_OK) return rc;
+    for (const CarryGdnPool* p : {&s, &d}) {
+      if (p->HV != r.HV || p->K != r.K || p->V != r.V) return CARRY_GDN_ERR_SHAPE;
+      if (p->res_fmt != r.res_fmt || p->resid_scale_mode != r.resid_scale_mode) return CARRY_GDN_ERR_FORMAT;
+      if (!pool_has_pointers(*p)) return CARRY_GDN_ERR_NULL;
+    }
+    if (a->src_slot <= 0 || a->src_slot >= s.num_slots || a->dst_slot <= 0 || a->dst_slot >= d.num_slots)
+      return CARRY_GDN_ERR_SHAPE;
+  }
+  const int rc = carry::launch_pool_copy_layers(*a, static_cast<cudaStream_t>(stream));
+  if (rc == CARRY_GDN_OK) g_last_kernel = 4;
+  return rc;
+}
+
+int carry_gdn_write_ids(int32_t* dst, const int32_t* ids, int32_t n, void* stream) {
+  clear_stale_error();
+  if (n < 0) return CARRY_GDN_ERR_SHAPE;
+  if (n == 0) return CARRY_GDN_OK;
+  if (!dst || !ids) return CARRY_GDN_ERR_NULL;
+  return carry::launch_write_ids(dst, ids, n, static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

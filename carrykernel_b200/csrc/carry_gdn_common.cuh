@@ -181,6 +181,30 @@ __device__ __forceinline__ Tile resolve_tile(const KParams& p, int n, int hv) {
   return t;
 }
 
+// Programmatic dependent launch.  A kernel launched through launch_dependent() may start while the kernel ahead of
+// it in the stream runs out; it calls depend_wait() before it touches global memory (everything earlier has
+// completed and is visible after that) and lets its own successor move in with depend_release().  For calls that
+// follow one another on small batches this takes the launch gap between two kernels from 1.5 us to about half.
+__device__ __forceinline__ void depend_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void depend_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... P, class... A>
+int launch_dependent(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, kern, args...) == cudaSuccess) return CARRY_GDN_OK;
+  cudaGetLastError();
+  return CARRY_GDN_ERR_LAUNCH;
+}
+
 // kernels / launchers implemented in the other translation units
 int launch_generic(const KParams& p, cudaStream_t stream);
 int launch_fp32(const CarryGdnFp32Args& a, cudaStream_t stream);
@@ -193,5 +217,7 @@ int launch_noef128(const KParams& p, cudaStream_t stream);
 int launch_pool_store(const CarryGdnPoolStoreArgs& a, cudaStream_t stream);
 int launch_pool_load(const CarryGdnPoolLoadArgs& a, cudaStream_t stream);
 int launch_pool_copy(const CarryGdnPoolCopyArgs& a, cudaStream_t stream);
+int launch_pool_copy_layers(const CarryGdnPoolCopyLayersArgs& a, cudaStream_t stream);
+int launch_write_ids(int32_t* dst, const int32_t* ids, int n, cudaStream_t stream);
 
 }  // namespace carry

@@ -598,6 +598,40 @@ __global__ void __launch_bounds__(kThreads) pool_copy_kernel(CarryGdnPoolCopyArg
   }
 }
 
+// One slot of up to kMoveLayers layers, by address.  A slot's four tensors are four contiguous runs per layer; the
+// grid cuts them into pieces of kPiece bytes (4 reads of 16 bytes in flight per thread), so that a single
+// slot keeps the machine busy: 12 layers of 32 heads, int4 residual, are 600 pieces.  A cache move was one launch
+// of 32 CTAs per layer before, with two host-to-device copies for the ids.
+constexpr int kMoveLayers = 48;
+constexpr int kPiece = kThreads * 64;
+struct MoveTable {
+  void* dst[kMoveLayers][4];
+  const void* src[kMoveLayers][4];
+  long long bytes[4];
+  int pieces[4];         // per run, rounded up
+};
+static_assert(sizeof(MoveTable) <= 4000, "kernel arguments");
+__global__ void __launch_bounds__(kThreads) pool_copy_layers_kernel(const __grid_constant__ MoveTable m) {
+  depend_release();
+  int piece = (int)blockIdx.x, run = 0;
+  while (run < 3 && piece >= m.pieces[run]) piece -= m.pieces[run++];
+  const long long off = (long long)piece * kPiece, left = m.bytes[run] - off;
+  depend_wait();
+  copy_bytes(static_cast<uint8_t*>(m.dst[blockIdx.y][run]) + off, static_cast<const uint8_t*>(m.src[blockIdx.y][run]) + off,
+             left < kPiece ? left : kPiece);
+}
+
+// slot ids from kernel arguments to device memory
+constexpr int kIdsPerLaunch = 960;
+struct IdBlock {
+  int32_t v[kIdsPerLaunch];
+};
+__global__ void __launch_bounds__(kThreads) write_ids_kernel(int32_t* dst, int n, const __grid_constant__ IdBlock ids) {
+  depend_release();
+  depend_wait();
+  for (int i = threadIdx.x; i < n; i += kThreads) dst[i] = ids.v[i];
+}
+
 int grid_for(long long tiles) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -652,6 +686,43 @@ int launch_pool_copy(const CarryGdnPoolCopyArgs& a, cudaStream_t stream) {
   const int grid = grid_for((long long)a.B * a.src.HV);
   pool_copy_kernel<<<grid, kThreads, 0, stream>>>(a);
   return finish_launch();
+}
+
+int launch_pool_copy_layers(const CarryGdnPoolCopyLayersArgs& a, cudaStream_t stream) {
+  const CarryGdnPool& r = a.src[0];
+  const long long VK = (long long)r.V * r.K, HV = r.HV;
+  for (int l0 = 0; l0 < a.layers; l0 += kMoveLayers) {
+    const int layers = a.layers - l0 < kMoveLayers ? a.layers - l0 : kMoveLayers;
+    MoveTable m = {};
+    m.bytes[0] = HV * VK;
+    m.bytes[1] = r.res_fmt == CARRY_RES_INT4 ? HV * VK / 2 : HV * VK;
+    m.bytes[2] = HV * r.V * 4;
+    m.bytes[3] = r.resid_scale_mode == CARRY_SCALE_PER_HEAD ? HV * 4 : HV * r.V * 4;
+    long long pieces = 0;
+    for (int i = 0; i < 4; ++i) pieces += m.pieces[i] = (int)((m.bytes[i] + kPiece - 1) / kPiece);
+    for (int l = 0; l < layers; ++l) {
+      const CarryGdnPool &s = a.src[l0 + l], &d = a.dst[l0 + l];
+      const long long from = a.src_slot, to = a.dst_slot;
+      m.src[l][0] = s.state_codes + from * s.stride_state_slot; m.dst[l][0] = d.state_codes + to * d.stride_state_slot;
+      m.src[l][1] = s.resid_codes + from * s.stride_resid_slot; m.dst[l][1] = d.resid_codes + to * d.stride_resid_slot;
+      m.src[l][2] = s.state_scale + from * s.stride_sscale_slot; m.dst[l][2] = d.state_scale + to * d.stride_sscale_slot;
+      m.src[l][3] = s.resid_scale + from * s.stride_rscale_slot; m.dst[l][3] = d.resid_scale + to * d.stride_rscale_slot;
+    }
+    const int rc = launch_dependent(pool_copy_layers_kernel, dim3((unsigned)pieces, (unsigned)layers), kThreads, 0, stream, m);
+    if (rc != CARRY_GDN_OK) return rc;
+  }
+  return CARRY_GDN_OK;
+}
+
+int launch_write_ids(int32_t* dst, const int32_t* ids, int n, cudaStream_t stream) {
+  for (int i = 0; i < n; i += kIdsPerLaunch) {
+    const int m = n - i < kIdsPerLaunch ? n - i : kIdsPerLaunch;
+    IdBlock b;
+    for (int j = 0; j < m; ++j) b.v[j] = ids[i + j];
+    const int rc = launch_dependent(write_ids_kernel, dim3(1), kThreads, 0, stream, dst + i, m, b);
+    if (rc != CARRY_GDN_OK) return rc;
+  }
+  return CARRY_GDN_OK;
 }
 
 }  // namespace carry

@@ -189,6 +189,13 @@ def gdn_quant_step_fused(h_int8, scale, e, e_scale, q, k, v, alpha, beta,
     ``None`` unless the residual is int8/int4.  ``BLOCK_V`` is accepted for
     signature compatibility and ignored.
     """
+    lib = _lib._lib or _lib.load_library()
+    if resid_scale in _SCALE_MODE and state_scale in _SCALE_MODE:
+        made = lib.native.quant_step(lib.native_table, h_int8, scale, e, e_scale, q, k, v, alpha, beta, bits, res_fmt,
+                                     resid_scale == "v", state_scale == "v")
+        if made is not None:
+            return made
+    # something to convert, or to refuse
     assert h_int8.dtype == torch.int8, f"h_int8 must be int8, got {h_int8.dtype}"
     assert h_int8.dim() == 4, f"expected [B, HV, K, V], got {tuple(h_int8.shape)}"
     _scale_mode(resid_scale), _scale_mode(state_scale)
@@ -239,6 +246,10 @@ def gdn_quant_step_fused(h_int8, scale, e, e_scale, q, k, v, alpha, beta,
 
 def gdn_step_fused_fp32(h, q, k, v, alpha, beta, BLOCK_V: int = 32):
     """Fused fp32 GDN step (no quantisation).  Returns ``(h_out, o)``."""
+    lib = _lib._lib or _lib.load_library()
+    made = lib.native.fp32_step(lib.native_table, h, q, k, v, alpha, beta)
+    if made is not None:
+        return made
     assert h.dim() == 4, f"expected [B, HV, K, V], got {tuple(h.shape)}"
     B, HV, K, V = h.shape
     dev = h.device
@@ -262,7 +273,6 @@ def gdn_step_fused_fp32(h, q, k, v, alpha, beta, BLOCK_V: int = 32):
     a.alpha, a.beta, a.o, a.h_out = alpha.data_ptr(), beta.data_ptr(), o.data_ptr(), h_out.data_ptr()
     a.B, a.HV, a.K, a.V = B, HV, K, V
     a.qkv_dtype, a.o_dtype = _lib.dtype_id(q), _lib.F32
-    lib = _lib.load_library()
     with torch.cuda.device(dev):
         rc = lib.carry_gdn_fp32_step(a, _lib.current_stream_ptr(dev))
     _lib.check(rc, "carry_gdn_fp32_step")
@@ -276,6 +286,12 @@ def gdn_quant_decode_fused(h0, q, k, v, alpha, beta, T, bits: int = 8,
     ``v [T, B, HV, V]``, ``alpha/beta [T, B, HV]``.  Returns
     ``(o [T, B, HV, V], h_int8, scale, e, e_scale)``."""
     h_int8, scale, e, e_scale = init_quant_state(h0, bits, res_fmt, resid_scale, state_scale)
+    lib = _lib._lib or _lib.load_library()
+    # the state is this call's own: all steps in place, launched back to back
+    o = lib.native.quant_decode(lib.native_table, h_int8, scale, e, e_scale, q, k, v, alpha, beta, T, bits, res_fmt,
+                                resid_scale == "v", state_scale == "v")
+    if o is not None:
+        return o, h_int8, scale, e, e_scale
     outs = []
     for t in range(T):
         o, h_int8, scale, e, e_scale = gdn_quant_step_fused(

@@ -179,10 +179,15 @@ def quantized_gated_delta_rule_packed_decode(
     kernel ORs its status bits into -- a slot id beyond the pool (that request is treated as padding:
     zeros to ``out``, pool untouched) or a wait that ran out.  Without it such a request is silently a
     padding request.  See ``_lib.raise_for_status``."""
+    lib = _lib._lib or _lib.load_library()
+    if lib.native.packed_decode(lib.native_table, False, mixed_qkv, a, b, A_log, dt_bias, scale, state_codes,
+                                state_scale, resid_codes, resid_scale, out, ssm_state_indices,
+                                use_qk_l2norm_in_kernel, resid_fmt, status):
+        return out
+    # not a call the native path takes as it stands: the checks below say what is wrong with it, if anything
     args, _keep = _packed_args(mixed_qkv, a, b, A_log, dt_bias, scale, state_codes, state_scale, resid_codes,
                                resid_scale, out, lambda B, HV, V: (B, 1, HV, V), ssm_state_indices,
                                use_qk_l2norm_in_kernel, resid_fmt, status)
-    lib = _lib.load_library()
     dev = state_codes.device
     with torch.cuda.device(dev):
         rc = lib.carry_gdn_packed_decode(args, _lib.current_stream_ptr(dev))
@@ -217,6 +222,11 @@ def quantized_gated_delta_rule_packed_decode_multi(
     speculative-decoding path.)  Shapes the streaming kernels do not take (K or V other than
     128, ...) fall back to one single-token call per token, which allocates a ``[B, 1, HV, V]``
     scratch block: that path is not CUDA-graph capturable.  ``status`` as in the single-token call."""
+    lib = _lib._lib or _lib.load_library()
+    if lib.native.packed_decode(lib.native_table, True, mixed_qkv, a, b, A_log, dt_bias, scale, state_codes,
+                                state_scale, resid_codes, resid_scale, out, ssm_state_indices,
+                                use_qk_l2norm_in_kernel, resid_fmt, status):
+        return out
     if mixed_qkv.dim() != 3 or a.dim() != 3 or b.dim() != 3:
         raise ValueError("mixed_qkv, a and b must be 3-D: [B, T, ...]")
     B, T = mixed_qkv.shape[0], mixed_qkv.shape[1]
@@ -229,7 +239,6 @@ def quantized_gated_delta_rule_packed_decode_multi(
     args.step = step
     args.T = T
     args.stride_mixed_t, args.stride_a_t, args.stride_b_t = mixed_qkv.stride(1), a.stride(1), b.stride(1)
-    lib = _lib.load_library()
     dev = state_codes.device
     with torch.cuda.device(dev):
         rc = lib.carry_gdn_packed_decode_multi(args, _lib.current_stream_ptr(dev))

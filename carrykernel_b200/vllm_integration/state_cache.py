@@ -23,9 +23,9 @@ an engine that drives the decode calls itself:
   :meth:`rollback` when some are rejected, :meth:`release_checkpoint` when all
   are accepted.
 
-Every move is ``state_pool.copy_slots`` -- one launch per layer, all four
-tensors of the slot bit for bit, on the current stream, nothing allocated and
-nothing read back -- so an interrupted request ends with exactly the pool
+Every move copies all four tensors of the slot bit for bit in every layer --
+one launch for the whole stack of layers, on the current stream, nothing
+allocated and nothing read back -- so an interrupted request ends with exactly the pool
 contents of an uninterrupted one.  The bookkeeping is host-side Python, the
 engine's scheduler thread being its only caller (no locking).  Registration
 with vLLM's own cache manager (``MambaSpec``) is engine code and not part of
@@ -38,6 +38,7 @@ from typing import Dict, Hashable, Iterable, List, Optional
 
 import torch
 
+from .. import _lib
 from . import quantized_packed_decode as qpd
 from . import state_pool
 
@@ -154,10 +155,20 @@ class SlotCache:
             if pad_to < len(ids):
                 raise ValueError("pad_to is shorter than the batch")
             ids += [NULL_SLOT] * (pad_to - len(ids))
+        if self.device.type == "cuda" and ids:
+            lib = _lib._lib or _lib.load_library()
+            # as kernel arguments: a copy from pageable memory would wait for everything ahead in the stream
+            made = lib.native.ids_tensor(lib.native_table, ids, self.pools[0][0].get_device())
+            if made is not None:
+                return made
         return torch.tensor(ids, dtype=torch.int32, device=self.device)
 
     # ---- moves ------------------------------------------------------------
     def _copy(self, src: _Pools, src_slot: int, dst: _Pools, dst_slot: int) -> None:
+        if self.device.type == "cuda":
+            lib = _lib._lib or _lib.load_library()
+            if lib.native.pool_copy_layers(lib.native_table, src.layers, src_slot, dst.layers, dst_slot, self.resid_fmt):
+                return
         s = torch.tensor([src_slot], dtype=torch.int32, device=self.device)
         d = torch.tensor([dst_slot], dtype=torch.int32, device=self.device)
         for sp, dp in zip(src.layers, dst.layers):

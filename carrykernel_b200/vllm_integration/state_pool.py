@@ -104,6 +104,9 @@ def _state_tensor(h, B, HV, V, K, device, name):
 def store_state(h, pool, ssm_state_indices, resid_fmt: int = RESID_INT8, keep_error: bool = False, status=None):
     """Quantise ``h [B, HV, V, K]`` (fp32, bf16 or fp16) into slots
     ``ssm_state_indices [B]`` of ``pool``.  Slot ids ``<= 0`` are skipped."""
+    lib = _lib._lib or _lib.load_library()
+    if lib.native.pool_move(lib.native_table, True, h, pool, ssm_state_indices, resid_fmt, keep_error, status):
+        return
     p = _pool_struct(pool, resid_fmt)
     dev = pool[0].device
     args = _lib.PoolStoreArgs()
@@ -114,7 +117,6 @@ def store_state(h, pool, ssm_state_indices, resid_fmt: int = RESID_INT8, keep_er
     args.keep_error = int(bool(keep_error))
     args.qmax = QMAX_INT8
     args.status = _lib.status_ptr(status, dev)
-    lib = _lib.load_library()
     with torch.cuda.device(dev):
         rc = lib.carry_gdn_pool_store(args, _lib.current_stream_ptr(dev))
     _lib.check(rc, "carry_gdn_pool_store")
@@ -125,6 +127,10 @@ def load_state(pool, ssm_state_indices, out=None, dtype=torch.float32, resid_fmt
     """``out[n] = codes * scale (+ resid_codes * resid_scale)`` of slot
     ``ssm_state_indices[n]``; zeros for slot ids ``<= 0``.  ``out`` is allocated
     (``dtype``) when not given.  Returns ``out [B, HV, V, K]``."""
+    lib = _lib._lib or _lib.load_library()
+    if out is not None and lib.native.pool_move(lib.native_table, False, out, pool, ssm_state_indices, resid_fmt,
+                                                with_residual, status):
+        return out
     p = _pool_struct(pool, resid_fmt)
     dev = pool[0].device
     B = ssm_state_indices.shape[0] if ssm_state_indices.dim() == 1 else 0
@@ -137,7 +143,6 @@ def load_state(pool, ssm_state_indices, out=None, dtype=torch.float32, resid_fmt
     args.h, args.stride_h_req, args.h_dtype = _state_tensor(out, B, p.HV, p.V, p.K, dev, "out")
     args.with_residual = int(bool(with_residual))
     args.status = _lib.status_ptr(status, dev)
-    lib = _lib.load_library()
     with torch.cuda.device(dev):
         rc = lib.carry_gdn_pool_load(args, _lib.current_stream_ptr(dev))
     _lib.check(rc, "carry_gdn_pool_load")
@@ -150,6 +155,9 @@ def copy_slots(src_pool, src_indices, dst_indices, dst_pool=None, resid_fmt: int
     with an id ``<= 0`` are skipped; no destination may also be a source or a
     second destination in the same call."""
     dst_pool = src_pool if dst_pool is None else dst_pool
+    lib = _lib._lib or _lib.load_library()
+    if lib.native.pool_copy(lib.native_table, src_pool, dst_pool, src_indices, dst_indices, resid_fmt, status):
+        return
     s = _pool_struct(src_pool, resid_fmt)
     d = _pool_struct(dst_pool, resid_fmt)
     if (s.HV, s.V, s.K) != (d.HV, d.V, d.K) or s.resid_scale_mode != d.resid_scale_mode:
@@ -165,7 +173,6 @@ def copy_slots(src_pool, src_indices, dst_indices, dst_pool=None, resid_fmt: int
     args.dst_slots, args.stride_dst_slots = _indices(dst_indices, "dst_indices", dev)
     args.B = src_indices.shape[0]
     args.status = _lib.status_ptr(status, dev)
-    lib = _lib.load_library()
     with torch.cuda.device(dev):
         rc = lib.carry_gdn_pool_copy(args, _lib.current_stream_ptr(dev))
     _lib.check(rc, "carry_gdn_pool_copy")

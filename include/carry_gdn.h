@@ -285,6 +285,30 @@ typedef struct CarryGdnPoolCopyArgs {
 
 int carry_gdn_pool_copy(const CarryGdnPoolCopyArgs* args, void* stream);
 
+/*
+ * The same for one slot of a whole stack of layers in one launch: slot src_slot
+ * of src[l] to slot dst_slot of dst[l] for every layer l.  `src` and `dst` are
+ * host arrays of `layers` pools of one shape and format; the slot ids are
+ * given by value and have to lie in 1 .. num_slots - 1 of every pool
+ * (CARRY_GDN_ERR_SHAPE otherwise).  What a cache manager does when it preempts,
+ * resumes, forks, checkpoints or rolls back one request.
+ */
+typedef struct CarryGdnPoolCopyLayersArgs {
+  const CarryGdnPool* src;
+  const CarryGdnPool* dst;
+  int32_t layers;
+  int32_t src_slot, dst_slot;
+} CarryGdnPoolCopyLayersArgs;
+
+int carry_gdn_pool_copy_layers(const CarryGdnPoolCopyLayersArgs* args, void* stream);
+
+/*
+ * Write n int32 values (slot ids) from host memory to device memory in stream
+ * order.  They travel as kernel arguments: the call reads `ids` before it
+ * returns and neither stages nor synchronises.
+ */
+int carry_gdn_write_ids(int32_t* dst, const int32_t* ids, int32_t n, void* stream);
+
 /* Human-readable text for a CARRY_GDN_ERR_* code (static storage). */
 const char* carry_gdn_strerror(int code);
 
