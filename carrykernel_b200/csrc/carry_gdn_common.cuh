@@ -61,6 +61,14 @@ struct KParams {
   void* out;
 };
 
+// head counts as shifts where they are powers of two (split_tile)
+inline void fill_shifts(KParams& p) {
+  auto log2_or_minus1 = [](int x) { int s = 0; while ((1 << s) < x) ++s; return (1 << s) == x ? s : -1; };
+  p.hv_shift = log2_or_minus1(p.HV);
+  p.group = p.HV / p.H;
+  p.group_shift = log2_or_minus1(p.group);
+}
+
 __device__ __forceinline__ float load_as_float(const void* p, long long i, int dtype) {
   if (dtype == CARRY_F32) return reinterpret_cast<const float*>(p)[i];
   if (dtype == CARRY_BF16) return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[i]);
@@ -212,6 +220,8 @@ bool tile128_eligible(const KParams& p);
 int launch_tile128(const KParams& p, cudaStream_t stream);
 int launch_multi(const KParams& p, int T, long long stride_mixed_t, long long stride_a_t, long long stride_b_t,
                  cudaStream_t stream);
+bool narrow64_eligible(const KParams& p);
+int launch_narrow64(const KParams& p, cudaStream_t stream);
 bool noef128_eligible(const KParams& p);
 int launch_noef128(const KParams& p, cudaStream_t stream);
 int launch_pool_store(const CarryGdnPoolStoreArgs& a, cudaStream_t stream);

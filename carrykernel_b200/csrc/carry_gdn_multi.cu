@@ -208,10 +208,7 @@ int launch_multi_dtype(const KParams& p, const MultiExtra& x, cudaStream_t strea
 int launch_multi(const KParams& p_in, int T, long long stride_mixed_t, long long stride_a_t, long long stride_b_t,
                  cudaStream_t stream) {
   KParams p = p_in;
-  auto log2_or_minus1 = [](int v) { int s = 0; while ((1 << s) < v) ++s; return (1 << s) == v ? s : -1; };
-  p.hv_shift = log2_or_minus1(p.HV);
-  p.group = p.HV / p.H;
-  p.group_shift = log2_or_minus1(p.group);
+  fill_shifts(p);
   MultiExtra x = {T, stride_mixed_t, stride_a_t, stride_b_t};
   const bool i4 = p.res_fmt == CARRY_RES_INT4, pv = p.rscale_mode == CARRY_SCALE_PER_V;
   if (i4) return pv ? launch_multi_dtype<CARRY_RES_INT4, CARRY_SCALE_PER_V>(p, x, stream)
