@@ -68,6 +68,16 @@ __device__ __forceinline__ void s4x8(uint32_t w, float2 (&e)[4]) {
   e[0] = pair(0x7440); e[1] = pair(0x7441); e[2] = pair(0x7442); e[3] = pair(0x7443);
 }
 
+// One element whose remainder lies within the tie guard, by the true quotient.  Element by element: a state that its
+// inputs hold at a fixed point has remainders near half a step in every row, so a word of codes often has one.
+__device__ __forceinline__ void redecide(float x, float& e, float& y, float s, float thr) {
+  if (fabsf(e) > thr) {
+    const float code = exact_code(x, s);
+    y = __fadd_rn(code, kMagicRound);
+    e = __fadd_rn(x, -__fmul_rn(code, s));
+  }
+}
+
 // round_half_even(x / s) of a row of 64 by the reciprocal (exact: see the tie guard in carry_gdn_tile128.cuh), handed to
 // `put` pair by pair as code + kMagicRound; KEEP: the remainders x - code * s, the product rounded first, stay in x.
 // Returns the largest remainder.
@@ -86,12 +96,11 @@ __device__ __forceinline__ float quantize_row(float2 (&x)[kN / 2], float s, Put&
       e[i] = add2(x[j + i], product2(add2(y[i], nmagic2), ns2));
       m = max3abs(m, e[i]);
     }
-    if (m > thr) {                      // rare: a quotient that the reciprocal may have tipped over a tie
+    if (m > thr) {                      // a quotient that the reciprocal may have tipped over a tie
       m = 0.f;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        y[i] = add2(make_float2(exact_code(x[j + i].x, s), exact_code(x[j + i].y, s)), magic2);
-        e[i] = add2(x[j + i], product2(add2(y[i], nmagic2), ns2));
+        redecide(x[j + i].x, e[i].x, y[i].x, s, thr); redecide(x[j + i].y, e[i].y, y[i].y, s, thr);
         m = max3abs(m, e[i]);
       }
     }
