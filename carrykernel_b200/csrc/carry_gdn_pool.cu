@@ -558,6 +558,204 @@ __global__ void __launch_bounds__(kThreads, 4) pool_load_kernel(CarryGdnPoolLoad
 }
 
 // ---------------------------------------------------------------------------
+// square tiles of 128 or 64: the whole tile in registers
+// ---------------------------------------------------------------------------
+// A tile's row is KL lanes x 4 elements (KL = 32 or 16), a lane holds ROWS rows of it (16 or 4), a CTA of 8 warps the
+// whole tile: 64 or 16 elements per lane, every load of a tile in flight at once, each element read and
+// written once.  Row maxima by a halving exchange that leaves one row's maximum in each lane, so a row's scale and
+// reciprocal are worked out once instead of in all 32 lanes.  The error of a per-head residual waits in
+// registers for the tile's maximum (the loops below read and encode the tile a second time for it).
+template <int KL>
+struct TileRows {
+  static constexpr int kRowsPerLane = KL == 32 ? 16 : 4;
+  static constexpr int kLanesPerRow = KL / kRowsPerLane;      // lanes that end up with the same row's maximum
+  static constexpr int kEdge = 4 * KL;                        // K = V
+  static_assert(kEdge == kWarps * (32 / KL) * kRowsPerLane, "8 warps cover the tile");
+};
+
+// m[r]: this lane's part of row r's maximum.  Returns the maximum of row lane_in_row / kLanesPerRow.
+template <int KL>
+__device__ __forceinline__ float row_max_transposed(float (&m)[TileRows<KL>::kRowsPerLane], int lane) {
+  int half = KL / 2;
+#pragma unroll
+  for (int n = TileRows<KL>::kRowsPerLane / 2; n >= 1; n /= 2) {
+    const bool up = lane & half;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const float keep = up ? m[n + i] : m[i], send = up ? m[i] : m[n + i];
+      m[i] = fmaxf(keep, __shfl_xor_sync(0xffffffffu, send, half));
+    }
+    half /= 2;
+  }
+#pragma unroll
+  for (; half >= 1; half /= 2) m[0] = fmaxf(m[0], __shfl_xor_sync(0xffffffffu, m[0], half));
+  return m[0];
+}
+
+__device__ __forceinline__ float abs_max4(const float (&x)[4]) {
+  return fmaxf(fmaxf(fabsf(x[0]), fabsf(x[1])), fmaxf(fabsf(x[2]), fabsf(x[3])));
+}
+
+// codes of four elements as code + kMagic, and their remainders x - code * s (the product rounded first) in x
+__device__ __forceinline__ void encode4(float (&x)[4], float s, float inv, float qmax, float (&y)[4]) {
+  float e[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    y[i] = fmaf(x[i], inv, kMagic);
+    e[i] = __fadd_rn(x[i], -__fmul_rn(y[i] - kMagic, s));
+  }
+  if (abs_max4(e) > kTieGuard * s) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (fabsf(e[i]) > kTieGuard * s) {
+        y[i] = quantize_div(x[i], s, qmax) + kMagic;
+        e[i] = __fadd_rn(x[i], -__fmul_rn(y[i] - kMagic, s));
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) x[i] = e[i];
+}
+
+template <int DT>
+__device__ __forceinline__ void load4(const void* base, long long off, float (&x)[4]) { load_row<4>(base, off, DT, x); }
+
+template <int KL, int DT>
+__global__ void __launch_bounds__(kThreads, KL == 32 ? 2 : 6) pool_store_tile_kernel(const __grid_constant__ CarryGdnPoolStoreArgs a) {
+  using R = TileRows<KL>;
+  constexpr int N = R::kRowsPerLane, K = R::kEdge;
+  __shared__ float s_emax[kWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lk = lane & (KL - 1), base = lane & ~(KL - 1);
+  const int v0 = (warp * (32 / KL) + lane / KL) * N, k = 4 * lk;          // my rows v0 .. v0 + N - 1, columns k .. k + 3
+  const int my_row = lk / R::kLanesPerRow;
+  const CarryGdnPool& pool = a.pool;
+  const bool int4 = pool.res_fmt == CARRY_RES_INT4, per_head = pool.resid_scale_mode == CARRY_SCALE_PER_HEAD;
+  const float rq = int4 ? 7.0f : 127.0f;
+  const int rrow = int4 ? K / 2 : K;
+  depend_release();
+  const int n = (int)(blockIdx.x / pool.HV), hv = (int)(blockIdx.x % pool.HV);
+  depend_wait();
+  const long long at = (long long)n * a.stride_h_req + ((long long)hv * K + v0) * K + k;
+  float x[N][4];
+#pragma unroll
+  for (int r = 0; r < N; ++r) load4<DT>(a.h, at + r * K, x[r]);
+  const int slot = slot_of(a.slots, a.stride_slots, n, pool.num_slots, a.status);
+  if (slot < 0) return;
+  const PoolView t = view_of(pool, slot, hv);
+  int8_t* crow = t.codes + v0 * K + k;
+  int8_t* prow = t.resid + v0 * rrow + (int4 ? k >> 1 : k);
+  auto put_resid = [&](int r, const float (&y)[4]) {
+    if (int4) store_nibbles<4>(prow + r * rrow, 0, true, y);
+    else store_codes<4>(prow, r * rrow, y);
+  };
+
+  float m[N];
+#pragma unroll
+  for (int r = 0; r < N; ++r) m[r] = abs_max4(x[r]);
+  const float s_mine = scale_from_amax(row_max_transposed<KL>(m, lk), a.qmax, CARRY_EPS_ON_AMAX);
+  const float i_mine = rcp_refined(s_mine);
+  if (lk % R::kLanesPerRow == 0) t.sscale[v0 + my_row] = s_mine;
+#pragma unroll
+  for (int r = 0; r < N; ++r) {
+    const float s = __shfl_sync(0xffffffffu, s_mine, base + r * R::kLanesPerRow);
+    const float inv = __shfl_sync(0xffffffffu, i_mine, base + r * R::kLanesPerRow);
+    float y[4];
+    encode4(x[r], s, inv, a.qmax, y);
+    store_codes<4>(crow, r * K, y);
+    m[r] = abs_max4(x[r]);
+  }
+  if (!a.keep_error) {
+    const float zero[4] = {kMagic, kMagic, kMagic, kMagic};
+#pragma unroll
+    for (int r = 0; r < N; ++r) put_resid(r, zero);
+    if (per_head) {
+      if (threadIdx.x == 0) t.rscale[0] = 0.0f;
+    } else if (lk % R::kLanesPerRow == 0) {
+      t.rscale[v0 + my_row] = 0.0f;
+    }
+    return;
+  }
+  float es_mine;
+  if (per_head) {
+    float top = 0.f;
+#pragma unroll
+    for (int r = 0; r < N; ++r) top = fmaxf(top, m[r]);
+    top = warp_max_nonneg(top);
+    if (lane == 0) s_emax[warp] = top;
+    __syncthreads();
+    es_mine = scale_from_amax(warp_max_nonneg(s_emax[lane & (kWarps - 1)]), rq, CARRY_EPS_ON_SCALE);
+    if (threadIdx.x == 0) t.rscale[0] = es_mine;
+  } else {
+    es_mine = scale_from_amax(row_max_transposed<KL>(m, lk), rq, CARRY_EPS_ON_SCALE);
+    if (lk % R::kLanesPerRow == 0) t.rscale[v0 + my_row] = es_mine;
+  }
+  const float ie_mine = rcp_refined(es_mine);
+#pragma unroll
+  for (int r = 0; r < N; ++r) {
+    const float es = per_head ? es_mine : __shfl_sync(0xffffffffu, es_mine, base + r * R::kLanesPerRow);
+    const float inv = per_head ? ie_mine : __shfl_sync(0xffffffffu, ie_mine, base + r * R::kLanesPerRow);
+    float y[4];
+    encode4(x[r], es, inv, rq, y);
+    put_resid(r, y);
+  }
+}
+
+template <int KL, int DT>
+__global__ void __launch_bounds__(kThreads, KL == 32 ? 3 : 6) pool_load_tile_kernel(const __grid_constant__ CarryGdnPoolLoadArgs a) {
+  using R = TileRows<KL>;
+  constexpr int N = R::kRowsPerLane, K = R::kEdge;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lk = lane & (KL - 1);
+  const int v0 = (warp * (32 / KL) + lane / KL) * N, k = 4 * lk;
+  const CarryGdnPool& pool = a.pool;
+  const bool int4 = pool.res_fmt == CARRY_RES_INT4, per_head = pool.resid_scale_mode == CARRY_SCALE_PER_HEAD;
+  const int rrow = int4 ? K / 2 : K;
+  depend_release();
+  const int n = (int)(blockIdx.x / pool.HV), hv = (int)(blockIdx.x % pool.HV);
+  depend_wait();
+  const int slot = slot_of(a.slots, a.stride_slots, n, pool.num_slots, a.status);
+  const long long at = (long long)n * a.stride_h_req + ((long long)hv * K + v0) * K + k;
+  if (slot < 0) {
+    const float zero[4] = {};
+#pragma unroll
+    for (int r = 0; r < N; ++r) store_row<4>(a.h, at + r * K, DT, zero);
+    return;
+  }
+  const PoolView t = view_of(pool, slot, hv);
+  const int8_t* crow = t.codes + v0 * K + k;
+  const int8_t* prow = t.resid + v0 * rrow + (int4 ? k >> 1 : k);
+  uint32_t cw[N], rw[N];
+#pragma unroll
+  for (int r = 0; r < N; ++r) cw[r] = *reinterpret_cast<const uint32_t*>(crow + r * K);
+#pragma unroll
+  for (int r = 0; r < N; ++r) {
+    rw[r] = 0u;
+    if (a.with_residual)
+      rw[r] = int4 ? (uint32_t)*reinterpret_cast<const uint16_t*>(prow + r * rrow) : *reinterpret_cast<const uint32_t*>(prow + r * rrow);
+  }
+  const float es_head = a.with_residual && per_head ? t.rscale[0] : 0.f;
+#pragma unroll
+  for (int r0 = 0; r0 < N; r0 += 4) {
+    const float4 s4 = *reinterpret_cast<const float4*>(t.sscale + v0 + r0);
+    float4 e4 = make_float4(es_head, es_head, es_head, es_head);
+    if (a.with_residual && !per_head) e4 = *reinterpret_cast<const float4*>(t.rscale + v0 + r0);
+    const float s[4] = {s4.x, s4.y, s4.z, s4.w}, es[4] = {e4.x, e4.y, e4.z, e4.w};
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      float x[4], cd[4], rd[4];
+      codes_of<4>(cw[r0 + r], cd);
+      if (int4) nibbles_of<4>(rw[r0 + r], rd);
+      else codes_of<4>(rw[r0 + r], rd);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        x[i] = __fmul_rn(cd[i], s[r]);
+        if (a.with_residual) x[i] = __fadd_rn(x[i], __fmul_rn(rd[i], es[r]));
+      }
+      store_row<4>(a.h, at + (r0 + r) * K, DT, x);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
 // slot -> slot
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void copy_bytes(void* dst, const void* src, long long bytes) {
@@ -664,7 +862,25 @@ int finish_launch() { return cudaGetLastError() == cudaSuccess ? CARRY_GDN_OK : 
 
 }  // namespace
 
+namespace {
+// Square tiles of 128 or 64 whose rows start on the vector boundaries; any other shape goes through the loops.
+int square_tile(const CarryGdnPool& pool, const void* h, long long stride_h_req, int h_dtype, int B) {
+  if (pool.K != pool.V || (pool.K != 128 && pool.K != 64)) return 0;
+  if ((long long)B * pool.HV > 0x7fffffffLL) return 0;
+  return vector_ok(pool, h, stride_h_req, h_dtype) ? pool.K : 0;
+}
+template <class Args>
+int launch_square(const Args& a, int edge, void (*k128[3])(Args), void (*k64[3])(Args), cudaStream_t stream) {
+  return launch_dependent((edge == 128 ? k128 : k64)[a.h_dtype], dim3((unsigned)(a.B * a.pool.HV)), kThreads, 0, stream, a);
+}
+}  // namespace
+
 int launch_pool_store(const CarryGdnPoolStoreArgs& a, cudaStream_t stream) {
+  if (const int edge = square_tile(a.pool, a.h, a.stride_h_req, a.h_dtype, a.B)) {
+    void (*k128[3])(CarryGdnPoolStoreArgs) = {pool_store_tile_kernel<32, CARRY_F32>, pool_store_tile_kernel<32, CARRY_BF16>, pool_store_tile_kernel<32, CARRY_F16>};
+    void (*k64[3])(CarryGdnPoolStoreArgs) = {pool_store_tile_kernel<16, CARRY_F32>, pool_store_tile_kernel<16, CARRY_BF16>, pool_store_tile_kernel<16, CARRY_F16>};
+    return launch_square(a, edge, k128, k64, stream);
+  }
   const int grid = grid_for((long long)a.B * a.pool.HV);
   if (vector_ok(a.pool, a.h, a.stride_h_req, a.h_dtype))
     pool_store_kernel<4><<<grid, kThreads, 0, stream>>>(a);
@@ -674,6 +890,11 @@ int launch_pool_store(const CarryGdnPoolStoreArgs& a, cudaStream_t stream) {
 }
 
 int launch_pool_load(const CarryGdnPoolLoadArgs& a, cudaStream_t stream) {
+  if (const int edge = square_tile(a.pool, a.h, a.stride_h_req, a.h_dtype, a.B)) {
+    void (*k128[3])(CarryGdnPoolLoadArgs) = {pool_load_tile_kernel<32, CARRY_F32>, pool_load_tile_kernel<32, CARRY_BF16>, pool_load_tile_kernel<32, CARRY_F16>};
+    void (*k64[3])(CarryGdnPoolLoadArgs) = {pool_load_tile_kernel<16, CARRY_F32>, pool_load_tile_kernel<16, CARRY_BF16>, pool_load_tile_kernel<16, CARRY_F16>};
+    return launch_square(a, edge, k128, k64, stream);
+  }
   const int grid = grid_for((long long)a.B * a.pool.HV);
   if (vector_ok(a.pool, a.h, a.stride_h_req, a.h_dtype))
     pool_load_kernel<4><<<grid, kThreads, 0, stream>>>(a);
