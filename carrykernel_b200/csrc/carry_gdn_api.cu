@@ -16,17 +16,12 @@ int dispatch(const carry::KParams& p, cudaStream_t stream) {
   if ((long long)p.B * p.HV == 0) return CARRY_GDN_OK;
   if (carry::tile128_eligible(p)) {
     const int rc = carry::launch_tile128(p, stream);
-    if (rc == CARRY_GDN_OK) g_last_kernel = 2;
+    if (rc == CARRY_GDN_OK) g_last_kernel = p.res_fmt == CARRY_RES_NONE ? 5 : 2;
     return rc;
   }
   if (carry::narrow64_eligible(p)) {
     const int rc = carry::launch_narrow64(p, stream);
     if (rc == CARRY_GDN_OK) g_last_kernel = 6;
-    return rc;
-  }
-  if (carry::noef128_eligible(p)) {
-    const int rc = carry::launch_noef128(p, stream);
-    if (rc == CARRY_GDN_OK) g_last_kernel = 5;
     return rc;
   }
   const int rc = carry::launch_generic(p, stream);

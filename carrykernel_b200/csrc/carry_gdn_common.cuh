@@ -222,8 +222,6 @@ int launch_multi(const KParams& p, int T, long long stride_mixed_t, long long st
                  cudaStream_t stream);
 bool narrow64_eligible(const KParams& p);
 int launch_narrow64(const KParams& p, cudaStream_t stream);
-bool noef128_eligible(const KParams& p);
-int launch_noef128(const KParams& p, cudaStream_t stream);
 int launch_pool_store(const CarryGdnPoolStoreArgs& a, cudaStream_t stream);
 int launch_pool_load(const CarryGdnPoolLoadArgs& a, cudaStream_t stream);
 int launch_pool_copy(const CarryGdnPoolCopyArgs& a, cudaStream_t stream);

@@ -24,7 +24,7 @@
 //     the next tile).
 //   * statequant layout [K][V] (scale per column): lane = 4 contiguous columns
 //     x the warp's 16 rows; column sums are finished across the 8 warps through
-//     shared memory (three meetings per tile).
+//     shared memory (three meetings per tile).  Here a step may also have no residual at all.
 //
 // Arithmetic.  Everything that feeds a state code keeps the reference's operation
 // order, with the contractions written out as explicit fused multiply-adds:
@@ -350,7 +350,7 @@ __device__ __forceinline__ float scale_fast(float amax, float qmax, float rq, in
 // the per-warp q scratch (slot layout) or the column-reduction space (statequant
 // layout).  Upper bounds, used to size the ring.
 constexpr int kStaticVK = 11776;        // per group
-constexpr int kStaticKV = 24064;
+constexpr int kStaticKV = 22528;
 constexpr int kStaticOf(int layout) { return layout == 0 ? kStaticVK : kStaticKV; }
 constexpr int kSmemPerCta = 231424;     // one CTA per SM: 227 KB less 1 KB
 
@@ -359,15 +359,18 @@ struct StageLayout {
   static constexpr int kVecBytes = kT * (QDT == CARRY_F32 ? 4 : 2);
   // integer residuals carry a scale (per V or per head); the float ones (fp32, fp16, fp8-e5m2) do not
   static constexpr bool kFloatResid = RES == CARRY_RES_FP32 || RES == CARRY_RES_FP16 || RES == CARRY_RES_FP8;
-  static constexpr int kResidBytes = (RES == CARRY_RES_INT4) ? kT * kT / 2
+  static constexpr bool kNoResid = RES == CARRY_RES_NONE;     // statequant layout only; RSCALE then says how the STATE is scaled
+  static constexpr bool kHeadState = kNoResid && RSCALE == CARRY_SCALE_PER_HEAD;
+  static constexpr int kResidBytes = kNoResid ? 0 : (RES == CARRY_RES_INT4) ? kT * kT / 2
                                      : (RES == CARRY_RES_FP32) ? kT * kT * 4
                                      : (RES == CARRY_RES_FP16) ? kT * kT * 2 : kT * kT;
   static constexpr int kCodes = 0;
   static constexpr int kResid = kT * kT;
   static constexpr int kSScale = kResid + kResidBytes;       // 128 floats
   static constexpr int kRScale = kSScale + 512;              // 128 floats (per V), or the 16 bytes that hold
-  static constexpr int kRScaleBytes = kFloatResid ? 0 : (RSCALE == CARRY_SCALE_PER_V) ? 512 : 16;   // this head's scale (per head)
-  static constexpr int kQ = kRScale + (kFloatResid ? 0 : (RSCALE == CARRY_SCALE_PER_V) ? 512 : 128);   // raw q, k, v of this head
+  static constexpr int kSScaleBytes = kHeadState ? 0 : 512;  // one scale per head comes with the tile's facts (TileMeta::k_mul)
+  static constexpr int kRScaleBytes = (kFloatResid || kNoResid) ? 0 : (RSCALE == CARRY_SCALE_PER_V) ? 512 : 16;   // this head's scale (per head)
+  static constexpr int kQ = kRScale + ((kFloatResid || kNoResid) ? 0 : (RSCALE == CARRY_SCALE_PER_V) ? 512 : 128);   // raw q, k, v of this head
   static constexpr int kK = kQ + kVecBytes;
   static constexpr int kV = kK + kVecBytes;
   static constexpr int kBytes = kV + kVecBytes;
@@ -472,9 +475,12 @@ __device__ __forceinline__ GateRaw gate_loads(const KParams& p, int n, int hv, l
     r.A_log = load_raw(p.A_log, hv, p.A_log_dtype);
     r.dt_bias = load_raw(p.dt_bias, hv, p.dt_bias_dtype);
   } else {
-    r.a = __float_as_uint(__ldcg(p.alpha + (long long)n * p.HV + hv));
-    r.b = __float_as_uint(__ldcg(p.beta + (long long)n * p.HV + hv));
-    r.A_log = r.dt_bias = 0u;
+    const long long nh = (long long)n * p.HV + hv;
+    r.a = __float_as_uint(__ldcg(p.alpha + nh + tok_a));
+    r.b = __float_as_uint(__ldcg(p.beta + nh + tok_b));
+    // a state scaled per head brings its scale along here
+    r.A_log = p.sscale_mode == CARRY_SCALE_PER_HEAD ? __float_as_uint(__ldcg(p.sscale_in + nh)) : __float_as_uint(1.0f);
+    r.dt_bias = 0u;
   }
   return r;
 }
@@ -499,7 +505,8 @@ __device__ __forceinline__ void split_tile(const KParams& p, int tile, int& n, i
 struct __align__(16) TileMeta {
   int n, hv, slot;
   float alpha, beta;
-  float k_mul, q_mul;   // 1/|k| and scale/|q| (1 when the L2 norm is off or on the statequant path)
+  float k_mul, q_mul;   // 1/|k| and scale/|q| (1 when the L2 norm is off); statequant path: the state's scale
+                        // where it has one per head, else 1, and 1
   float kq;             // <k, q> after those factors
 };
 static_assert(sizeof(TileMeta) == 32, "TileMeta is read as two 16-byte words");
@@ -520,6 +527,7 @@ __device__ __forceinline__ void tile_addresses(const KParams& p, int n, int hv, 
   constexpr long long KV = kT * kT;
   constexpr long long RB = (RES == CARRY_RES_INT4) ? KV / 2 : (RES == CARRY_RES_FP32) ? 4 * KV
                            : (RES == CARRY_RES_FP16) ? 2 * KV : KV;
+  constexpr bool head_state = RES == CARRY_RES_NONE && RSCALE == CARRY_SCALE_PER_HEAD;
   const long long nh = (long long)n * p.HV + hv;
   if (p.packed) {
     a[D_CODES] = reinterpret_cast<unsigned long long>(p.codes_out + slot * p.stride_state_slot + hv * KV);
@@ -535,7 +543,7 @@ __device__ __forceinline__ void tile_addresses(const KParams& p, int n, int hv, 
   } else {
     a[D_CODES] = reinterpret_cast<unsigned long long>(p.codes_out + nh * KV);
     a[D_RESID] = reinterpret_cast<unsigned long long>(reinterpret_cast<uint8_t*>(p.resid_out) + nh * RB);
-    a[D_SSCALE] = reinterpret_cast<unsigned long long>(p.sscale_out + nh * kT);
+    a[D_SSCALE] = reinterpret_cast<unsigned long long>(p.sscale_out + (head_state ? nh : nh * kT));
     a[D_RSCALE] = reinterpret_cast<unsigned long long>(p.rscale_out + (RSCALE == CARRY_SCALE_PER_V ? nh * kT : nh));
     a[D_RSCALE_IN] = reinterpret_cast<unsigned long long>(p.rscale_in + (RSCALE == CARRY_SCALE_PER_V ? nh * kT : (nh & ~3LL)));
     a[D_Q] = reinterpret_cast<unsigned long long>(reinterpret_cast<const uint8_t*>(p.q) + nh * kT * qes);
@@ -576,7 +584,7 @@ __device__ __forceinline__ void meta_vectors(const KParams& p, int n, int hv, in
     q_off = (long long)n * p.stride_mixed_tok + (long long)h * kT + tok_qkv;
     k_off = q_off + (long long)p.H * kT;
   } else {
-    q_off = k_off = ((long long)n * p.HV + hv) * kT;
+    q_off = k_off = ((long long)n * p.HV + hv) * kT + tok_qkv;
   }
   qp = reinterpret_cast<const uint8_t*>(p.q) + (q_off + MetaRaw<QDT, LPT>::kElems * sub) * qes;
   kp = reinterpret_cast<const uint8_t*>(p.k) + (k_off + MetaRaw<QDT, LPT>::kElems * sub) * qes;
@@ -683,6 +691,7 @@ __device__ __forceinline__ void meta_math(const KParams& p, const MetaRaw<QDT, L
     m.q_mul *= p.qscale;
   }
   m.kq = kqsum * (m.k_mul * m.q_mul);
+  if (!p.packed) m.k_mul = __uint_as_float(r.g.A_log);
 }
 // A slot id beyond the pool is treated as padding (and reported by meta_put); the tile's addresses follow
 // from the slot id that is left.  No side effects: this, too, can run ahead of the dependency wait.
@@ -738,10 +747,10 @@ __device__ __forceinline__ void issue_copies(const KParams& p, uint8_t* sb, uint
   const long long d_codes = reinterpret_cast<const uint8_t*>(p.codes_in) - reinterpret_cast<const uint8_t*>(p.codes_out);
   const long long d_resid = reinterpret_cast<const uint8_t*>(p.resid_in) - reinterpret_cast<const uint8_t*>(p.resid_out);
   const long long d_sscale = reinterpret_cast<const uint8_t*>(p.sscale_in) - reinterpret_cast<const uint8_t*>(p.sscale_out);
-  mbar_arrive_expect_tx(bar, kT * kT + L::kResidBytes + 512 + rscale_bytes + 3 * L::kVecBytes + test_extra_tx(tile));
+  mbar_arrive_expect_tx(bar, kT * kT + L::kResidBytes + L::kSScaleBytes + rscale_bytes + 3 * L::kVecBytes + test_extra_tx(tile));
   bulk_load(sb + L::kCodes, reinterpret_cast<const void*>(a[D_CODES] + d_codes), kT * kT, bar);
-  bulk_load(sb + L::kResid, reinterpret_cast<const void*>(a[D_RESID] + d_resid), L::kResidBytes, bar);
-  bulk_load(sb + L::kSScale, reinterpret_cast<const void*>(a[D_SSCALE] + d_sscale), 512, bar);
+  if constexpr (L::kResidBytes > 0) bulk_load(sb + L::kResid, reinterpret_cast<const void*>(a[D_RESID] + d_resid), L::kResidBytes, bar);
+  if constexpr (L::kSScaleBytes > 0) bulk_load(sb + L::kSScale, reinterpret_cast<const void*>(a[D_SSCALE] + d_sscale), L::kSScaleBytes, bar);
   if constexpr (rscale_bytes > 0) bulk_load(sb + L::kRScale, reinterpret_cast<const void*>(a[D_RSCALE_IN]), rscale_bytes, bar);
   bulk_load(sb + L::kQ, reinterpret_cast<const void*>(a[D_Q]), L::kVecBytes, bar);
   bulk_load(sb + L::kK, reinterpret_cast<const void*>(a[D_K]), L::kVecBytes, bar);
@@ -789,9 +798,10 @@ gdn_tile128_kernel(const __grid_constant__ KParams p) {
   __shared__ TileMeta meta_cache[kCache + G * kWarps];   // this CTA's first tiles; one spare entry per warp
   __shared__ TileDesc desc_cache[kCache + G * kWarps];   // their addresses
   __shared__ __align__(16) float q_warp[(LAYOUT == LAYOUT_VK) ? G * kWarps * kT : 4];   // per warp: q, scaled, as pairs
-  __shared__ __align__(16) float col_red_all[(LAYOUT == LAYOUT_KV) ? G * kWarps * kT * 4 : 4];
+  __shared__ __align__(16) float col_red_all[(LAYOUT == LAYOUT_KV) ? G * kWarps * kT * 3 : 4];
+  __shared__ __align__(16) float4 kq_rows[(LAYOUT == LAYOUT_KV) ? G * kWarps * 16 : 1];   // per warp: {k, k, q, q} of its rows
   static_assert(sizeof(full_bar) + sizeof(claimed) + sizeof(first_cnt) + sizeof(stage_tile) + sizeof(head_red) + sizeof(meta_cache) + sizeof(desc_cache) +
-                        sizeof(q_warp) + sizeof(col_red_all) + 64 <= L::kStatic,
+                        sizeof(q_warp) + sizeof(col_red_all) + sizeof(kq_rows) + 64 <= L::kStatic,
                 "static shared memory exceeds what the stage ring was sized for");
   static_assert(S >= 2 * G, "every group needs a stage in use and one on the way");
 
@@ -799,7 +809,7 @@ gdn_tile128_kernel(const __grid_constant__ KParams p) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int grp = (G == 1) ? 0 : (warp >> 3), gw = warp & 7, gtid = tid & (kThreads - 1);
   const int bar0 = 3 * grp;                          // this group's named barriers are bar0 + 1 .. bar0 + 3
-  float* col_red = col_red_all + ((LAYOUT == LAYOUT_KV) ? grp * kWarps * kT * 4 : 0);
+  float* col_red = col_red_all + ((LAYOUT == LAYOUT_KV) ? grp * kWarps * kT * 3 : 0);
   const int total = p.B * p.HV;
   const int my_tiles = (total - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
   volatile int* poison = &poison_flag;
@@ -860,8 +870,8 @@ gdn_tile128_kernel(const __grid_constant__ KParams p) {
           const long long d_resid = reinterpret_cast<const uint8_t*>(p.resid_in) - reinterpret_cast<const uint8_t*>(p.resid_out);
           const long long d_sscale = reinterpret_cast<const uint8_t*>(p.sscale_in) - reinterpret_cast<const uint8_t*>(p.sscale_out);
           l2_prefetch_bulk(reinterpret_cast<const void*>(a[D_CODES] + d_codes), kT * kT);
-          l2_prefetch_bulk(reinterpret_cast<const void*>(a[D_RESID] + d_resid), L::kResidBytes);
-          l2_prefetch_bulk(reinterpret_cast<const void*>(a[D_SSCALE] + d_sscale), 512);
+          if constexpr (L::kResidBytes > 0) l2_prefetch_bulk(reinterpret_cast<const void*>(a[D_RESID] + d_resid), L::kResidBytes);
+          if constexpr (L::kSScaleBytes > 0) l2_prefetch_bulk(reinterpret_cast<const void*>(a[D_SSCALE] + d_sscale), L::kSScaleBytes);
         }
       }
       meta_math<QDT, LPT>(p, before, m);
@@ -1039,32 +1049,49 @@ gdn_tile128_kernel(const __grid_constant__ KParams p) {
         // ---------------- statequant layout [K][V]: lane = 4 columns x 16 rows ----
         // columns {c0, c0+1} are held as pair A, {c0+2, c0+3} as pair B
         const int r0 = 16 * gw, c0 = 4 * lane;
-        float* red_dot = col_red;                       // [warp][col][2]
-        float* red_max = col_red + kWarps * kT * 2;     // [warp][col]
-        float* red_emax = red_max + kWarps * kT;        // [warp][col]
-        // k and q of this warp's 16 rows are the same in every lane; they are read from the stage where they
-        // are used (a broadcast load) instead of being held in 32 registers.  k_mul and q_mul are 1 in this
-        // layout's callers but are applied all the same.
-        auto k_of = [&](int i) { return act<QDT>(sb + L::kK, r0 + i) * k_mul; };
-        auto q_of = [&](int i) { return act<QDT>(sb + L::kQ, r0 + i) * q_mul; };
-        float scol[4];
+        // Reduction space, three units of [warp][col]: sums (two units), maxima, remainder maxima.  The last share a
+        // unit with the sums, which everybody has read by the second meeting; that the next tile's sums, written with
+        // no meeting in between, do not run into them, the units trade places from tile to tile.
+        const int odd = cnt & 1;
+        float* red_dot = col_red + odd * kWarps * kT;                   // [warp][col][2]
+        float* red_max = col_red + (odd ? 0 : 2) * kWarps * kT;         // [warp][col]
+        float* red_emax = col_red + (odd ? 2 : 0) * kWarps * kT;        // [warp][col]
+        // k and q of this warp's 16 rows are the same in every lane.  One lane per value turns them to fp32 and
+        // writes each twice, side by side, so that a row's {k, k} and {q, q} are one broadcast load that feeds packed
+        // instructions as it is (three loads, three conversions and the register moves to pair a scalar up, per row,
+        // before: 1.15x at 256 requests).
+        float4* kq_row = kq_rows + warp * 16;
         {
+          const float x = act<QDT>(sb + (lane < 16 ? L::kK : L::kQ), r0 + (lane & 15));
+          *reinterpret_cast<float2*>(reinterpret_cast<float*>(kq_row + (lane & 15)) + (lane < 16 ? 0 : 2)) = splat(x);
+        }
+        float scol[4];
+        if constexpr (L::kHeadState) {
+          scol[0] = scol[1] = scol[2] = scol[3] = k_mul;
+        } else {
           const float4 s4 = *reinterpret_cast<const float4*>(sscale + c0);
           scol[0] = s4.x; scol[1] = s4.y; scol[2] = s4.z; scol[3] = s4.w;
         }
+        // Int4 residual and no residual: the sums run over the bare codes, a column's scale * decay goes on the
+        // totals (see carry_gdn_slot_tile.inc on what that moves).  The other formats keep the reference's order.
+        constexpr bool kFold = RES == CARRY_RES_INT4 || L::kNoResid;
         const float2 sA = make_float2(scol[0], scol[1]), sB = make_float2(scol[2], scol[3]);
+        const float2 saA = mul2(sA, alpha2), saB = mul2(sB, alpha2);
         float2 hA[16], hB[16];
         float2 dkA = make_float2(0.f, 0.f), dkB = dkA, dqA = dkA, dqB = dkA;
+        __syncwarp();
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          const uint32_t w = *reinterpret_cast<const uint32_t*>(sb + L::kCodes + (r0 + i) * kT + c0) ^ 0x80808080u;
-          const float2 a = mul2(mul2(s8x2_to_float<0, 1>(w), sA), alpha2);
-          const float2 b = mul2(mul2(s8x2_to_float<2, 3>(w), sB), alpha2);
+          const uint32_t w = *reinterpret_cast<const uint32_t*>(sb + L::kCodes + (r0 + i) * kT + c0);
+          float2 a = s8x2_cvt<0, 1>(w), b = s8x2_to_float<2, 3>(w ^ 0x80808080u);
+          if constexpr (!kFold) { a = mul2(mul2(a, sA), alpha2); b = mul2(mul2(b, sB), alpha2); }
           hA[i] = a; hB[i] = b;
-          const float2 kr = splat(k_of(i)), qr = splat(q_of(i));
+          const float4 kq4 = kq_row[i];
+          const float2 kr = make_float2(kq4.x, kq4.y), qr = make_float2(kq4.z, kq4.w);
           dkA = fma2(a, kr, dkA); dkB = fma2(b, kr, dkB);
           dqA = fma2(a, qr, dqA); dqB = fma2(b, qr, dqB);
         }
+        if constexpr (kFold) { dkA = mul2(dkA, saA); dkB = mul2(dkB, saB); dqA = mul2(dqA, saA); dqB = mul2(dqB, saB); }
         // finish the column sums across the 8 warps
         float dk[4], dq[4];
         {
@@ -1087,40 +1114,51 @@ gdn_tile128_kernel(const __grid_constant__ KParams p) {
         for (int b = 0; b < 4; ++b) {
           dv[b] = __fmul_rn(beta, __fadd_rn(act<QDT>(sb + L::kV, c0 + b), -dk[b]));
           oval[b] = fmaf(dv[b], kq, dq[b]);
-          es_col[b] = L::kFloatResid ? 0.f : (RSCALE == CARRY_SCALE_PER_V) ? rscale[c0 + b] : es_head;
+          es_col[b] = (L::kFloatResid || L::kNoResid) ? 0.f : (RSCALE == CARRY_SCALE_PER_V) ? rscale[c0 + b] : es_head;
         }
         const float2 dvA = make_float2(dv[0], dv[1]), dvB = make_float2(dv[2], dv[3]);
+        const float2 esA = make_float2(es_col[0], es_col[1]), esB = make_float2(es_col[2], es_col[3]);
+        const float2 nbA = mul2(esA, splat(-136.0f)), nbB = mul2(esB, splat(-136.0f));
         float amax[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          float2 eA, eB;
-          if constexpr (RES == CARRY_RES_FP32) {
-            const float4 e4 = *reinterpret_cast<const float4*>(sb + L::kResid + ((r0 + i) * kT + c0) * 4);
-            eA = make_float2(e4.x, e4.y); eB = make_float2(e4.z, e4.w);
-          } else if constexpr (RES == CARRY_RES_FP16) {
-            const uint2 e2 = *reinterpret_cast<const uint2*>(sb + L::kResid + ((r0 + i) * kT + c0) * 2);
-            eA = __half22float2(*reinterpret_cast<const __half2*>(&e2.x));
-            eB = __half22float2(*reinterpret_cast<const __half2*>(&e2.y));
-          } else if constexpr (RES == CARRY_RES_FP8) {
-            e5m2x4_to_float(*reinterpret_cast<const uint32_t*>(sb + L::kResid + (r0 + i) * kT + c0), eA, eB);
+          const float2 kr = *reinterpret_cast<const float2*>(kq_row + i);
+          float2 tA, tB;
+          if constexpr (L::kNoResid) {
+            tA = fma2(hA[i], saA, mul2(kr, dvA)); tB = fma2(hB[i], saB, mul2(kr, dvB));
           } else if constexpr (RES == CARRY_RES_INT4) {
+            // a nibble in offset binary lands in a float that reads 136 + code; 136 * es is in the innermost addend
             const uint32_t w =
                 (uint32_t)(*reinterpret_cast<const uint16_t*>(sb + L::kResid + (r0 + i) * (kT / 2) + c0 / 2)) ^ 0x8888u;
-            float2 lo, hi;                              // lo = cols {c0, c0+2}, hi = 16 * cols {c0+1, c0+3}
-            s4x4_to_float<0, 1>(w, lo, hi);
-            eA = mul2(make_float2(lo.x, hi.x), make_float2(es_col[0], es_col[1] * 0.0625f));
-            eB = mul2(make_float2(lo.y, hi.y), make_float2(es_col[2], es_col[3] * 0.0625f));
-          } else {
+            const uint32_t lo = w & 0x0F0Fu, hi = (w >> 4) & 0x0F0Fu;
+            const float2 nA = make_float2(__uint_as_float(__byte_perm(lo, 0x43000000u, 0x7044)), __uint_as_float(__byte_perm(hi, 0x43000000u, 0x7044)));
+            const float2 nB = make_float2(__uint_as_float(__byte_perm(lo, 0x43000000u, 0x7144)), __uint_as_float(__byte_perm(hi, 0x43000000u, 0x7144)));
+            tA = fma2(nA, esA, fma2(hA[i], saA, fma2(kr, dvA, nbA)));
+            tB = fma2(nB, esB, fma2(hB[i], saB, fma2(kr, dvB, nbB)));
+          } else if constexpr (RES == CARRY_RES_INT8) {
             const uint32_t w = *reinterpret_cast<const uint32_t*>(sb + L::kResid + (r0 + i) * kT + c0) ^ 0x80808080u;
-            eA = mul2(s8x2_to_float<0, 1>(w), make_float2(es_col[0], es_col[1]));
-            eB = mul2(s8x2_to_float<2, 3>(w), make_float2(es_col[2], es_col[3]));
+            tA = fma2(s8x2_to_float<0, 1>(w), esA, fma2(kr, dvA, hA[i]));
+            tB = fma2(s8x2_to_float<2, 3>(w), esB, fma2(kr, dvB, hB[i]));
+          } else {
+            float2 eA, eB;
+            if constexpr (RES == CARRY_RES_FP32) {
+              const float4 e4 = *reinterpret_cast<const float4*>(sb + L::kResid + ((r0 + i) * kT + c0) * 4);
+              eA = make_float2(e4.x, e4.y); eB = make_float2(e4.z, e4.w);
+            } else if constexpr (RES == CARRY_RES_FP16) {
+              const uint2 e2 = *reinterpret_cast<const uint2*>(sb + L::kResid + ((r0 + i) * kT + c0) * 2);
+              eA = __half22float2(*reinterpret_cast<const __half2*>(&e2.x));
+              eB = __half22float2(*reinterpret_cast<const __half2*>(&e2.y));
+            } else {
+              e5m2x4_to_float(*reinterpret_cast<const uint32_t*>(sb + L::kResid + (r0 + i) * kT + c0), eA, eB);
+            }
+            tA = add2(fma2(kr, dvA, hA[i]), eA);
+            tB = add2(fma2(kr, dvB, hB[i]), eB);
           }
-          const float2 kr = splat(k_of(i));
-          const float2 tA = add2(fma2(kr, dvA, hA[i]), eA);
-          const float2 tB = add2(fma2(kr, dvB, hB[i]), eB);
           hA[i] = tA; hB[i] = tB;
-          amax[0] = fmaxf(amax[0], fabsf(tA.x)); amax[1] = fmaxf(amax[1], fabsf(tA.y));
-          amax[2] = fmaxf(amax[2], fabsf(tB.x)); amax[3] = fmaxf(amax[3], fabsf(tB.y));
+          if (i & 1) {                                  // two rows per three-operand maximum
+            amax[0] = fmaxf(fmaxf(amax[0], fabsf(hA[i - 1].x)), fabsf(tA.x)); amax[1] = fmaxf(fmaxf(amax[1], fabsf(hA[i - 1].y)), fabsf(tA.y));
+            amax[2] = fmaxf(fmaxf(amax[2], fabsf(hB[i - 1].x)), fabsf(tB.x)); amax[3] = fmaxf(fmaxf(amax[3], fabsf(hB[i - 1].y)), fabsf(tB.y));
+          }
         }
         if (gw == 0) {
 #pragma unroll
@@ -1135,6 +1173,8 @@ gdn_tile128_kernel(const __grid_constant__ KParams p) {
           amax[2] = fmaxf(amax[2], x.z); amax[3] = fmaxf(amax[3], x.w);
         }
         float snew[4], thr[4];
+        if constexpr (L::kHeadState)                      // every warp holds all 128 column maxima
+          amax[0] = amax[1] = amax[2] = amax[3] = warp_max_nonneg(fmaxf(fmaxf(amax[0], amax[1]), fmaxf(amax[2], amax[3])));
 #pragma unroll
         for (int b = 0; b < 4; ++b) { snew[b] = scale_fast(amax[b], p.qmax, rqmax_state, p.eps_mode); thr[b] = snew[b] * kTieGuard; }
         const float2 invA = make_float2(rcp_refined(snew[0]), rcp_refined(snew[1]));
@@ -1148,8 +1188,10 @@ gdn_tile128_kernel(const __grid_constant__ KParams p) {
           hA[i] = fma2(add2(yA, nmagic2), nsA, hA[i]);
           hB[i] = fma2(add2(yB, nmagic2), nsB, hB[i]);
           cw[i] = pack4(__float_as_uint(yA.x), __float_as_uint(yA.y), __float_as_uint(yB.x), __float_as_uint(yB.y));
-          eamax[0] = fmaxf(eamax[0], fabsf(hA[i].x)); eamax[1] = fmaxf(eamax[1], fabsf(hA[i].y));
-          eamax[2] = fmaxf(eamax[2], fabsf(hB[i].x)); eamax[3] = fmaxf(eamax[3], fabsf(hB[i].y));
+          if (i & 1) {
+            eamax[0] = fmaxf(fmaxf(eamax[0], fabsf(hA[i - 1].x)), fabsf(hA[i].x)); eamax[1] = fmaxf(fmaxf(eamax[1], fabsf(hA[i - 1].y)), fabsf(hA[i].y));
+            eamax[2] = fmaxf(fmaxf(eamax[2], fabsf(hB[i - 1].x)), fabsf(hB[i].x)); eamax[3] = fmaxf(fmaxf(eamax[3], fabsf(hB[i - 1].y)), fabsf(hB[i].y));
+          }
         }
         if (fmaxf(fmaxf(eamax[0] - thr[0], eamax[1] - thr[1]), fmaxf(eamax[2] - thr[2], eamax[3] - thr[3])) > 0.f) {
           eamax[0] = eamax[1] = eamax[2] = eamax[3] = 0.f;      // rare: a quotient within the tie guard
@@ -1169,7 +1211,17 @@ gdn_tile128_kernel(const __grid_constant__ KParams p) {
 #pragma unroll
           for (int i = 0; i < 16; ++i) stg_b32(dst_codes + (r0 + i) * kT + c0, cw[i]);
         }
-        if constexpr (L::kFloatResid) {
+        if constexpr (L::kNoResid) {
+          if (lane == 0) claim_next(cnt);                 // the meeting only hands the stage on
+          warps_meet(bar0 + 3);
+          refill_stage(it);
+          if constexpr (L::kHeadState) {
+            if (gtid == 0) stg_b32(dst_of(D_SSCALE), __float_as_uint(snew[0]));
+          } else if ((lane >> 2) == gw) {
+            stg_v4(dst_of(D_SSCALE) + c0 * 4, make_uint4(__float_as_uint(snew[0]), __float_as_uint(snew[1]),
+                                                         __float_as_uint(snew[2]), __float_as_uint(snew[3])));
+          }
+        } else if constexpr (L::kFloatResid) {
           // the new residual is stored as it is, in its format; the meeting only hands the stage on
           if (lane == 0) claim_next(cnt);
           warps_meet(bar0 + 3);
@@ -1227,7 +1279,10 @@ gdn_tile128_kernel(const __grid_constant__ KParams p) {
           const uint32_t y0 = __float_as_uint(rA.x), y1 = __float_as_uint(rA.y);
           const uint32_t y2 = __float_as_uint(rB.x), y3 = __float_as_uint(rB.y);
           if constexpr (RES == CARRY_RES_INT4) {
-            const uint32_t v16 = (y0 & 0xFu) | ((y1 & 0xFu) << 4) | ((y2 & 0xFu) << 8) | ((y3 & 0xFu) << 12);
+            // 16 * odd + even (+ 136: both nibbles offset by 8) in one float, whose low byte is the pair
+            const uint32_t p01 = __float_as_uint(fmaf(__fadd_rn(rA.y, -kMagicRound), 16.0f, __fadd_rn(rA.x, 136.0f)));
+            const uint32_t p23 = __float_as_uint(fmaf(__fadd_rn(rB.y, -kMagicRound), 16.0f, __fadd_rn(rB.x, 136.0f)));
+            const uint32_t v16 = __byte_perm(p01, p23, 0x0040) ^ 0x8888u;
             stg_b16(dst_resid + (r0 + i) * (kT / 2) + c0 / 2, v16);
           } else {
             stg_b32(dst_resid + (r0 + i) * kT + c0, pack4(y0, y1, y2, y3));
@@ -1306,7 +1361,10 @@ int launch_dtype(const KParams& p, cudaStream_t stream, int sms) {
 // all variants of one memory layout
 template <int LAYOUT>
 int launch_layout(const KParams& p, cudaStream_t stream, int sms) {
-  if constexpr (LAYOUT == LAYOUT_KV) {     // the float residual formats exist on the statequant surfaces only
+  if constexpr (LAYOUT == LAYOUT_KV) {     // float residuals and none at all exist on the statequant surfaces only
+    if (p.res_fmt == CARRY_RES_NONE)
+      return p.sscale_mode == CARRY_SCALE_PER_V ? launch_dtype<LAYOUT, CARRY_RES_NONE, CARRY_SCALE_PER_V>(p, stream, sms)
+                                                : launch_dtype<LAYOUT, CARRY_RES_NONE, CARRY_SCALE_PER_HEAD>(p, stream, sms);
     if (p.res_fmt == CARRY_RES_FP32) return launch_dtype<LAYOUT, CARRY_RES_FP32, CARRY_SCALE_PER_V>(p, stream, sms);
     if (p.res_fmt == CARRY_RES_FP16) return launch_dtype<LAYOUT, CARRY_RES_FP16, CARRY_SCALE_PER_V>(p, stream, sms);
     if (p.res_fmt == CARRY_RES_FP8) return launch_dtype<LAYOUT, CARRY_RES_FP8, CARRY_SCALE_PER_V>(p, stream, sms);
