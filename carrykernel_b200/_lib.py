@@ -42,6 +42,10 @@ class StepArgs(C.Structure):
     ]
 
 
+class DecodeArgs(C.Structure):
+    _fields_ = [("step", StepArgs), ("h0", C.c_void_p), ("T", C.c_int32)]
+
+
 class Fp32Args(C.Structure):
     _fields_ = [
         ("h_in", C.c_void_p), ("q", C.c_void_p), ("k", C.c_void_p), ("v", C.c_void_p),
@@ -124,14 +128,15 @@ class PoolCopyLayersArgs(C.Structure):
 
 ERR_UNSUPPORTED = -5
 
-EXPORTS = ("carry_gdn_quant_step", "carry_gdn_fp32_step", "carry_gdn_packed_decode",
+EXPORTS = ("carry_gdn_quant_step", "carry_gdn_quant_decode", "carry_gdn_fp32_step", "carry_gdn_packed_decode",
            "carry_gdn_packed_decode_multi", "carry_gdn_pool_store", "carry_gdn_pool_load",
            "carry_gdn_pool_copy", "carry_gdn_pool_copy_layers", "carry_gdn_write_ids", "carry_gdn_strerror",
            "carry_gdn_abi_version", "carry_gdn_last_kernel")
 # what the native call path is given the addresses of, in the order it expects them (csrc/host_native.cpp, Table)
 _NATIVE_ENTRIES = ("carry_gdn_quant_step", "carry_gdn_fp32_step", "carry_gdn_packed_decode",
                    "carry_gdn_packed_decode_multi", "carry_gdn_pool_store", "carry_gdn_pool_load",
-                   "carry_gdn_pool_copy", "carry_gdn_pool_copy_layers", "carry_gdn_write_ids")
+                   "carry_gdn_pool_copy", "carry_gdn_pool_copy_layers", "carry_gdn_write_ids",
+                   "carry_gdn_quant_decode")
 
 _lib = None
 _lock = threading.Lock()
@@ -161,6 +166,7 @@ def load_library(path: str | None = None):
         lib.carry_gdn_abi_version.restype = C.c_int
         lib.carry_gdn_last_kernel.restype = C.c_int
         lib.carry_gdn_quant_step.argtypes = [C.POINTER(StepArgs), C.c_void_p]
+        lib.carry_gdn_quant_decode.argtypes = [C.POINTER(DecodeArgs), C.c_void_p]
         lib.carry_gdn_fp32_step.argtypes = [C.POINTER(Fp32Args), C.c_void_p]
         lib.carry_gdn_packed_decode.argtypes = [C.POINTER(PackedArgs), C.c_void_p]
         lib.carry_gdn_packed_decode_multi.argtypes = [C.POINTER(PackedMultiArgs), C.c_void_p]
@@ -171,7 +177,7 @@ def load_library(path: str | None = None):
         lib.carry_gdn_write_ids.argtypes = [C.c_void_p, C.c_void_p, C.c_int32, C.c_void_p]
         for fn in (lib.carry_gdn_quant_step, lib.carry_gdn_fp32_step, lib.carry_gdn_packed_decode,
                    lib.carry_gdn_packed_decode_multi, lib.carry_gdn_pool_store, lib.carry_gdn_pool_load,
-                   lib.carry_gdn_pool_copy, lib.carry_gdn_pool_copy_layers, lib.carry_gdn_write_ids):
+                   lib.carry_gdn_pool_copy, lib.carry_gdn_pool_copy_layers, lib.carry_gdn_write_ids, lib.carry_gdn_quant_decode):
             fn.restype = C.c_int
         if lib.carry_gdn_abi_version() != ABI_VERSION:
             raise CudaUnavailable(

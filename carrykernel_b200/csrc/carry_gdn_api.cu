@@ -78,6 +78,44 @@ int packed_params(const CarryGdnPackedArgs* a, KParams& p) {
   p.out = a->out;
   return CARRY_GDN_OK;
 }
+// Checks the arguments of a statequant step and turns them into kernel parameters.
+int step_params(const CarryGdnStepArgs* a, KParams& p) {
+  if (!a) return CARRY_GDN_ERR_NULL;
+  if (a->B < 0 || a->HV < 0 || a->K <= 0 || a->V <= 0) return CARRY_GDN_ERR_SHAPE;
+  if (!(a->qmax >= 1.0f && a->qmax <= 127.0f)) return CARRY_GDN_ERR_SHAPE;
+  if (!dtype_ok(a->qkv_dtype) || !dtype_ok(a->o_dtype)) return CARRY_GDN_ERR_DTYPE;
+  if (a->res_fmt < CARRY_RES_FP32 || a->res_fmt > CARRY_RES_NONE) return CARRY_GDN_ERR_FORMAT;
+  if (!scale_mode_ok(a->resid_scale_mode) || !scale_mode_ok(a->state_scale_mode) || !eps_ok(a->eps_mode))
+    return CARRY_GDN_ERR_FORMAT;
+  if (a->res_fmt == CARRY_RES_INT4 && (a->V & 1)) return CARRY_GDN_ERR_FORMAT;
+  if ((long long)a->B * a->HV == 0) return CARRY_GDN_OK;   // nothing to do; p is not filled
+  if (!a->h_in || !a->scale_in || !a->q || !a->k || !a->v || !a->alpha || !a->beta || !a->o ||
+      !a->h_out || !a->scale_out)
+    return CARRY_GDN_ERR_NULL;
+  const bool int_resid = a->res_fmt == CARRY_RES_INT8 || a->res_fmt == CARRY_RES_INT4;
+  if (a->res_fmt != CARRY_RES_NONE && (!a->e_in || !a->e_out)) return CARRY_GDN_ERR_NULL;
+  if (int_resid && (!a->e_scale_in || !a->e_scale_out)) return CARRY_GDN_ERR_NULL;
+
+  p = KParams{};
+  p.packed = 0;
+  p.B = a->B; p.H = a->HV; p.HV = a->HV; p.K = a->K; p.V = a->V;
+  p.qmax = a->qmax;
+  p.inv_qmax = 1.0f / a->qmax;
+  p.res_fmt = a->res_fmt; p.rscale_mode = a->resid_scale_mode; p.sscale_mode = a->state_scale_mode;
+  p.eps_mode = a->eps_mode;
+  p.qkv_dtype = a->qkv_dtype; p.o_dtype = a->o_dtype;
+  p.status = a->status;
+  p.codes_in = a->h_in; p.codes_out = a->h_out;
+  p.sscale_in = a->scale_in; p.sscale_out = a->scale_out;
+  p.resid_in = a->e_in; p.resid_out = a->e_out;
+  p.rscale_in = a->e_scale_in; p.rscale_out = a->e_scale_out;
+  p.q = a->q; p.k = a->k; p.v = a->v;
+  p.alpha = a->alpha; p.beta = a->beta;
+  p.qscale = 1.0f;
+  p.out = a->o;
+  return CARRY_GDN_OK;
+}
+
 }  // namespace carry
 
 // The runtime keeps a per-thread "last error" until somebody reads it.  Every entry point reads it away
@@ -108,40 +146,26 @@ const char* carry_gdn_strerror(int code) {
 
 int carry_gdn_quant_step(const CarryGdnStepArgs* a, void* stream) {
   clear_stale_error();
-  if (!a) return CARRY_GDN_ERR_NULL;
-  if (a->B < 0 || a->HV < 0 || a->K <= 0 || a->V <= 0) return CARRY_GDN_ERR_SHAPE;
-  if (!(a->qmax >= 1.0f && a->qmax <= 127.0f)) return CARRY_GDN_ERR_SHAPE;
-  if (!dtype_ok(a->qkv_dtype) || !dtype_ok(a->o_dtype)) return CARRY_GDN_ERR_DTYPE;
-  if (a->res_fmt < CARRY_RES_FP32 || a->res_fmt > CARRY_RES_NONE) return CARRY_GDN_ERR_FORMAT;
-  if (!scale_mode_ok(a->resid_scale_mode) || !scale_mode_ok(a->state_scale_mode) || !eps_ok(a->eps_mode))
-    return CARRY_GDN_ERR_FORMAT;
-  if (a->res_fmt == CARRY_RES_INT4 && (a->V & 1)) return CARRY_GDN_ERR_FORMAT;
-  if ((long long)a->B * a->HV == 0) return CARRY_GDN_OK;
-  if (!a->h_in || !a->scale_in || !a->q || !a->k || !a->v || !a->alpha || !a->beta || !a->o ||
-      !a->h_out || !a->scale_out)
-    return CARRY_GDN_ERR_NULL;
-  const bool int_resid = a->res_fmt == CARRY_RES_INT8 || a->res_fmt == CARRY_RES_INT4;
-  if (a->res_fmt != CARRY_RES_NONE && (!a->e_in || !a->e_out)) return CARRY_GDN_ERR_NULL;
-  if (int_resid && (!a->e_scale_in || !a->e_scale_out)) return CARRY_GDN_ERR_NULL;
-
-  carry::KParams p = {};
-  p.packed = 0;
-  p.B = a->B; p.H = a->HV; p.HV = a->HV; p.K = a->K; p.V = a->V;
-  p.qmax = a->qmax;
-  p.inv_qmax = 1.0f / a->qmax;
-  p.res_fmt = a->res_fmt; p.rscale_mode = a->resid_scale_mode; p.sscale_mode = a->state_scale_mode;
-  p.eps_mode = a->eps_mode;
-  p.qkv_dtype = a->qkv_dtype; p.o_dtype = a->o_dtype;
-  p.status = a->status;
-  p.codes_in = a->h_in; p.codes_out = a->h_out;
-  p.sscale_in = a->scale_in; p.sscale_out = a->scale_out;
-  p.resid_in = a->e_in; p.resid_out = a->e_out;
-  p.rscale_in = a->e_scale_in; p.rscale_out = a->e_scale_out;
-  p.q = a->q; p.k = a->k; p.v = a->v;
-  p.alpha = a->alpha; p.beta = a->beta;
-  p.qscale = 1.0f;
-  p.out = a->o;
+  carry::KParams p;
+  const int rc = carry::step_params(a, p);
+  if (rc != CARRY_GDN_OK || (long long)a->B * a->HV == 0) return rc;
   return dispatch(p, static_cast<cudaStream_t>(stream));
+}
+
+int carry_gdn_quant_decode(const CarryGdnDecodeArgs* a, void* stream) {
+  clear_stale_error();
+  if (!a) return CARRY_GDN_ERR_NULL;
+  if (a->T < 1) return CARRY_GDN_ERR_SHAPE;
+  CarryGdnStepArgs st = a->step;                          // the state comes from h0: in place from there on
+  st.h_in = st.h_out; st.scale_in = st.scale_out; st.e_in = st.e_out; st.e_scale_in = st.e_scale_out;
+  carry::KParams p;
+  const int rc = carry::step_params(&st, p);
+  if (rc != CARRY_GDN_OK || (long long)st.B * st.HV == 0) return rc;
+  if (!a->h0) return CARRY_GDN_ERR_NULL;
+  if (!carry::chain_eligible(p, a->h0)) return CARRY_GDN_ERR_UNSUPPORTED;
+  const int rc2 = carry::launch_chain(p, a->h0, a->T, static_cast<cudaStream_t>(stream));
+  if (rc2 == CARRY_GDN_OK) g_last_kernel = 7;
+  return rc2;
 }
 
 int carry_gdn_fp32_step(const CarryGdnFp32Args* a, void* stream) {

@@ -218,6 +218,8 @@ int launch_generic(const KParams& p, cudaStream_t stream);
 int launch_fp32(const CarryGdnFp32Args& a, cudaStream_t stream);
 bool tile128_eligible(const KParams& p);
 int launch_tile128(const KParams& p, cudaStream_t stream);
+bool chain_eligible(const KParams& p, const float* h0);
+int launch_chain(const KParams& p, const float* h0, int T, cudaStream_t stream);
 int launch_multi(const KParams& p, int T, long long stride_mixed_t, long long stride_a_t, long long stride_b_t,
                  cudaStream_t stream);
 bool narrow64_eligible(const KParams& p);

@@ -36,8 +36,9 @@ struct Table {
   int (*pool_copy)(const CarryGdnPoolCopyArgs*, void*);
   int (*pool_copy_layers)(const CarryGdnPoolCopyLayersArgs*, void*);
   int (*write_ids)(int32_t*, const int32_t*, int32_t, void*);
+  int (*quant_decode)(const CarryGdnDecodeArgs*, void*);
 };
-constexpr int kEntries = 9;
+constexpr int kEntries = 10;
 
 const Table* table_of(PyObject* o) { return static_cast<const Table*>(PyLong_AsVoidPtr(o)); }
 
@@ -357,6 +358,51 @@ PyObject* quant_decode(PyObject*, PyObject* const* o, Py_ssize_t n) {
   return r;
 }
 
+// The same from a floating-point state, all in one launch, for what the library's chain kernel takes.
+// (table, h0, q, k, v, alpha, beta, T, bits, res_fmt) -> (o [T, B, HV, V], h_int8, scale, e)
+PyObject* quant_chain(PyObject*, PyObject* const* o, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    if (n != 10) return nullptr;
+    const Table* tab = table_of(o[0]);
+    const at::Tensor* h0 = plain(o[1]);
+    long T, bits, fmt;
+    if (!tab || !as_int(o[7], T) || !as_int(o[8], bits) || !as_int(o[9], fmt) || !fits32(T)) return nullptr;
+    if (!h0 || h0->dim() != 4 || !h0->is_cuda() || !h0->is_contiguous() || h0->scalar_type() != at::kFloat) return nullptr;
+    // what the kernel takes, looked at before anything is allocated
+    if (fmt < CARRY_RES_FP32 || fmt > CARRY_RES_FP8 || bits < 3 || bits > 8 || h0->size(2) != 128 || h0->size(3) != 128) return nullptr;
+    const int dev = h0->get_device();
+    const int64_t B = h0->size(0), HV = h0->size(1), K = 128, V = 128;
+    if (!fits32(B) || !fits32(HV)) return nullptr;
+    static const at::ScalarType kinds[] = {at::kFloat, at::kHalf, at::kFloat8_e5m2};
+    const at::Tensor *q = plain(o[2]), *k = plain(o[3]), *v = plain(o[4]), *alpha = plain(o[5]), *beta = plain(o[6]);
+    CarryGdnDecodeArgs a = {};
+    CarryGdnStepArgs& p = a.step;
+    p.qkv_dtype = activations(q, k, v, alpha, beta, dev);
+    if (p.qkv_dtype < 0 || q->dim() != 4 || k->dim() != 4 || v->dim() != 4 || alpha->dim() != 3 || beta->dim() != 3) return nullptr;
+    for (const at::Tensor* t : {q, k, v, alpha, beta})
+      if (t->size(0) < T || t->size(1) != B || t->size(2) != HV) return nullptr;
+    if (q->size(3) != K || k->size(3) != K || v->size(3) != V) return nullptr;
+    const at::Tensor out = fresh({T, B, HV, V}, at::kFloat, dev), h = fresh({B, HV, K, V}, at::kChar, dev);
+    const at::Tensor scale = fresh({B, HV, V}, at::kFloat, dev), e = fresh({B, HV, K, V}, kinds[fmt], dev);
+    a.h0 = static_cast<const float*>(h0->data_ptr());
+    a.T = static_cast<int32_t>(T);
+    p.q = q->data_ptr(); p.k = k->data_ptr(); p.v = v->data_ptr();
+    p.alpha = static_cast<const float*>(alpha->data_ptr()); p.beta = static_cast<const float*>(beta->data_ptr());
+    p.o = out.data_ptr();
+    p.h_out = static_cast<int8_t*>(h.data_ptr());
+    p.scale_out = static_cast<float*>(scale.data_ptr());
+    p.e_out = e.data_ptr();
+    p.B = static_cast<int32_t>(B); p.HV = static_cast<int32_t>(HV); p.K = K; p.V = V;
+    p.o_dtype = CARRY_F32;
+    p.qmax = static_cast<float>((1 << (bits - 1)) - 1);
+    p.res_fmt = static_cast<int32_t>(fmt);
+    p.resid_scale_mode = p.state_scale_mode = CARRY_SCALE_PER_V;
+    p.eps_mode = CARRY_EPS_ON_AMAX;
+    if (!launch(dev, [&](void* s) { return tab->quant_decode(&a, s); })) return nullptr;
+    return tuple_of({&out, &h, &scale, &e});
+  });
+}
+
 // (table, h, q, k, v, alpha, beta) -> (h_out, o)
 PyObject* fp32_step(PyObject*, PyObject* const* o, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
@@ -555,7 +601,7 @@ PyObject* make_table(PyObject*, PyObject* const* o, Py_ssize_t n) {
 }
 
 #define CARRY_FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {CARRY_FAST(make_table), CARRY_FAST(packed_decode), CARRY_FAST(quant_step), CARRY_FAST(quant_decode),
+PyMethodDef methods[] = {CARRY_FAST(make_table), CARRY_FAST(packed_decode), CARRY_FAST(quant_step), CARRY_FAST(quant_decode), CARRY_FAST(quant_chain),
                          CARRY_FAST(fp32_step), CARRY_FAST(pool_move), CARRY_FAST(pool_copy), CARRY_FAST(pool_copy_layers),
                          CARRY_FAST(ids_tensor), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", "Native call path of the Python surfaces.", -1, methods};

@@ -285,8 +285,12 @@ def gdn_quant_decode_fused(h0, q, k, v, alpha, beta, T, bits: int = 8,
     """T chained fused steps.  ``h0 [B, HV, K, V]`` fp32; ``q/k [T, B, HV, K]``,
     ``v [T, B, HV, V]``, ``alpha/beta [T, B, HV]``.  Returns
     ``(o [T, B, HV, V], h_int8, scale, e, e_scale)``."""
-    h_int8, scale, e, e_scale = init_quant_state(h0, bits, res_fmt, resid_scale, state_scale)
     lib = _lib._lib or _lib.load_library()
+    if resid_scale in _SCALE_MODE and state_scale == "v":
+        made = lib.native.quant_chain(lib.native_table, h0, q, k, v, alpha, beta, T, bits, res_fmt)
+        if made is not None:
+            return (*made, None)
+    h_int8, scale, e, e_scale = init_quant_state(h0, bits, res_fmt, resid_scale, state_scale)
     # the state is this call's own: all steps in place, launched back to back
     o = lib.native.quant_decode(lib.native_table, h_int8, scale, e, e_scale, q, k, v, alpha, beta, T, bits, res_fmt,
                                 resid_scale == "v", state_scale == "v")

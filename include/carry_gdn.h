@@ -101,6 +101,23 @@ typedef struct CarryGdnStepArgs {
 int carry_gdn_quant_step(const CarryGdnStepArgs* args, void* stream);
 
 /*
+ * T chained steps from a floating-point state, in one call: h0 [B, HV, K, V] fp32 is quantised (scale =
+ * max(amax_K |h0|, 1e-12) * (1 / qmax), codes = round_half_even(h0 / scale), zero residual), then every request's
+ * token t = 0 .. T-1 is applied as carry_gdn_quant_step would.  Replaces the loop of statequant/kernel.py:435-452.
+ * `step` gives the formats, the sizes and the final state's buffers (h_out, scale_out, e_out); its *_in pointers are
+ * not read.  q, k, v, alpha, beta and o carry T in front: [T, B, HV, ...].  Only what the one-launch kernel takes is
+ * supported (K = V = 128, a floating-point residual, per-V state scales); anything else returns
+ * CARRY_GDN_ERR_UNSUPPORTED and the caller loops over tokens.
+ */
+typedef struct CarryGdnDecodeArgs {
+  CarryGdnStepArgs step;
+  const float* h0;
+  int32_t T;
+} CarryGdnDecodeArgs;
+
+int carry_gdn_quant_decode(const CarryGdnDecodeArgs* args, void* stream);
+
+/*
  * Unquantised fp32 step, state [B, HV, K, V] fp32.  Replaces
  * ext.gdn_fp32_step (cuda/gdn_state_kernel.cu:350-371) and
  * statequant/kernel.py:411-433.  h_out may alias h_in.
@@ -320,7 +337,7 @@ int carry_gdn_abi_version(void);
  * 0 = none yet, 1 = generic tile kernel, 2 = 128x128 streaming kernel,
  * 3 = multi-token kernel, 4 = a pool store / load / copy kernel,
  * 5 = 128x128 streaming kernel, step without error feedback,
- * 6 = slot-indexed kernel for 64x64 heads.
+ * 6 = slot-indexed kernel for 64x64 heads, 7 = kernel of chained steps.
  * Diagnostic only (tests use it to prove which path ran).
  */
 int carry_gdn_last_kernel(void);
