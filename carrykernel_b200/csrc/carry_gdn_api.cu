@@ -24,6 +24,11 @@ int dispatch(const carry::KParams& p, cudaStream_t stream) {
     if (rc == CARRY_GDN_OK) g_last_kernel = 6;
     return rc;
   }
+  if (carry::dense64_eligible(p)) {
+    const int rc = carry::launch_dense64(p, stream);
+    if (rc == CARRY_GDN_OK) g_last_kernel = 8;
+    return rc;
+  }
   const int rc = carry::launch_generic(p, stream);
   if (rc == CARRY_GDN_OK) g_last_kernel = 1;
   return rc;

@@ -218,6 +218,10 @@ int launch_generic(const KParams& p, cudaStream_t stream);
 int launch_fp32(const CarryGdnFp32Args& a, cudaStream_t stream);
 bool tile128_eligible(const KParams& p);
 int launch_tile128(const KParams& p, cudaStream_t stream);
+bool dense64_eligible(const KParams& p);
+int launch_dense64(const KParams& p, cudaStream_t stream);
+bool fp32_64_eligible(const CarryGdnFp32Args& a);
+int launch_fp32_64(const CarryGdnFp32Args& a, cudaStream_t stream);
 bool chain_eligible(const KParams& p, const float* h0);
 int launch_chain(const KParams& p, const float* h0, int T, cudaStream_t stream);
 int launch_multi(const KParams& p, int T, long long stride_mixed_t, long long stride_a_t, long long stride_b_t,

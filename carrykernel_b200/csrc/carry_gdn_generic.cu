@@ -334,6 +334,7 @@ int launch_generic(const KParams& p, cudaStream_t stream) {
 int launch_fp32(const CarryGdnFp32Args& a, cudaStream_t stream) {
   const long long all_tiles = (long long)a.B * a.HV;
   if (all_tiles == 0) return CARRY_GDN_OK;
+  if (fp32_64_eligible(a)) return launch_fp32_64(a, stream);
   if (a.K == kF && a.V == kF && ((uintptr_t)a.h_in % 16) == 0 && ((uintptr_t)a.h_out % 16) == 0) {
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

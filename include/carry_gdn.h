@@ -337,7 +337,8 @@ int carry_gdn_abi_version(void);
  * 0 = none yet, 1 = generic tile kernel, 2 = 128x128 streaming kernel,
  * 3 = multi-token kernel, 4 = a pool store / load / copy kernel,
  * 5 = 128x128 streaming kernel, step without error feedback,
- * 6 = slot-indexed kernel for 64x64 heads, 7 = kernel of chained steps.
+ * 6 = slot-indexed kernel for 64x64 heads, 7 = kernel of chained steps,
+ * 8 = statequant-layout kernel for 64x64 heads.
  * Diagnostic only (tests use it to prove which path ran).
  */
 int carry_gdn_last_kernel(void);
