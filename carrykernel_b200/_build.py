@@ -27,7 +27,8 @@ NATIVE = os.path.join(PKG, "_native.so")
 NATIVE_SOURCE = "host_native.cpp"
 SOURCES = ("carry_gdn_api.cu", "carry_gdn_generic.cu", "carry_gdn_tile128.cu",
            "carry_gdn_tile128_vk.cu", "carry_gdn_tile128_kv.cu", "carry_gdn_multi.cu",
-           "carry_gdn_pool.cu", "carry_gdn_narrow.cu", "carry_gdn_chain.cu", "carry_gdn_dense64.cu")
+           "carry_gdn_pool.cu", "carry_gdn_narrow.cu", "carry_gdn_chain.cu", "carry_gdn_dense64.cu",
+           "carry_gdn_dense128.cu")
 HEADERS = ("carry_gdn_common.cuh", "carry_gdn_tile128.cuh", "carry_gdn_slot_tile.inc", os.path.join("..", "..", "include", "carry_gdn.h"))
 NVCC_FLAGS = ("-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xptxas", "-v", "-Xcompiler", "-fPIC")
@@ -75,8 +76,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
     obj_dir = os.path.join(root, "build", "obj")
     os.makedirs(obj_dir, exist_ok=True)
 
-    # the sources whose code differs in the test-only twin (the streaming and multi-token kernels)
-    twin_sources = ("carry_gdn_tile128_vk.cu", "carry_gdn_tile128_kv.cu", "carry_gdn_multi.cu")
+    # the sources whose code differs in the test-only twin (the kernels that wait for bulk copies)
+    twin_sources = ("carry_gdn_tile128_vk.cu", "carry_gdn_tile128_kv.cu", "carry_gdn_multi.cu", "carry_gdn_dense128.cu")
 
     def compile_one(job):
         src, twin = job

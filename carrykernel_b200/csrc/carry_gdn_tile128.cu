@@ -6,13 +6,15 @@ namespace carry {
 
 int launch_tile128_vk(const KParams& p, cudaStream_t stream, int sms);
 int launch_tile128_kv(const KParams& p, cudaStream_t stream, int sms);
+int launch_dense128(const KParams& p, cudaStream_t stream, int sms);
 
 namespace {
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 }  // namespace
 
-// The streaming kernel needs K = V = 128, an integer residual (any residual format, or none, in the statequant
-// layout), a per-V state scale (or none and either granularity), qmax = 2^(bits-1) - 1 for 3..8 bits, and 16-byte aligned, dense rows for every bulk copy.
+// The streaming kernels need K = V = 128, an integer residual (any residual format, or none, in the statequant
+// layout), a per-V state scale (or none and either granularity), qmax = 2^(bits-1) - 1 for 3..8 bits, and 16-byte
+// aligned, dense rows for every bulk copy.
 bool tile128_eligible(const KParams& p) {
   if (p.K != 128 || p.V != 128) return false;
   const bool int_resid = p.res_fmt == CARRY_RES_INT8 || p.res_fmt == CARRY_RES_INT4;
@@ -26,9 +28,11 @@ bool tile128_eligible(const KParams& p) {
     return false;
   if (p.HV > 128 || (long long)p.B * p.HV > 0x7fffffffLL) return false;
   const int qes = p.qkv_dtype == CARRY_F32 ? 4 : 2;
+  // one residual scale per head: the slot layout copies the 16 bytes around it, the statequant layout reads it as it is
+  const bool copied_rscale = int_resid && (p.packed || p.rscale_mode == CARRY_SCALE_PER_V);
   if (!aligned16(p.codes_in) || !aligned16(p.codes_out) || (!no_resid && (!aligned16(p.resid_in) || !aligned16(p.resid_out))) ||
       (p.sscale_mode == CARRY_SCALE_PER_V && (!aligned16(p.sscale_in) || !aligned16(p.sscale_out))) ||
-      (int_resid && (!aligned16(p.rscale_in) || !aligned16(p.rscale_out))) ||
+      (copied_rscale && (!aligned16(p.rscale_in) || !aligned16(p.rscale_out))) ||
       !aligned16(p.q) || !aligned16(p.k) || !aligned16(p.v) || !aligned16(p.out))
     return false;
   if (p.packed) {
@@ -36,8 +40,6 @@ bool tile128_eligible(const KParams& p) {
     if (p.stride_state_slot % 16 || p.stride_resid_slot % 16 || p.stride_sscale_slot % 4) return false;
     if (p.rscale_mode == CARRY_SCALE_PER_V ? (p.stride_rscale_slot % 4) : (p.stride_rscale_slot % 4 || p.HV % 4))
       return false;
-  } else {
-    if (int_resid && p.rscale_mode == CARRY_SCALE_PER_HEAD && p.HV % 4) return false;
   }
   return true;
 }
@@ -56,7 +58,10 @@ int launch_tile128(const KParams& p, cudaStream_t stream) {
   }
   KParams q = p;
   fill_shifts(q);
-  return q.packed ? launch_tile128_vk(q, stream, sms[dev]) : launch_tile128_kv(q, stream, sms[dev]);
+  if (q.packed) return launch_tile128_vk(q, stream, sms[dev]);
+  const bool float_resid = q.res_fmt == CARRY_RES_FP32 || q.res_fmt == CARRY_RES_FP16 || q.res_fmt == CARRY_RES_FP8;
+  // A floating-point residual needs a stage of up to 82 KB: no room for two CTAs, so it stays with one of two groups.
+  return float_resid ? launch_tile128_kv(q, stream, sms[dev]) : launch_dense128(q, stream, sms[dev]);
 }
 
 }  // namespace carry

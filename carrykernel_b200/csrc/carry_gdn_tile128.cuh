@@ -1,5 +1,6 @@
 // Streaming kernel for the serving shape: K = V = 128, int8 state, int8 or packed
-// int4 residual.  One (request, head) tile is 16 KB of codes + 8/16 KB of
+// int4 residual in the slot layout, a floating-point residual in the statequant
+// layout (carry_gdn_dense128.cu has that layout's other formats).  One (request, head) tile is 16 KB of codes + 8/16 KB of
 // residual; all of it is contiguous in memory in both layouts, so every tile
 // moves with a handful of 1-D bulk async copies (TMA, no tensor map):
 //
@@ -24,7 +25,7 @@
 //     the next tile).
 //   * statequant layout [K][V] (scale per column): lane = 4 contiguous columns
 //     x the warp's 16 rows; column sums are finished across the 8 warps through
-//     shared memory (three meetings per tile).  Here a step may also have no residual at all.
+//     shared memory (three meetings per tile).
 //
 // Arithmetic.  Everything that feeds a state code keeps the reference's operation
 // order, with the contractions written out as explicit fused multiply-adds:
@@ -359,18 +360,15 @@ struct StageLayout {
   static constexpr int kVecBytes = kT * (QDT == CARRY_F32 ? 4 : 2);
   // integer residuals carry a scale (per V or per head); the float ones (fp32, fp16, fp8-e5m2) do not
   static constexpr bool kFloatResid = RES == CARRY_RES_FP32 || RES == CARRY_RES_FP16 || RES == CARRY_RES_FP8;
-  static constexpr bool kNoResid = RES == CARRY_RES_NONE;     // statequant layout only; RSCALE then says how the STATE is scaled
-  static constexpr bool kHeadState = kNoResid && RSCALE == CARRY_SCALE_PER_HEAD;
-  static constexpr int kResidBytes = kNoResid ? 0 : (RES == CARRY_RES_INT4) ? kT * kT / 2
+  static constexpr int kResidBytes = (RES == CARRY_RES_INT4) ? kT * kT / 2
                                      : (RES == CARRY_RES_FP32) ? kT * kT * 4
                                      : (RES == CARRY_RES_FP16) ? kT * kT * 2 : kT * kT;
   static constexpr int kCodes = 0;
   static constexpr int kResid = kT * kT;
   static constexpr int kSScale = kResid + kResidBytes;       // 128 floats
   static constexpr int kRScale = kSScale + 512;              // 128 floats (per V), or the 16 bytes that hold
-  static constexpr int kSScaleBytes = kHeadState ? 0 : 512;  // one scale per head comes with the tile's facts (TileMeta::k_mul)
-  static constexpr int kRScaleBytes = (kFloatResid || kNoResid) ? 0 : (RSCALE == CARRY_SCALE_PER_V) ? 512 : 16;   // this head's scale (per head)
-  static constexpr int kQ = kRScale + ((kFloatResid || kNoResid) ? 0 : (RSCALE == CARRY_SCALE_PER_V) ? 512 : 128);   // raw q, k, v of this head
+  static constexpr int kRScaleBytes = kFloatResid ? 0 : (RSCALE == CARRY_SCALE_PER_V) ? 512 : 16;   // this head's scale (per head)
+  static constexpr int kQ = kRScale + (kFloatResid ? 0 : (RSCALE == CARRY_SCALE_PER_V) ? 512 : 128);   // raw q, k, v of this head
   static constexpr int kK = kQ + kVecBytes;
   static constexpr int kV = kK + kVecBytes;
   static constexpr int kBytes = kV + kVecBytes;
@@ -478,9 +476,7 @@ __device__ __forceinline__ GateRaw gate_loads(const KParams& p, int n, int hv, l
     const long long nh = (long long)n * p.HV + hv;
     r.a = __float_as_uint(__ldcg(p.alpha + nh + tok_a));
     r.b = __float_as_uint(__ldcg(p.beta + nh + tok_b));
-    // a state scaled per head brings its scale along here
-    r.A_log = p.sscale_mode == CARRY_SCALE_PER_HEAD ? __float_as_uint(__ldcg(p.sscale_in + nh)) : __float_as_uint(1.0f);
-    r.dt_bias = 0u;
+    r.A_log = r.dt_bias = 0u;
   }
   return r;
 }
@@ -505,8 +501,7 @@ __device__ __forceinline__ void split_tile(const KParams& p, int tile, int& n, i
 struct __align__(16) TileMeta {
   int n, hv, slot;
   float alpha, beta;
-  float k_mul, q_mul;   // 1/|k| and scale/|q| (1 when the L2 norm is off); statequant path: the state's scale
-                        // where it has one per head, else 1, and 1
+  float k_mul, q_mul;   // 1/|k| and scale/|q| (1 when the L2 norm is off; statequant path: 1)
   float kq;             // <k, q> after those factors
 };
 static_assert(sizeof(TileMeta) == 32, "TileMeta is read as two 16-byte words");
@@ -527,7 +522,6 @@ __device__ __forceinline__ void tile_addresses(const KParams& p, int n, int hv, 
   constexpr long long KV = kT * kT;
   constexpr long long RB = (RES == CARRY_RES_INT4) ? KV / 2 : (RES == CARRY_RES_FP32) ? 4 * KV
                            : (RES == CARRY_RES_FP16) ? 2 * KV : KV;
-  constexpr bool head_state = RES == CARRY_RES_NONE && RSCALE == CARRY_SCALE_PER_HEAD;
   const long long nh = (long long)n * p.HV + hv;
   if (p.packed) {
     a[D_CODES] = reinterpret_cast<unsigned long long>(p.codes_out + slot * p.stride_state_slot + hv * KV);
@@ -543,7 +537,7 @@ __device__ __forceinline__ void tile_addresses(const KParams& p, int n, int hv, 
   } else {
     a[D_CODES] = reinterpret_cast<unsigned long long>(p.codes_out + nh * KV);
     a[D_RESID] = reinterpret_cast<unsigned long long>(reinterpret_cast<uint8_t*>(p.resid_out) + nh * RB);
-    a[D_SSCALE] = reinterpret_cast<unsigned long long>(p.sscale_out + (head_state ? nh : nh * kT));
+    a[D_SSCALE] = reinterpret_cast<unsigned long long>(p.sscale_out + nh * kT);
     a[D_RSCALE] = reinterpret_cast<unsigned long long>(p.rscale_out + (RSCALE == CARRY_SCALE_PER_V ? nh * kT : nh));
     a[D_RSCALE_IN] = reinterpret_cast<unsigned long long>(p.rscale_in + (RSCALE == CARRY_SCALE_PER_V ? nh * kT : (nh & ~3LL)));
     a[D_Q] = reinterpret_cast<unsigned long long>(reinterpret_cast<const uint8_t*>(p.q) + nh * kT * qes);
@@ -691,7 +685,6 @@ __device__ __forceinline__ void meta_math(const KParams& p, const MetaRaw<QDT, L
     m.q_mul *= p.qscale;
   }
   m.kq = kqsum * (m.k_mul * m.q_mul);
-  if (!p.packed) m.k_mul = __uint_as_float(r.g.A_log);
 }
 // A slot id beyond the pool is treated as padding (and reported by meta_put); the tile's addresses follow
 // from the slot id that is left.  No side effects: this, too, can run ahead of the dependency wait.
@@ -747,10 +740,10 @@ __device__ __forceinline__ void issue_copies(const KParams& p, uint8_t* sb, uint
   const long long d_codes = reinterpret_cast<const uint8_t*>(p.codes_in) - reinterpret_cast<const uint8_t*>(p.codes_out);
   const long long d_resid = reinterpret_cast<const uint8_t*>(p.resid_in) - reinterpret_cast<const uint8_t*>(p.resid_out);
   const long long d_sscale = reinterpret_cast<const uint8_t*>(p.sscale_in) - reinterpret_cast<const uint8_t*>(p.sscale_out);
-  mbar_arrive_expect_tx(bar, kT * kT + L::kResidBytes + L::kSScaleBytes + rscale_bytes + 3 * L::kVecBytes + test_extra_tx(tile));
+  mbar_arrive_expect_tx(bar, kT * kT + L::kResidBytes + 512 + rscale_bytes + 3 * L::kVecBytes + test_extra_tx(tile));
   bulk_load(sb + L::kCodes, reinterpret_cast<const void*>(a[D_CODES] + d_codes), kT * kT, bar);
-  if constexpr (L::kResidBytes > 0) bulk_load(sb + L::kResid, reinterpret_cast<const void*>(a[D_RESID] + d_resid), L::kResidBytes, bar);
-  if constexpr (L::kSScaleBytes > 0) bulk_load(sb + L::kSScale, reinterpret_cast<const void*>(a[D_SSCALE] + d_sscale), L::kSScaleBytes, bar);
+  bulk_load(sb + L::kResid, reinterpret_cast<const void*>(a[D_RESID] + d_resid), L::kResidBytes, bar);
+  bulk_load(sb + L::kSScale, reinterpret_cast<const void*>(a[D_SSCALE] + d_sscale), 512, bar);
   if constexpr (rscale_bytes > 0) bulk_load(sb + L::kRScale, reinterpret_cast<const void*>(a[D_RSCALE_IN]), rscale_bytes, bar);
   bulk_load(sb + L::kQ, reinterpret_cast<const void*>(a[D_Q]), L::kVecBytes, bar);
   bulk_load(sb + L::kK, reinterpret_cast<const void*>(a[D_K]), L::kVecBytes, bar);
@@ -870,8 +863,8 @@ gdn_tile128_kernel(const __grid_constant__ KParams p) {
           const long long d_resid = reinterpret_cast<const uint8_t*>(p.resid_in) - reinterpret_cast<const uint8_t*>(p.resid_out);
           const long long d_sscale = reinterpret_cast<const uint8_t*>(p.sscale_in) - reinterpret_cast<const uint8_t*>(p.sscale_out);
           l2_prefetch_bulk(reinterpret_cast<const void*>(a[D_CODES] + d_codes), kT * kT);
-          if constexpr (L::kResidBytes > 0) l2_prefetch_bulk(reinterpret_cast<const void*>(a[D_RESID] + d_resid), L::kResidBytes);
-          if constexpr (L::kSScaleBytes > 0) l2_prefetch_bulk(reinterpret_cast<const void*>(a[D_SSCALE] + d_sscale), L::kSScaleBytes);
+          l2_prefetch_bulk(reinterpret_cast<const void*>(a[D_RESID] + d_resid), L::kResidBytes);
+          l2_prefetch_bulk(reinterpret_cast<const void*>(a[D_SSCALE] + d_sscale), 512);
         }
       }
       meta_math<QDT, LPT>(p, before, m);
@@ -1049,13 +1042,8 @@ gdn_tile128_kernel(const __grid_constant__ KParams p) {
         // ---------------- statequant layout [K][V]: lane = 4 columns x 16 rows ----
         // columns {c0, c0+1} are held as pair A, {c0+2, c0+3} as pair B
         const int r0 = 16 * gw, c0 = 4 * lane;
-        // Reduction space, three units of [warp][col]: sums (two units), maxima, remainder maxima.  The last share a
-        // unit with the sums, which everybody has read by the second meeting; that the next tile's sums, written with
-        // no meeting in between, do not run into them, the units trade places from tile to tile.
-        const int odd = cnt & 1;
-        float* red_dot = col_red + odd * kWarps * kT;                   // [warp][col][2]
-        float* red_max = col_red + (odd ? 0 : 2) * kWarps * kT;         // [warp][col]
-        float* red_emax = col_red + (odd ? 2 : 0) * kWarps * kT;        // [warp][col]
+        float* red_dot = col_red;                                       // [warp][col][2]
+        float* red_max = col_red + 2 * kWarps * kT;                     // [warp][col]
         // k and q of this warp's 16 rows are the same in every lane.  One lane per value turns them to fp32 and
         // writes each twice, side by side, so that a row's {k, k} and {q, q} are one broadcast load that feeds packed
         // instructions as it is (three loads, three conversions and the register moves to pair a scalar up, per row,
@@ -1065,33 +1053,22 @@ gdn_tile128_kernel(const __grid_constant__ KParams p) {
           const float x = act<QDT>(sb + (lane < 16 ? L::kK : L::kQ), r0 + (lane & 15));
           *reinterpret_cast<float2*>(reinterpret_cast<float*>(kq_row + (lane & 15)) + (lane < 16 ? 0 : 2)) = splat(x);
         }
-        float scol[4];
-        if constexpr (L::kHeadState) {
-          scol[0] = scol[1] = scol[2] = scol[3] = k_mul;
-        } else {
-          const float4 s4 = *reinterpret_cast<const float4*>(sscale + c0);
-          scol[0] = s4.x; scol[1] = s4.y; scol[2] = s4.z; scol[3] = s4.w;
-        }
-        // Int4 residual and no residual: the sums run over the bare codes, a column's scale * decay goes on the
-        // totals (see carry_gdn_slot_tile.inc on what that moves).  The other formats keep the reference's order.
-        constexpr bool kFold = RES == CARRY_RES_INT4 || L::kNoResid;
-        const float2 sA = make_float2(scol[0], scol[1]), sB = make_float2(scol[2], scol[3]);
-        const float2 saA = mul2(sA, alpha2), saB = mul2(sB, alpha2);
+        const float4 s4 = *reinterpret_cast<const float4*>(sscale + c0);
+        const float2 sA = make_float2(s4.x, s4.y), sB = make_float2(s4.z, s4.w);
         float2 hA[16], hB[16];
         float2 dkA = make_float2(0.f, 0.f), dkB = dkA, dqA = dkA, dqB = dkA;
         __syncwarp();
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           const uint32_t w = *reinterpret_cast<const uint32_t*>(sb + L::kCodes + (r0 + i) * kT + c0);
-          float2 a = s8x2_cvt<0, 1>(w), b = s8x2_to_float<2, 3>(w ^ 0x80808080u);
-          if constexpr (!kFold) { a = mul2(mul2(a, sA), alpha2); b = mul2(mul2(b, sB), alpha2); }
+          const float2 a = mul2(mul2(s8x2_cvt<0, 1>(w), sA), alpha2);
+          const float2 b = mul2(mul2(s8x2_to_float<2, 3>(w ^ 0x80808080u), sB), alpha2);
           hA[i] = a; hB[i] = b;
           const float4 kq4 = kq_row[i];
           const float2 kr = make_float2(kq4.x, kq4.y), qr = make_float2(kq4.z, kq4.w);
           dkA = fma2(a, kr, dkA); dkB = fma2(b, kr, dkB);
           dqA = fma2(a, qr, dqA); dqB = fma2(b, qr, dqB);
         }
-        if constexpr (kFold) { dkA = mul2(dkA, saA); dkB = mul2(dkB, saB); dqA = mul2(dqA, saA); dqB = mul2(dqB, saB); }
         // finish the column sums across the 8 warps
         float dk[4], dq[4];
         {
@@ -1109,51 +1086,29 @@ gdn_tile128_kernel(const __grid_constant__ KParams p) {
             dk[2] += x1.x; dq[2] += x1.y; dk[3] += x1.z; dq[3] += x1.w;
           }
         }
-        float dv[4], oval[4], es_col[4];
+        float dv[4], oval[4];
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
           dv[b] = __fmul_rn(beta, __fadd_rn(act<QDT>(sb + L::kV, c0 + b), -dk[b]));
           oval[b] = fmaf(dv[b], kq, dq[b]);
-          es_col[b] = (L::kFloatResid || L::kNoResid) ? 0.f : (RSCALE == CARRY_SCALE_PER_V) ? rscale[c0 + b] : es_head;
         }
         const float2 dvA = make_float2(dv[0], dv[1]), dvB = make_float2(dv[2], dv[3]);
-        const float2 esA = make_float2(es_col[0], es_col[1]), esB = make_float2(es_col[2], es_col[3]);
-        const float2 nbA = mul2(esA, splat(-136.0f)), nbB = mul2(esB, splat(-136.0f));
         float amax[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           const float2 kr = *reinterpret_cast<const float2*>(kq_row + i);
-          float2 tA, tB;
-          if constexpr (L::kNoResid) {
-            tA = fma2(hA[i], saA, mul2(kr, dvA)); tB = fma2(hB[i], saB, mul2(kr, dvB));
-          } else if constexpr (RES == CARRY_RES_INT4) {
-            // a nibble in offset binary lands in a float that reads 136 + code; 136 * es is in the innermost addend
-            const uint32_t w =
-                (uint32_t)(*reinterpret_cast<const uint16_t*>(sb + L::kResid + (r0 + i) * (kT / 2) + c0 / 2)) ^ 0x8888u;
-            const uint32_t lo = w & 0x0F0Fu, hi = (w >> 4) & 0x0F0Fu;
-            const float2 nA = make_float2(__uint_as_float(__byte_perm(lo, 0x43000000u, 0x7044)), __uint_as_float(__byte_perm(hi, 0x43000000u, 0x7044)));
-            const float2 nB = make_float2(__uint_as_float(__byte_perm(lo, 0x43000000u, 0x7144)), __uint_as_float(__byte_perm(hi, 0x43000000u, 0x7144)));
-            tA = fma2(nA, esA, fma2(hA[i], saA, fma2(kr, dvA, nbA)));
-            tB = fma2(nB, esB, fma2(hB[i], saB, fma2(kr, dvB, nbB)));
-          } else if constexpr (RES == CARRY_RES_INT8) {
-            const uint32_t w = *reinterpret_cast<const uint32_t*>(sb + L::kResid + (r0 + i) * kT + c0) ^ 0x80808080u;
-            tA = fma2(s8x2_to_float<0, 1>(w), esA, fma2(kr, dvA, hA[i]));
-            tB = fma2(s8x2_to_float<2, 3>(w), esB, fma2(kr, dvB, hB[i]));
+          float2 eA, eB;
+          if constexpr (RES == CARRY_RES_FP32) {
+            const float4 e4 = *reinterpret_cast<const float4*>(sb + L::kResid + ((r0 + i) * kT + c0) * 4);
+            eA = make_float2(e4.x, e4.y); eB = make_float2(e4.z, e4.w);
+          } else if constexpr (RES == CARRY_RES_FP16) {
+            const uint2 e2 = *reinterpret_cast<const uint2*>(sb + L::kResid + ((r0 + i) * kT + c0) * 2);
+            eA = __half22float2(*reinterpret_cast<const __half2*>(&e2.x));
+            eB = __half22float2(*reinterpret_cast<const __half2*>(&e2.y));
           } else {
-            float2 eA, eB;
-            if constexpr (RES == CARRY_RES_FP32) {
-              const float4 e4 = *reinterpret_cast<const float4*>(sb + L::kResid + ((r0 + i) * kT + c0) * 4);
-              eA = make_float2(e4.x, e4.y); eB = make_float2(e4.z, e4.w);
-            } else if constexpr (RES == CARRY_RES_FP16) {
-              const uint2 e2 = *reinterpret_cast<const uint2*>(sb + L::kResid + ((r0 + i) * kT + c0) * 2);
-              eA = __half22float2(*reinterpret_cast<const __half2*>(&e2.x));
-              eB = __half22float2(*reinterpret_cast<const __half2*>(&e2.y));
-            } else {
-              e5m2x4_to_float(*reinterpret_cast<const uint32_t*>(sb + L::kResid + (r0 + i) * kT + c0), eA, eB);
-            }
-            tA = add2(fma2(kr, dvA, hA[i]), eA);
-            tB = add2(fma2(kr, dvB, hB[i]), eB);
+            e5m2x4_to_float(*reinterpret_cast<const uint32_t*>(sb + L::kResid + (r0 + i) * kT + c0), eA, eB);
           }
+          const float2 tA = add2(fma2(kr, dvA, hA[i]), eA), tB = add2(fma2(kr, dvB, hB[i]), eB);
           hA[i] = tA; hB[i] = tB;
           if (i & 1) {                                  // two rows per three-operand maximum
             amax[0] = fmaxf(fmaxf(amax[0], fabsf(hA[i - 1].x)), fabsf(tA.x)); amax[1] = fmaxf(fmaxf(amax[1], fabsf(hA[i - 1].y)), fabsf(tA.y));
@@ -1173,8 +1128,6 @@ gdn_tile128_kernel(const __grid_constant__ KParams p) {
           amax[2] = fmaxf(amax[2], x.z); amax[3] = fmaxf(amax[3], x.w);
         }
         float snew[4], thr[4];
-        if constexpr (L::kHeadState)                      // every warp holds all 128 column maxima
-          amax[0] = amax[1] = amax[2] = amax[3] = warp_max_nonneg(fmaxf(fmaxf(amax[0], amax[1]), fmaxf(amax[2], amax[3])));
 #pragma unroll
         for (int b = 0; b < 4; ++b) { snew[b] = scale_fast(amax[b], p.qmax, rqmax_state, p.eps_mode); thr[b] = snew[b] * kTieGuard; }
         const float2 invA = make_float2(rcp_refined(snew[0]), rcp_refined(snew[1]));
@@ -1211,94 +1164,28 @@ gdn_tile128_kernel(const __grid_constant__ KParams p) {
 #pragma unroll
           for (int i = 0; i < 16; ++i) stg_b32(dst_codes + (r0 + i) * kT + c0, cw[i]);
         }
-        if constexpr (L::kNoResid) {
-          if (lane == 0) claim_next(cnt);                 // the meeting only hands the stage on
-          warps_meet(bar0 + 3);
-          refill_stage(it);
-          if constexpr (L::kHeadState) {
-            if (gtid == 0) stg_b32(dst_of(D_SSCALE), __float_as_uint(snew[0]));
-          } else if ((lane >> 2) == gw) {
-            stg_v4(dst_of(D_SSCALE) + c0 * 4, make_uint4(__float_as_uint(snew[0]), __float_as_uint(snew[1]),
-                                                         __float_as_uint(snew[2]), __float_as_uint(snew[3])));
-          }
-        } else if constexpr (L::kFloatResid) {
-          // the new residual is stored as it is, in its format; the meeting only hands the stage on
-          if (lane == 0) claim_next(cnt);
-          warps_meet(bar0 + 3);
-          refill_stage(it);
-          const unsigned long long dst_resid = dst_of(D_RESID);
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            if constexpr (RES == CARRY_RES_FP32) {
-              stg_v4(dst_resid + ((r0 + i) * kT + c0) * 4,
-                     make_uint4(__float_as_uint(hA[i].x), __float_as_uint(hA[i].y), __float_as_uint(hB[i].x),
-                                __float_as_uint(hB[i].y)));
-            } else if constexpr (RES == CARRY_RES_FP16) {
-              const __half2 a2 = __floats2half2_rn(hA[i].x, hA[i].y), b2 = __floats2half2_rn(hB[i].x, hB[i].y);
-              stg_v2_at<0>(dst_resid + ((r0 + i) * kT + c0) * 2,
-                           make_uint2(*reinterpret_cast<const uint32_t*>(&a2), *reinterpret_cast<const uint32_t*>(&b2)));
-            } else {
-              stg_b32(dst_resid + (r0 + i) * kT + c0, float4_to_e5m2x4(hA[i], hB[i]));
-            }
-          }
-          if ((lane >> 2) == gw)
-            stg_v4(dst_of(D_SSCALE) + c0 * 4, make_uint4(__float_as_uint(snew[0]), __float_as_uint(snew[1]),
-                                                         __float_as_uint(snew[2]), __float_as_uint(snew[3])));
-        } else {
-        float esn[4];
-        if constexpr (RSCALE == CARRY_SCALE_PER_V) {
-          *reinterpret_cast<float4*>(red_emax + (size_t)gw * kT + c0) =
-              make_float4(eamax[0], eamax[1], eamax[2], eamax[3]);
-          if (lane == 0) claim_next(cnt);
-          warps_meet(bar0 + 3);
-          refill_stage(it);
-#pragma unroll
-          for (int w = 0; w < kWarps; ++w) {
-            const float4 x = *reinterpret_cast<const float4*>(red_emax + (size_t)w * kT + c0);
-            eamax[0] = fmaxf(eamax[0], x.x); eamax[1] = fmaxf(eamax[1], x.y);
-            eamax[2] = fmaxf(eamax[2], x.z); eamax[3] = fmaxf(eamax[3], x.w);
-          }
-#pragma unroll
-          for (int b = 0; b < 4; ++b) esn[b] = scale_fast(eamax[b], rqmax, rrqmax, p.eps_mode);
-        } else {
-          float m = warp_max_nonneg(fmaxf(fmaxf(eamax[0], eamax[1]), fmaxf(eamax[2], eamax[3])));
-          if (lane == 0) { head_red[grp][cnt & 1][gw] = m; claim_next(cnt); }
-          warps_meet(bar0 + 3);
-          refill_stage(it);
-          m = head_red[grp][cnt & 1][0];
-#pragma unroll
-          for (int w = 1; w < kWarps; ++w) m = fmaxf(m, head_red[grp][cnt & 1][w]);
-          esn[0] = esn[1] = esn[2] = esn[3] = scale_fast(m, rqmax, rrqmax, p.eps_mode);
-        }
-        const float2 ieA = make_float2(rcp_refined(esn[0]), rcp_refined(esn[1]));
-        const float2 ieB = make_float2(rcp_refined(esn[2]), rcp_refined(esn[3]));
+        // the new residual is stored as it is, in its format; the meeting only hands the stage on
+        if (lane == 0) claim_next(cnt);
+        warps_meet(bar0 + 3);
+        refill_stage(it);
         const unsigned long long dst_resid = dst_of(D_RESID);
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          const float2 rA = fma2(hA[i], ieA, magic2), rB = fma2(hB[i], ieB, magic2);
-          const uint32_t y0 = __float_as_uint(rA.x), y1 = __float_as_uint(rA.y);
-          const uint32_t y2 = __float_as_uint(rB.x), y3 = __float_as_uint(rB.y);
-          if constexpr (RES == CARRY_RES_INT4) {
-            // 16 * odd + even (+ 136: both nibbles offset by 8) in one float, whose low byte is the pair
-            const uint32_t p01 = __float_as_uint(fmaf(__fadd_rn(rA.y, -kMagicRound), 16.0f, __fadd_rn(rA.x, 136.0f)));
-            const uint32_t p23 = __float_as_uint(fmaf(__fadd_rn(rB.y, -kMagicRound), 16.0f, __fadd_rn(rB.x, 136.0f)));
-            const uint32_t v16 = __byte_perm(p01, p23, 0x0040) ^ 0x8888u;
-            stg_b16(dst_resid + (r0 + i) * (kT / 2) + c0 / 2, v16);
+          if constexpr (RES == CARRY_RES_FP32) {
+            stg_v4(dst_resid + ((r0 + i) * kT + c0) * 4,
+                   make_uint4(__float_as_uint(hA[i].x), __float_as_uint(hA[i].y), __float_as_uint(hB[i].x),
+                              __float_as_uint(hB[i].y)));
+          } else if constexpr (RES == CARRY_RES_FP16) {
+            const __half2 a2 = __floats2half2_rn(hA[i].x, hA[i].y), b2 = __floats2half2_rn(hB[i].x, hB[i].y);
+            stg_v2_at<0>(dst_resid + ((r0 + i) * kT + c0) * 2,
+                         make_uint2(*reinterpret_cast<const uint32_t*>(&a2), *reinterpret_cast<const uint32_t*>(&b2)));
           } else {
-            stg_b32(dst_resid + (r0 + i) * kT + c0, pack4(y0, y1, y2, y3));
+            stg_b32(dst_resid + (r0 + i) * kT + c0, float4_to_e5m2x4(hA[i], hB[i]));
           }
         }
-        // scales: every warp holds all 128 of them; warp w publishes its 16-column share
-        // (columns 16w..16w+15 are held by lanes 4w..4w+3)
-        if ((lane >> 2) == gw) {
+        if ((lane >> 2) == gw)
           stg_v4(dst_of(D_SSCALE) + c0 * 4, make_uint4(__float_as_uint(snew[0]), __float_as_uint(snew[1]),
                                                        __float_as_uint(snew[2]), __float_as_uint(snew[3])));
-          if (RSCALE == CARRY_SCALE_PER_V)
-            stg_v4(dst_of(D_RSCALE) + c0 * 4, make_uint4(__float_as_uint(esn[0]), __float_as_uint(esn[1]),
-                                                   __float_as_uint(esn[2]), __float_as_uint(esn[3])));
-        }
-        if (RSCALE == CARRY_SCALE_PER_HEAD && gtid == 0) stg_b32(dst_of(D_RSCALE), __float_as_uint(esn[0]));
-        }
       }
     }
     it = *reinterpret_cast<volatile int*>(&claimed[grp][cnt & 1]);   // written before this tile's last meeting
@@ -1361,19 +1248,17 @@ int launch_dtype(const KParams& p, cudaStream_t stream, int sms) {
 // all variants of one memory layout
 template <int LAYOUT>
 int launch_layout(const KParams& p, cudaStream_t stream, int sms) {
-  if constexpr (LAYOUT == LAYOUT_KV) {     // float residuals and none at all exist on the statequant surfaces only
-    if (p.res_fmt == CARRY_RES_NONE)
-      return p.sscale_mode == CARRY_SCALE_PER_V ? launch_dtype<LAYOUT, CARRY_RES_NONE, CARRY_SCALE_PER_V>(p, stream, sms)
-                                                : launch_dtype<LAYOUT, CARRY_RES_NONE, CARRY_SCALE_PER_HEAD>(p, stream, sms);
+  if constexpr (LAYOUT == LAYOUT_KV) {
     if (p.res_fmt == CARRY_RES_FP32) return launch_dtype<LAYOUT, CARRY_RES_FP32, CARRY_SCALE_PER_V>(p, stream, sms);
     if (p.res_fmt == CARRY_RES_FP16) return launch_dtype<LAYOUT, CARRY_RES_FP16, CARRY_SCALE_PER_V>(p, stream, sms);
-    if (p.res_fmt == CARRY_RES_FP8) return launch_dtype<LAYOUT, CARRY_RES_FP8, CARRY_SCALE_PER_V>(p, stream, sms);
+    return launch_dtype<LAYOUT, CARRY_RES_FP8, CARRY_SCALE_PER_V>(p, stream, sms);
+  } else {
+    const bool i4 = p.res_fmt == CARRY_RES_INT4, pv = p.rscale_mode == CARRY_SCALE_PER_V;
+    if (i4) return pv ? launch_dtype<LAYOUT, CARRY_RES_INT4, CARRY_SCALE_PER_V>(p, stream, sms)
+                      : launch_dtype<LAYOUT, CARRY_RES_INT4, CARRY_SCALE_PER_HEAD>(p, stream, sms);
+    return pv ? launch_dtype<LAYOUT, CARRY_RES_INT8, CARRY_SCALE_PER_V>(p, stream, sms)
+              : launch_dtype<LAYOUT, CARRY_RES_INT8, CARRY_SCALE_PER_HEAD>(p, stream, sms);
   }
-  const bool i4 = p.res_fmt == CARRY_RES_INT4, pv = p.rscale_mode == CARRY_SCALE_PER_V;
-  if (i4) return pv ? launch_dtype<LAYOUT, CARRY_RES_INT4, CARRY_SCALE_PER_V>(p, stream, sms)
-                    : launch_dtype<LAYOUT, CARRY_RES_INT4, CARRY_SCALE_PER_HEAD>(p, stream, sms);
-  return pv ? launch_dtype<LAYOUT, CARRY_RES_INT8, CARRY_SCALE_PER_V>(p, stream, sms)
-            : launch_dtype<LAYOUT, CARRY_RES_INT8, CARRY_SCALE_PER_HEAD>(p, stream, sms);
 }
 
 }  // namespace

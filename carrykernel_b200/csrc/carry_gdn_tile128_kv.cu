@@ -1,5 +1,5 @@
-// Streaming kernel, statequant layout [K][V] (every residual format, scale mode
-// and activation type): see carry_gdn_tile128.cuh.
+// Streaming kernel, statequant layout [K][V] (fp32, fp16 and fp8 residuals, every
+// activation type): see carry_gdn_tile128.cuh.
 #include "carry_gdn_tile128.cuh"
 
 namespace carry {

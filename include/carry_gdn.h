@@ -334,7 +334,7 @@ int carry_gdn_abi_version(void);
 
 /*
  * Which kernel the last successful call on this host thread selected:
- * 0 = none yet, 1 = generic tile kernel, 2 = 128x128 streaming kernel,
+ * 0 = none yet, 1 = generic tile kernel, 2 = 128x128 streaming kernel (of either layout),
  * 3 = multi-token kernel, 4 = a pool store / load / copy kernel,
  * 5 = 128x128 streaming kernel, step without error feedback,
  * 6 = slot-indexed kernel for 64x64 heads, 7 = kernel of chained steps,

@@ -1,0 +1,103 @@
+"""The statequant-layout kernels for 128- and 64-wide heads against the generic kernel, which takes the same call when the
+codes do not start on a vector boundary: one tile, head counts that are no multiple of anything, one tile more than there
+are CTAs (2 x 148), and enough of them to go round a CTA's ring of stages.  The two sum in different orders, so codes at a
+rounding tie may differ; tolerances are those of the comparison with the oracle."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from oracle import gdn_oracle as orc
+from parity import assert_close, check_quant_step, seeded_inputs
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _off_grid(x):
+    """A contiguous copy that starts one element behind a 16-byte boundary."""
+    wide = torch.empty(x.numel() + 16, dtype=x.dtype, device=x.device)
+    view = wide[1:1 + x.numel()].view(x.shape)
+    view.copy_(x)
+    return view
+
+
+@pytest.mark.parametrize("edge", [128, 64])
+@pytest.mark.parametrize("B,HV", [(1, 1), (2, 3), (27, 11), (47, 32)])
+@pytest.mark.parametrize("res_fmt,rscale,sscale", [(3, "v", "v"), (3, "head", "v"), (4, "v", "v"), (4, "head", "v"),
+                                                   (5, "v", "v"), (5, "v", "head")])
+@pytest.mark.parametrize("dtype,bits", [(torch.float32, 8), (torch.bfloat16, 4), (torch.float16, 3)])
+def test_step_against_the_generic_kernel(edge, B, HV, res_fmt, rscale, sscale, dtype, bits):
+    from carrykernel_b200 import _lib
+    from carrykernel_b200.statequant import kernel as sq
+    assert (res_fmt, sq.RES_INT8, sq.RES_INT4) == (res_fmt, 3, 4) and sq.RES_NONE == orc.RES_NONE == 5
+    h0, q, k, v, alpha, beta = seeded_inputs(B, HV, edge, edge, seed=B, dtype=dtype, alpha_mode="gated")
+    h0[0, 0, :, 2] = 0.0
+    state = orc.init_quant_state(h0[:2], bits, res_fmt, rscale, sscale)
+    reps = -(-B // state[0].shape[0])
+    state = [None if x is None else x.repeat(reps, *([1] * (x.dim() - 1)))[:B].to(DEV) for x in state]
+    g = torch.Generator(device=DEV).manual_seed(1)
+    if res_fmt == 3:
+        state[2] = torch.randint(-127, 128, state[2].shape, generator=g, dtype=torch.int8, device=DEV)
+    elif res_fmt == 4:                                    # two codes of -7..7 per byte
+        lo, hi = (torch.randint(-7, 8, state[2].shape, generator=g, dtype=torch.int8, device=DEV) for _ in range(2))
+        state[2] = (lo & 15) | (hi << 4)
+    if state[3] is not None:
+        state[3] = torch.rand(state[3].shape, generator=g, device=DEV) * 1e-6 + 1e-7
+    acts = [x.to(DEV) for x in (q, k, v, alpha, beta)]
+    kw = dict(bits=bits, res_fmt=res_fmt, resid_scale=rscale, state_scale=sscale)
+    got = sq.gdn_quant_step_fused(*state, *acts, **kw)
+    kernel = _lib.load_library().carry_gdn_last_kernel()
+    assert kernel == (8 if edge == 64 else 5 if res_fmt == 5 else 2)
+    want = sq.gdn_quant_step_fused(_off_grid(state[0]), *state[1:], *acts, **kw)
+    assert _lib.load_library().carry_gdn_last_kernel() == 1
+    # at most 6e-4 of the int8 residual codes differ at 8 bits, fewer at fewer bits (a residual step is then larger against
+    # the unit in the last place of its target); the smallest case has 4096 codes, 2.3 of them expected: allow 8 more
+    check_quant_step(got, [None if x is None else x.cpu() for x in want], res_fmt, unpack_int4=orc.unpack_int4,
+                     what=f"{edge} {res_fmt} {rscale} {sscale}", max_frac=1e-3 + 8 / got[1].numel())
+
+
+@pytest.mark.parametrize("B,HV", [(1, 1), (2, 3), (40, 31)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_fp32_step_of_narrow_heads(B, HV, dtype):
+    """Sums of 64 products of magnitude 0.1: 1e-6 apart in another order."""
+    from carrykernel_b200.statequant import kernel as sq
+    h0, q, k, v, alpha, beta = [x.to(DEV) for x in seeded_inputs(B, HV, 64, 64, seed=B, dtype=dtype, alpha_mode="gated")]
+    h, o = sq.gdn_step_fused_fp32(h0, q, k, v, alpha, beta)
+    hr, orf = orc.gdn_step(h0.cpu(), q.float().cpu(), k.float().cpu(), v.float().cpu(), alpha.cpu(), beta.cpu())
+    assert_close(h.cpu(), hr, "state", rtol=1e-5, atol=2e-6)
+    assert_close(o.cpu(), orf, "output", rtol=1e-5, atol=4e-6)
+
+
+@pytest.mark.parametrize("resid_fmt", [orc.RESID_INT8, orc.RESID_INT4])
+@pytest.mark.parametrize("rscale", ["v", "head"])
+@pytest.mark.parametrize("keep_error", [False, True])
+@pytest.mark.parametrize("edge", [64, 128])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_square_tiles_in_and_out_of_the_pool(resid_fmt, rscale, keep_error, edge, dtype):
+    """Bit for bit the oracle's, with a padding request and a pool whose slots are further apart than they need be."""
+    from carrykernel_b200.vllm_integration import state_pool as sp
+    B, HV, slots = 4, 3, 7
+    g = torch.Generator().manual_seed(edge)
+    h = torch.randn(B, HV, edge, edge, generator=g) * 0.1
+    h[0, 0, 0] = 0.0
+    h[0, 0, 1] *= 1e-20
+    h[0, 0, 2] = (torch.arange(edge) % 253 - 126).float() + 0.5      # ties
+    h[0, 0, 2, 0] = 127.0
+    h = h.to(dtype)
+    idx = torch.tensor([5, 0, 2, 6], dtype=torch.int32)
+    want = list(orc.init_quantized_pool(slots, HV, edge, edge, resid_fmt=resid_fmt, resid_scale=rscale))
+    got = []
+    for t in want:
+        wide = torch.zeros(slots, t[0].numel() + 16, dtype=t.dtype, device=DEV)
+        got.append(wide.as_strided(t.shape, (wide.stride(0), *t.stride()[1:])))
+        got[-1].copy_(t)
+    orc.pool_store(h, *want, idx, resid_fmt=resid_fmt, keep_error=keep_error)
+    sp.store_state(h.to(DEV), got, idx.to(DEV), resid_fmt=resid_fmt, keep_error=keep_error)
+    for x, y in zip(got, want):
+        assert torch.equal(x.cpu(), y)
+    out = torch.full((B, HV, edge, edge), 9.0, dtype=dtype, device=DEV)
+    sp.load_state(got, idx.to(DEV), resid_fmt=resid_fmt, out=out)
+    ref = orc.pool_load(*want, idx, resid_fmt=resid_fmt)
+    assert torch.equal(out.cpu(), ref.to(dtype))
