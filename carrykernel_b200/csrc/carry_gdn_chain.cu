@@ -5,7 +5,7 @@
 //
 // What it saves: 8 tokens of 64 requests x 32 heads with an fp32 residual were nine passes of eager kernels for the
 // initial state (0.4 ms) and 8 launches that each move 10 bytes per element (0.54 ms, at 85 % of the copy rate).  Here the
-// state crosses HBM once, 9 bytes per element in all, and the arithmetic bounds: 1011 -> 250 us.
+// state crosses HBM once, 9 bytes per element in all, and the arithmetic bounds: 1021 -> 306 us.
 //
 // One CTA of 8 warps per tile, two per SM.  Lane = 4 columns x the warp's 16 rows, column sums and maxima finished
 // across the warps through shared memory (two meetings per token).  Codes stay in registers from token to token, the
@@ -78,14 +78,20 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_chain_kernel(const __grid_con
   const float2 magic2 = splat(kMagicRound), nmagic2 = splat(-kMagicRound);
 
   // column maxima of all warps -> every lane's four columns
-  auto column_max = [&](float (&m)[4]) {
+  auto column_max = [&](float (&m)[4], auto&& larger) {
     *reinterpret_cast<float4*>(red_max + warp * kT + c0) = make_float4(m[0], m[1], m[2], m[3]);
     __syncthreads();
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) {
       const float4 y = *reinterpret_cast<const float4*>(red_max + w * kT + c0);
-      m[0] = fmaxf(m[0], y.x); m[1] = fmaxf(m[1], y.y); m[2] = fmaxf(m[2], y.z); m[3] = fmaxf(m[3], y.w);
+      m[0] = larger(m[0], y.x); m[1] = larger(m[1], y.y); m[2] = larger(m[2], y.z); m[3] = larger(m[3], y.w);
     }
+  };
+  // a NaN in the initial state has to reach its column's scale, as it does through torch's maximum; fmaxf drops it
+  auto max_or_nan = [](float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
   };
 
   uint32_t cw[16];                                        // codes of my 4 columns x 16 rows
@@ -104,16 +110,17 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_chain_kernel(const __grid_con
     float m[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      m[0] = fmaxf(m[0], fabsf(hA[i].x)); m[1] = fmaxf(m[1], fabsf(hA[i].y));
-      m[2] = fmaxf(m[2], fabsf(hB[i].x)); m[3] = fmaxf(m[3], fabsf(hB[i].y));
+      m[0] = max_or_nan(m[0], fabsf(hA[i].x)); m[1] = max_or_nan(m[1], fabsf(hA[i].y));
+      m[2] = max_or_nan(m[2], fabsf(hB[i].x)); m[3] = max_or_nan(m[3], fabsf(hB[i].y));
     }
-    column_max(m);
+    column_max(m, max_or_nan);
     float inv[4];
 #pragma unroll
-    for (int b = 0; b < 4; ++b) { scol[b] = __fmul_rn(fmaxf(m[b], kEps), p.inv_qmax); inv[b] = rcp_refined(scol[b]); }
+    for (int b = 0; b < 4; ++b) { scol[b] = __fmul_rn(max_or_nan(m[b], kEps), p.inv_qmax); inv[b] = rcp_refined(scol[b]); }
     auto code = [&](float v, int b) {                     // code + kMagicRound
       float y = fmaf(v, inv[b], kMagicRound);
       if (fabsf(fmaf(__fadd_rn(y, -kMagicRound), -scol[b], v)) > scol[b] * kTieGuard) y = __fadd_rn(exact_code(v, scol[b]), kMagicRound);
+      if (!(y == y)) y = kMagicRound;                     // a column with a NaN or an infinity: the conversion to int8 makes 0 of a NaN
       return __float_as_uint(fminf(fmaxf(y, kMagicRound - p.qmax), kMagicRound + p.qmax));
     };
 #pragma unroll
@@ -148,7 +155,7 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_chain_kernel(const __grid_con
         const void* src = which == 0 ? p.q : which == 1 ? p.k : p.v;
         const long long row = (x.first_token + t + tt) * step_rows + tile;
         *reinterpret_cast<uint4*>(sm + S::kVecs + tt * 3 * S::kVec + 16 * c) =
-            __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(src) + row * kT * qes) + (c - which * kPer));
+            __ldcg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(src) + row * kT * qes) + (c - which * kPer));
       }
       if (warp < nt) {
         const long long rows = (x.first_token + t + warp) * step_rows;
@@ -222,7 +229,7 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_chain_kernel(const __grid_con
         amax[2] = fmaxf(fmaxf(amax[2], fabsf(hB[i - 1].x)), fabsf(hB[i].x)); amax[3] = fmaxf(fmaxf(amax[3], fabsf(hB[i - 1].y)), fabsf(hB[i].y));
       }
     }
-    column_max(amax);
+    column_max(amax, [](float a, float b) { return fmaxf(a, b); });
 
     // new scales, codes, residual
     float thr[4];
