@@ -47,7 +47,21 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_multi_kernel(const __grid_con
   const int tile = (int)blockIdx.x;
   int n, hv, h;
   split_tile(p, tile, n, hv, h);
-  long long slot = p.slot_idx[(long long)n * p.stride_idx];
+  // CTAs that the launch ahead leaves room for start while its last ones run.  What they may do before it has finished
+  // is ask the L2 for the state of the slot that the index names now.  Against a launch that starts when the one ahead
+  // has ended: 2 us less per launch (32 requests x 32 heads, 4 tokens: 69.0 -> 66.6 us; 8 requests: 22.6 -> 20.6).
+  depend_release();
+  if (tid == 0) {
+    const long long guess = __ldcg(p.slot_idx + (long long)n * p.stride_idx);
+    if (guess > 0 && guess < p.num_slots) {
+      unsigned long long a8[8];
+      tile_addresses<RES, RSCALE, QDT>(p, n, hv, h, guess, a8);
+      l2_prefetch_bulk(reinterpret_cast<const void*>(a8[D_CODES]), kT * kT);
+      l2_prefetch_bulk(reinterpret_cast<const void*>(a8[D_RESID]), L::kResidBytes);
+    }
+  }
+  depend_wait();
+  long long slot = __ldcg(p.slot_idx + (long long)n * p.stride_idx);
   if (slot >= p.num_slots) {
     if (tid == 0 && p.status) atomicOr(p.status, CARRY_GDN_STATUS_BAD_SLOT);
     slot = 0;
@@ -93,7 +107,7 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_multi_kernel(const __grid_con
         const int tt = i / kVecChunks, c = i - tt * kVecChunks;
         const int which = c / (L::kVecBytes / 16), cc = c - which * (L::kVecBytes / 16);
         const uint8_t* src = reinterpret_cast<const uint8_t*>(addr[D_Q + which]) + (long long)(t + tt) * x.stride_mixed_t * qes;
-        *reinterpret_cast<uint4*>(&vec_t[tt][16 * c]) = __ldg(reinterpret_cast<const uint4*>(src) + cc);
+        *reinterpret_cast<uint4*>(&vec_t[tt][16 * c]) = __ldcg(reinterpret_cast<const uint4*>(src) + cc);
       }
       if (warp < nt)
         tile_meta<RES, RSCALE, QDT, 32>(p, tile, lane, true, &meta_t[warp], nullptr,
@@ -190,8 +204,7 @@ int launch_multi_variant(const KParams& p, const MultiExtra& x, cudaStream_t str
     }
     configured[dev] = true;
   }
-  kern<<<(unsigned)((long long)p.B * p.HV), kThreads, smem, stream>>>(p, x);
-  return cudaGetLastError() == cudaSuccess ? CARRY_GDN_OK : CARRY_GDN_ERR_LAUNCH;
+  return launch_dependent(kern, dim3((unsigned)((long long)p.B * p.HV)), kThreads, smem, stream, p, x);
 }
 
 template <int RES, int RSCALE>
