@@ -5,12 +5,13 @@
 //
 // What it saves: 8 tokens of 64 requests x 32 heads with an fp32 residual were nine passes of eager kernels for the
 // initial state (0.4 ms) and 8 launches that each move 10 bytes per element (0.54 ms, at 85 % of the copy rate).  Here the
-// state crosses HBM once, 9 bytes per element in all, and the arithmetic bounds: 1021 -> 306 us.
+// state crosses HBM once, 9 bytes per element in all, and the arithmetic bounds: 1021 -> 254 us.
 //
-// One CTA of 8 warps per tile, two per SM.  Lane = 4 columns x the warp's 16 rows, column sums and maxima finished
-// across the warps through shared memory (two meetings per token).  Codes stay in registers from token to token, the
-// residual in shared memory in its own format; a token's k and q are spread per warp as {k, k, q, q} rows so that packed
-// instructions read them as they are.
+// One CTA of 8 warps per tile, two per SM.  Lane = 4 columns x the warp's 16 rows.  A column's sums and its maximum are
+// finished by one lane, through shared memory, and handed to the others the same way: four meetings per token.  (Every
+// warp finishing all 128 columns for itself needs two, but takes 306 us instead of 254.)  Codes stay in registers from
+// token to token, the residual in shared memory in its own format; a token's k and q are spread per warp as {k, k, q, q}
+// rows so that packed instructions read them as they are.
 #include "carry_gdn_tile128.cuh"
 
 namespace carry {
@@ -33,7 +34,8 @@ struct ChainShared {
   static constexpr int kDot = kVecs + kChainChunk * 3 * kVec;         // [warp][col][2]
   static constexpr int kMax = kDot + kWarps * kT * 8;                 // [warp][col]
   static constexpr int kRows = kMax + kWarps * kT * 4;                // [warp][16] {k, k, q, q}
-  static constexpr int kMeta = kRows + kWarps * 16 * 16;
+  static constexpr int kCol = kRows + kWarps * 16 * 16;               // per column: delta; scale; its reciprocal
+  static constexpr int kMeta = kCol + 3 * kT * 4;
   static constexpr int kBytes = kMeta + kChainChunk * (int)sizeof(TileMeta);
 };
 
@@ -71,29 +73,30 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_chain_kernel(const __grid_con
   float* red_dot = reinterpret_cast<float*>(sm + S::kDot);
   float* red_max = reinterpret_cast<float*>(sm + S::kMax);
   float4* kq_row = reinterpret_cast<float4*>(sm + S::kRows) + warp * 16;
+  float* delta = reinterpret_cast<float*>(sm + S::kCol);
+  float *scale_of = delta + kT, *inv_of = delta + 2 * kT;
   TileMeta* meta = reinterpret_cast<TileMeta*>(sm + S::kMeta);
   const int tile = (int)blockIdx.x;                       // request * HV + head
   const long long el0 = (long long)tile * kT * kT;
   const long long step_rows = (long long)p.B * p.HV;      // (request, head) pairs of one token
   const float2 magic2 = splat(kMagicRound), nmagic2 = splat(-kMagicRound);
 
-  // column maxima of all warps -> every lane's four columns
-  auto column_max = [&](float (&m)[4], auto&& larger) {
-    *reinterpret_cast<float4*>(red_max + warp * kT + c0) = make_float4(m[0], m[1], m[2], m[3]);
-    __syncthreads();
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) {
-      const float4 y = *reinterpret_cast<const float4*>(red_max + w * kT + c0);
-      m[0] = larger(m[0], y.x); m[1] = larger(m[1], y.y); m[2] = larger(m[2], y.z); m[3] = larger(m[3], y.w);
-    }
-  };
   // a NaN in the initial state has to reach its column's scale, as it does through torch's maximum; fmaxf drops it
   auto max_or_nan = [](float a, float b) {
     float r;
     asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
     return r;
   };
-
+  // ... column maxima of all warps -> every lane's four columns
+  auto column_max = [&](float (&m)[4]) {
+    *reinterpret_cast<float4*>(red_max + warp * kT + c0) = make_float4(m[0], m[1], m[2], m[3]);
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      const float4 y = *reinterpret_cast<const float4*>(red_max + w * kT + c0);
+      m[0] = max_or_nan(m[0], y.x); m[1] = max_or_nan(m[1], y.y); m[2] = max_or_nan(m[2], y.z); m[3] = max_or_nan(m[3], y.w);
+    }
+  };
   uint32_t cw[16];                                        // codes of my 4 columns x 16 rows
   float scol[4];                                          // their scales
   float2 hA[16], hB[16];
@@ -113,7 +116,7 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_chain_kernel(const __grid_con
       m[0] = max_or_nan(m[0], fabsf(hA[i].x)); m[1] = max_or_nan(m[1], fabsf(hA[i].y));
       m[2] = max_or_nan(m[2], fabsf(hB[i].x)); m[3] = max_or_nan(m[3], fabsf(hB[i].y));
     }
-    column_max(m, max_or_nan);
+    column_max(m);
     float inv[4];
 #pragma unroll
     for (int b = 0; b < 4; ++b) { scol[b] = __fmul_rn(max_or_nan(m[b], kEps), p.inv_qmax); inv[b] = rcp_refined(scol[b]); }
@@ -186,36 +189,26 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_chain_kernel(const __grid_con
       dkA = fma2(a, kr, dkA); dkB = fma2(b, kr, dkB);
       dqA = fma2(a, qr, dqA); dqB = fma2(b, qr, dqB);
     }
-    float dv[4], oval[4];
+    // a column's reductions are finished by its lane of the first four warps, in the order of the streaming kernel
     {
       float4* dst = reinterpret_cast<float4*>(red_dot + (warp * kT + c0) * 2);
       dst[0] = make_float4(dkA.x, dqA.x, dkA.y, dqA.y);
       dst[1] = make_float4(dkB.x, dqB.x, dkB.y, dqB.y);
       __syncthreads();
-      float dk[4] = {0.f, 0.f, 0.f, 0.f}, dq[4] = {0.f, 0.f, 0.f, 0.f};
+      if (tid < kT) {
+        float2 d = splat(0.f);
 #pragma unroll
-      for (int w = 0; w < kWarps; ++w) {
-        const float4* src = reinterpret_cast<const float4*>(red_dot + (w * kT + c0) * 2);
-        const float4 x0 = src[0], x1 = src[1];
-        dk[0] += x0.x; dq[0] += x0.y; dk[1] += x0.z; dq[1] += x0.w;
-        dk[2] += x1.x; dq[2] += x1.y; dk[3] += x1.z; dq[3] += x1.w;
+        for (int w = 0; w < kWarps; ++w) d = add2(d, *reinterpret_cast<const float2*>(red_dot + (w * kT + tid) * 2));
+        const float dv = __fmul_rn(beta, __fadd_rn(act<QDT>(vec + 2 * S::kVec, tid), -d.x));
+        delta[tid] = dv;
+        store_from_float(p.out, ((x.first_token + t) * step_rows + tile) * kT + tid, p.o_dtype, fmaf(dv, kq, d.y));
       }
-      const float4 v4 = act4<QDT>(vec + 2 * S::kVec, c0);
-      const float v[4] = {v4.x, v4.y, v4.z, v4.w};
-#pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        dv[b] = __fmul_rn(beta, __fadd_rn(v[b], -dk[b]));
-        oval[b] = fmaf(dv[b], kq, dq[b]);
-      }
-    }
-    if (warp == 0) {
-      const long long at = ((x.first_token + t) * step_rows + tile) * kT + c0;
-#pragma unroll
-      for (int b = 0; b < 4; ++b) store_from_float(p.out, at + b, p.o_dtype, oval[b]);
+      __syncthreads();
     }
 
     // rank-1 write, residual, column maxima
-    const float2 dvA = make_float2(dv[0], dv[1]), dvB = make_float2(dv[2], dv[3]);
+    const float4 dv4 = *reinterpret_cast<const float4*>(delta + c0);
+    const float2 dvA = make_float2(dv4.x, dv4.y), dvB = make_float2(dv4.z, dv4.w);
     float amax[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
@@ -229,13 +222,23 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_chain_kernel(const __grid_con
         amax[2] = fmaxf(fmaxf(amax[2], fabsf(hB[i - 1].x)), fabsf(hB[i].x)); amax[3] = fmaxf(fmaxf(amax[3], fabsf(hB[i - 1].y)), fabsf(hB[i].y));
       }
     }
-    column_max(amax, [](float a, float b) { return fmaxf(a, b); });
+    *reinterpret_cast<float4*>(red_max + warp * kT + c0) = make_float4(amax[0], amax[1], amax[2], amax[3]);
+    __syncthreads();
+    if (tid < kT) {
+      float m = 0.f;
+#pragma unroll
+      for (int w = 0; w < kWarps; w += 2) m = fmaxf(fmaxf(m, red_max[w * kT + tid]), red_max[(w + 1) * kT + tid]);
+      const float sc = scale_fast(m, p.qmax, p.inv_qmax, p.eps_mode);
+      scale_of[tid] = sc;
+      inv_of[tid] = rcp_refined(sc);
+    }
+    __syncthreads();
 
     // new scales, codes, residual
-    float thr[4];
-#pragma unroll
-    for (int b = 0; b < 4; ++b) { scol[b] = scale_fast(amax[b], p.qmax, p.inv_qmax, p.eps_mode); thr[b] = scol[b] * kTieGuard; }
-    const float2 invA = make_float2(rcp_refined(scol[0]), rcp_refined(scol[1])), invB = make_float2(rcp_refined(scol[2]), rcp_refined(scol[3]));
+    const float4 s4 = *reinterpret_cast<const float4*>(scale_of + c0), i4 = *reinterpret_cast<const float4*>(inv_of + c0);
+    scol[0] = s4.x; scol[1] = s4.y; scol[2] = s4.z; scol[3] = s4.w;
+    const float thr[4] = {s4.x * kTieGuard, s4.y * kTieGuard, s4.z * kTieGuard, s4.w * kTieGuard};
+    const float2 invA = make_float2(i4.x, i4.y), invB = make_float2(i4.z, i4.w);
     const float2 nsA = make_float2(-scol[0], -scol[1]), nsB = make_float2(-scol[2], -scol[3]);
     float eamax[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
