@@ -49,9 +49,12 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_multi_kernel(const __grid_con
   split_tile(p, tile, n, hv, h);
   // CTAs that the launch ahead leaves room for start while its last ones run.  What they may do before it has finished
   // is ask the L2 for the state of the slot that the index names now.  Against a launch that starts when the one ahead
-  // has ended: 2 us less per launch (32 requests x 32 heads, 4 tokens: 69.0 -> 66.6 us; 8 requests: 22.6 -> 20.6).
+  // has ended: 3 us less per launch (32 requests x 32 heads, 4 tokens: 69.1 -> 65.9 us; 2 tokens: 43.4 -> 41.3).  The CTAs
+  // behind the first wave find the launch ahead finished, and the look at the index is in their way: hints from all
+  // of them, 66.4 and 41.9 us.
   depend_release();
-  if (tid == 0) {
+  constexpr int kFirstWave = 2 * 148;                // two CTAs on each SM
+  if (tid == 0 && blockIdx.x < kFirstWave) {
     const long long guess = __ldcg(p.slot_idx + (long long)n * p.stride_idx);
     if (guess > 0 && guess < p.num_slots) {
       unsigned long long a8[8];
