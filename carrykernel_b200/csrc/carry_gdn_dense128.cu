@@ -8,7 +8,7 @@
 // delta, the scales and their reciprocals) in shared memory (four lanes per column, over all 16 warps, measured 5 % slower:
 // more instructions in all); a scale per head needs one maximum per warp
 // only.  256 requests x 32 heads, against that shape: no residual, one scale per head 129 -> 98 us, per V 133 -> 105; int8
-// residual 164 -> 147, int4 172 -> 151 (one scale per head); 16 requests, int8 16.7 -> 13.2.
+// residual 164 -> 147, int4 172 -> 152 (one scale per head); 16 requests, int8 16.7 -> 13.2.
 //
 // A CTA is persistent (tile = blockIdx.x + number * gridDim.x) and loads with bulk copies into a ring of up to 4 stages; a
 // stage is requested again after the meeting behind the last read of it.  Addresses follow from the tile's index, the
@@ -205,20 +205,16 @@ __global__ void __launch_bounds__(kWide, 2) gdn_dense128_kernel(const __grid_con
         const float4 e4 = *reinterpret_cast<const float4*>(sb + D::kRScale + 4 * c0);
         esA = make_float2(e4.x, e4.y); esB = make_float2(e4.z, e4.w);
       }
-      const float2 nbA = mul2(esA, splat(-136.0f)), nbB = mul2(esB, splat(-136.0f));
 #pragma unroll
       for (int i = 0; i < kLaneRows; ++i) {
         const float2 kr = *reinterpret_cast<const float2*>(kq_row + i);
         if constexpr (D::kNone) {
           hA[i] = fma2(hA[i], saA, mul2(kr, dvA)); hB[i] = fma2(hB[i], saB, mul2(kr, dvB));
         } else if constexpr (D::kInt4) {
-          // a nibble in offset binary lands in a float that reads 136 + code; 136 * es is in the innermost addend
-          const uint32_t w = (uint32_t)(*reinterpret_cast<const uint16_t*>(sb + D::kResid + (r0 + i) * (kT / 2) + c0 / 2)) ^ 0x8888u;
-          const uint32_t lo = w & 0x0F0Fu, hi = (w >> 4) & 0x0F0Fu;
-          const float2 nA = make_float2(__uint_as_float(__byte_perm(lo, 0x43000000u, 0x7044)), __uint_as_float(__byte_perm(hi, 0x43000000u, 0x7044)));
-          const float2 nB = make_float2(__uint_as_float(__byte_perm(lo, 0x43000000u, 0x7144)), __uint_as_float(__byte_perm(hi, 0x43000000u, 0x7144)));
-          hA[i] = fma2(nA, esA, fma2(hA[i], saA, fma2(kr, dvA, nbA)));
-          hB[i] = fma2(nB, esB, fma2(hB[i], saB, fma2(kr, dvB, nbB)));
+          float2 nA, nB;
+          s4x4_pairs(*reinterpret_cast<const uint16_t*>(sb + D::kResid + (r0 + i) * (kT / 2) + c0 / 2), nA, nB);
+          hA[i] = fma2(nA, esA, fma2(hA[i], saA, mul2(kr, dvA)));
+          hB[i] = fma2(nB, esB, fma2(hB[i], saB, mul2(kr, dvB)));
         } else {
           const uint32_t w = *reinterpret_cast<const uint32_t*>(sb + D::kResid + (r0 + i) * kT + c0) ^ 0x80808080u;
           hA[i] = fma2(s8x2_to_float<0, 1>(w), esA, fma2(kr, dvA, hA[i]));

@@ -132,7 +132,6 @@ __global__ void __launch_bounds__(kPair, RES == CARRY_RES_NONE ? 8 : 6) gdn_dens
   // rank-1 write, residual, column maxima
   const float2 dvA = make_float2(dv[0], dv[1]), dvB = make_float2(dv[2], dv[3]);
   const float2 esA = make_float2(es_col[0], es_col[1]), esB = make_float2(es_col[2], es_col[3]);
-  const float2 nbA = mul2(esA, splat(-136.0f)), nbB = mul2(esB, splat(-136.0f));
   float amax[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
@@ -140,11 +139,10 @@ __global__ void __launch_bounds__(kPair, RES == CARRY_RES_NONE ? 8 : 6) gdn_dens
     if constexpr (kNone) {
       hA[i] = fma2(hA[i], saA, mul2(kr, dvA)); hB[i] = fma2(hB[i], saB, mul2(kr, dvB));
     } else if constexpr (kInt4) {
-      const uint32_t w = ew[i] ^ 0x8888u, lo = w & 0x0F0Fu, hi = (w >> 4) & 0x0F0Fu;
-      const float2 nA = make_float2(__uint_as_float(__byte_perm(lo, 0x43000000u, 0x7044)), __uint_as_float(__byte_perm(hi, 0x43000000u, 0x7044)));
-      const float2 nB = make_float2(__uint_as_float(__byte_perm(lo, 0x43000000u, 0x7144)), __uint_as_float(__byte_perm(hi, 0x43000000u, 0x7144)));
-      hA[i] = fma2(nA, esA, fma2(hA[i], saA, fma2(kr, dvA, nbA)));
-      hB[i] = fma2(nB, esB, fma2(hB[i], saB, fma2(kr, dvB, nbB)));
+      float2 nA, nB;
+      s4x4_pairs(ew[i], nA, nB);
+      hA[i] = fma2(nA, esA, fma2(hA[i], saA, mul2(kr, dvA)));
+      hB[i] = fma2(nB, esB, fma2(hB[i], saB, mul2(kr, dvB)));
     } else {
       const uint32_t w = ew[i] ^ 0x80808080u;
       hA[i] = fma2(s8x2_to_float<0, 1>(w), esA, fma2(kr, dvA, hA[i]));

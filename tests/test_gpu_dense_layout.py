@@ -58,6 +58,38 @@ def test_step_against_the_generic_kernel(edge, B, HV, res_fmt, rscale, sscale, d
                      what=f"{edge} {res_fmt} {rscale} {sscale}", max_frac=1e-3 + 8 / got[1].numel())
 
 
+@pytest.mark.parametrize("edge", [128, 64])
+@pytest.mark.parametrize("rscale", ["v", "head"])
+def test_int4_residual_scale_of_a_larger_column(edge, rscale):
+    """Columns of very different magnitudes under residual scales that belong to the largest one: a residual code of 0 adds
+    exactly 0, so that a column a million times smaller is rounded as well as the largest, and a zero column stays zero.
+
+    A target is three roundings of its own size and a sum of `edge` products: within 2e-5 of the column's step of the oracle's,
+    which flips 4e-5 of the codes."""
+    from carrykernel_b200 import _lib
+    from carrykernel_b200.statequant import kernel as sq
+    B, HV = 3, 8
+    h0, q, k, v, alpha, beta = seeded_inputs(B, HV, edge, edge, seed=edge, alpha_mode="gated")
+    mags = torch.tensor([1.0, 1e-2, 1e-4, 1e-6, 0.0])
+    kind = torch.arange(edge) % len(mags)
+    h0, v = h0 * mags[kind], v * mags[kind]
+    h, scale, _, _ = orc.init_quant_state(h0, 8, orc.RES_INT4, rscale)
+    codes = torch.randint(-7, 8, h.shape, generator=torch.Generator().manual_seed(2)) * (kind == 0)
+    top = scale.amax(-1) / 14.0                            # half a step of the largest column is 7 codes
+    es = top if rscale == "head" else top[..., None].expand(B, HV, edge).contiguous()
+    state = (h, scale, orc.pack_int4(codes.to(torch.int8)), es)
+    want = orc.quant_step(*state, q, k, v, alpha, beta, res_fmt=orc.RES_INT4, resid_scale=rscale)
+    got = sq.gdn_quant_step_fused(*[x.to(DEV) for x in (*state, q, k, v, alpha, beta)], res_fmt=sq.RES_INT4, resid_scale=rscale)
+    assert _lib.load_library().carry_gdn_last_kernel() == (8 if edge == 64 else 2)
+    for j, mag in enumerate(mags.tolist()):
+        of_kind = kind == j
+        a, b = got[1].cpu()[..., of_kind], want[1][..., of_kind]
+        assert int((a.int() - b.int()).abs().max()) <= 1, mag
+        assert float((a != b).float().mean()) <= 2e-4, mag
+        assert_close(got[2].cpu()[..., of_kind], want[2][..., of_kind], f"scales of columns x {mag}", rtol=1e-5, atol=0.0)
+    assert not got[1].cpu()[..., kind == 4].any()
+
+
 @pytest.mark.parametrize("B,HV", [(1, 1), (2, 3), (40, 31)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 def test_fp32_step_of_narrow_heads(B, HV, dtype):
