@@ -14,7 +14,7 @@ bool eps_ok(int m) { return m == CARRY_EPS_ON_AMAX || m == CARRY_EPS_ON_SCALE; }
 
 int dispatch(const carry::KParams& p, cudaStream_t stream) {
   if ((long long)p.B * p.HV == 0) return CARRY_GDN_OK;
-  if (carry::tile128_eligible(p)) {
+  if (carry::tile128_eligible(p) || carry::noresid128_eligible(p)) {
     const int rc = carry::launch_tile128(p, stream);
     if (rc == CARRY_GDN_OK) g_last_kernel = p.res_fmt == CARRY_RES_NONE ? 5 : 2;
     return rc;

@@ -69,6 +69,11 @@ inline void fill_shifts(KParams& p) {
   p.group_shift = log2_or_minus1(p.group);
 }
 
+// the values of qmax for which the streaming kernels' way to divide by it (div_qmax) is exact: 3 to 8 bits
+inline bool div_qmax_exact(float qmax) {
+  return qmax == 3.f || qmax == 7.f || qmax == 15.f || qmax == 31.f || qmax == 63.f || qmax == 127.f;
+}
+
 __device__ __forceinline__ float load_as_float(const void* p, long long i, int dtype) {
   if (dtype == CARRY_F32) return reinterpret_cast<const float*>(p)[i];
   if (dtype == CARRY_BF16) return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[i]);
@@ -217,6 +222,7 @@ int launch_dependent(void (*kern)(P...), dim3 grid, unsigned threads, size_t sme
 int launch_generic(const KParams& p, cudaStream_t stream);
 int launch_fp32(const CarryGdnFp32Args& a, cudaStream_t stream);
 bool tile128_eligible(const KParams& p);
+bool noresid128_eligible(const KParams& p);
 int launch_tile128(const KParams& p, cudaStream_t stream);
 bool dense64_eligible(const KParams& p);
 int launch_dense64(const KParams& p, cudaStream_t stream);

@@ -14,6 +14,11 @@
 // stage is requested again after the meeting behind the last read of it.  Addresses follow from the tile's index, the
 // gates are loaded one tile ahead and <k, q> is one warp's work meanwhile, so a launch begins with its first tile's
 // copies and nothing ahead of them.
+//
+// Without a residual there is a second form (LOOSE) for calls that the bulk copies or the division shortcut do not take:
+// activations and scales that start off a 16-byte boundary, a qmax that is not 2^(bits-1) - 1 for 3..8 bits.  It copies
+// the codes alone and reads the vectors where they are used: 256 requests x 32 heads on 2 bits 113 us with one scale per head
+// (133 per V), where the generic kernel takes 3.3 ms.
 #include "carry_gdn_tile128.cuh"
 
 namespace carry {
@@ -23,8 +28,9 @@ constexpr int kWide = 512;              // threads of a CTA
 constexpr int kWideWarps = kWide / 32;
 constexpr int kLaneRows = kT / kWideWarps;
 
-template <int RES, int RSCALE, int QDT>
+template <int RES, int RSCALE, int QDT, bool LOOSE>
 struct Dense128 {
+  static_assert(!LOOSE || RES == CARRY_RES_NONE, "the other formats have the generic kernel");
   static constexpr bool kNone = RES == CARRY_RES_NONE, kInt4 = RES == CARRY_RES_INT4;
   static constexpr bool kHeadState = kNone && RSCALE == CARRY_SCALE_PER_HEAD;     // RSCALE: the state's granularity then
   static constexpr bool kHeadResid = !kNone && RSCALE == CARRY_SCALE_PER_HEAD;
@@ -34,11 +40,11 @@ struct Dense128 {
   static constexpr int kResidBytes = kNone ? 0 : kInt4 ? kT * kT / 2 : kT * kT;
   static constexpr int kResid = kT * kT;
   static constexpr int kSScale = kResid + kResidBytes;
-  static constexpr int kRScale = kSScale + (kColState ? 512 : 0);
+  static constexpr int kRScale = kSScale + (kColState && !LOOSE ? 512 : 0);
   static constexpr int kQ = kRScale + (kColResid ? 512 : 0);
   static constexpr int kK = kQ + kVec;
   static constexpr int kV = kK + kVec;
-  static constexpr int kStage = kV + kVec;
+  static constexpr int kStage = LOOSE ? kQ : kV + kVec;
   static_assert(kStage % 128 == 0, "stages keep the ring's alignment");
   // behind the ring; partial results lie [warp][column]
   static constexpr int kDotRow = kT * 8, kMaxRow = kT * 4;
@@ -57,10 +63,15 @@ struct Dense128 {
 };
 
 // One thread requests a tile: the bytes to come are announced, then copied.
-template <int RES, int RSCALE, int QDT>
+template <int RES, int RSCALE, int QDT, bool LOOSE>
 __device__ __forceinline__ void request_tile(const KParams& p, uint8_t* sb, uint64_t* bar, int tile) {
-  using D = Dense128<RES, RSCALE, QDT>;
+  using D = Dense128<RES, RSCALE, QDT, LOOSE>;
   const long long nh = tile;
+  if constexpr (LOOSE) {
+    mbar_arrive_expect_tx(bar, kT * kT + test_extra_tx(tile));
+    bulk_load(sb, p.codes_in + nh * kT * kT, kT * kT, bar);
+    return;
+  }
   mbar_arrive_expect_tx(bar, kT * kT + D::kResidBytes + (D::kColState ? 512 : 0) + (D::kColResid ? 512 : 0) + 3 * D::kVec + test_extra_tx(tile));
   bulk_load(sb, p.codes_in + nh * kT * kT, kT * kT, bar);
   if constexpr (D::kColState) bulk_load(sb + D::kSScale, p.sscale_in + nh * kT, 512, bar);
@@ -71,9 +82,9 @@ __device__ __forceinline__ void request_tile(const KParams& p, uint8_t* sb, uint
   if constexpr (D::kColResid) bulk_load(sb + D::kRScale, p.rscale_in + nh * kT, 512, bar);
 }
 
-template <int RES, int RSCALE, int QDT>
+template <int RES, int RSCALE, int QDT, bool LOOSE>
 __global__ void __launch_bounds__(kWide, 2) gdn_dense128_kernel(const __grid_constant__ KParams p) {
-  using D = Dense128<RES, RSCALE, QDT>;
+  using D = Dense128<RES, RSCALE, QDT, LOOSE>;
   constexpr int S = D::kStages;
   constexpr bool kFold = D::kInt4 || D::kNone;           // sums over the bare codes, the column's scale on the totals
   constexpr float rqmax = D::kInt4 ? 7.0f : 127.0f, rrqmax = 1.0f / rqmax;
@@ -104,7 +115,7 @@ __global__ void __launch_bounds__(kWide, 2) gdn_dense128_kernel(const __grid_con
   depend_wait();
   if (tid == 0)
     for (int s = 0; s < S && (int)blockIdx.x + s * step < total; ++s)
-      request_tile<RES, RSCALE, QDT>(p, smem + s * D::kStage, &full_bar[s], (int)blockIdx.x + s * step);
+      request_tile<RES, RSCALE, QDT, LOOSE>(p, smem + s * D::kStage, &full_bar[s], (int)blockIdx.x + s * step);
   // gates (and a scale per head) of the tile in hand and of the next one
   float alpha_next = __ldcg(p.alpha + blockIdx.x), beta_next = __ldcg(p.beta + blockIdx.x), head_next = 0.f;
   const float* head_scale = D::kHeadState ? p.sscale_in : p.rscale_in;
@@ -125,6 +136,10 @@ __global__ void __launch_bounds__(kWide, 2) gdn_dense128_kernel(const __grid_con
     const float top = warp_max_nonneg(fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3])));
     if (lane == 0) head_max[warp] = top;
   };
+  auto new_scale = [&](float m) {
+    if constexpr (LOOSE) return scale_from_amax(m, p.qmax, p.eps_mode);
+    return scale_fast(m, p.qmax, p.inv_qmax, p.eps_mode);
+  };
   auto all_heads = [&]() { return warp_max_nonneg(head_max[lane & (kWideWarps - 1)]); };
 
   int s = 0;
@@ -138,15 +153,28 @@ __global__ void __launch_bounds__(kWide, 2) gdn_dense128_kernel(const __grid_con
     }
     uint8_t* sb = smem + s * D::kStage;
     healthy = mbar_wait(&full_bar[s], parity, poison, p.status);
+    const long long vec0 = (long long)tile * kT;         // where this tile's vectors start
+    auto vec_at = [&](const void* x, int stage_off, int i) {
+      if constexpr (LOOSE) return raw_to_float(load_raw(x, vec0 + i, QDT), QDT);
+      return act<QDT>(sb + stage_off, i);
+    };
 
     // k and q of my warp's rows, each twice side by side
     {
-      const float x = act<QDT>(sb + ((lane & 8) ? D::kQ : D::kK), r0 + (lane & 7));
+      const float x = vec_at((lane & 8) ? p.q : p.k, (lane & 8) ? D::kQ : D::kK, r0 + (lane & 7));
       if (lane < 16) *reinterpret_cast<float2*>(reinterpret_cast<float*>(kq_row + (lane & 7)) + ((lane & 8) ? 2 : 0)) = splat(x);
       __syncwarp();
     }
     if (warp == kWideWarps - 1) {
-      const float4 k4 = act4<QDT>(sb + D::kK, 4 * lane), q4 = act4<QDT>(sb + D::kQ, 4 * lane);
+      float4 k4, q4;
+      if constexpr (LOOSE) {
+        auto four = [&](const void* x) {
+          return make_float4(vec_at(x, 0, 4 * lane), vec_at(x, 0, 4 * lane + 1), vec_at(x, 0, 4 * lane + 2), vec_at(x, 0, 4 * lane + 3));
+        };
+        k4 = four(p.k); q4 = four(p.q);
+      } else {
+        k4 = act4<QDT>(sb + D::kK, 4 * lane); q4 = act4<QDT>(sb + D::kQ, 4 * lane);
+      }
       float y = fmaf(k4.w, q4.w, fmaf(k4.z, q4.z, fmaf(k4.y, q4.y, k4.x * q4.x)));
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
@@ -159,6 +187,9 @@ __global__ void __launch_bounds__(kWide, 2) gdn_dense128_kernel(const __grid_con
       float2 sA, sB;
       if constexpr (D::kHeadState) {
         sA = sB = splat(head_in);
+      } else if constexpr (LOOSE) {
+        const float* x = p.sscale_in + vec0 + c0;
+        sA = make_float2(__ldcg(x), __ldcg(x + 1)); sB = make_float2(__ldcg(x + 2), __ldcg(x + 3));
       } else {
         const float4 s4 = *reinterpret_cast<const float4*>(sb + D::kSScale + 4 * c0);
         sA = make_float2(s4.x, s4.y); sB = make_float2(s4.z, s4.w);
@@ -190,7 +221,7 @@ __global__ void __launch_bounds__(kWide, 2) gdn_dense128_kernel(const __grid_con
 #pragma unroll
       for (int w = 4; w < kWideWarps; ++w) d[w & 3] = add2(d[w & 3], x[w * kT]);
       const float2 sum = add2(add2(d[0], d[1]), add2(d[2], d[3]));
-      const float dv = __fmul_rn(beta, __fadd_rn(act<QDT>(sb + D::kV, col), -sum.x));
+      const float dv = __fmul_rn(beta, __fadd_rn(vec_at(p.v, D::kV, col), -sum.x));
       delta[col] = dv;
       store_from_float(p.out, (long long)tile * kT + col, p.o_dtype, fmaf(dv, *kq_sum, sum.y));
     }
@@ -228,17 +259,17 @@ __global__ void __launch_bounds__(kWide, 2) gdn_dense128_kernel(const __grid_con
     }
     if constexpr (D::kHeadState) head_of(m); else put_max(m);
     __syncthreads();
-    if (tid == 0 && tile + S * step < total) request_tile<RES, RSCALE, QDT>(p, sb, &full_bar[s], tile + S * step);   // the stage has been read
+    if (tid == 0 && tile + S * step < total) request_tile<RES, RSCALE, QDT, LOOSE>(p, sb, &full_bar[s], tile + S * step);   // the stage has been read
     // new state scales
     float2 snA, snB, inA, inB;
     if constexpr (D::kHeadState) {
-      const float sn = scale_fast(all_heads(), p.qmax, p.inv_qmax, p.eps_mode);
+      const float sn = new_scale(all_heads());
       snA = snB = splat(sn);
       inA = inB = splat(rcp_refined(sn));
       if (tid == 0) p.sscale_out[tile] = sn;
     } else {
       if (finisher) {
-        const float sn = scale_fast(col_max(), p.qmax, p.inv_qmax, p.eps_mode);
+        const float sn = new_scale(col_max());
         scale_of[col] = sn;
         inv_of[col] = rcp_refined(sn);
         p.sscale_out[(long long)tile * kT + col] = sn;
@@ -323,10 +354,10 @@ __global__ void __launch_bounds__(kWide, 2) gdn_dense128_kernel(const __grid_con
   }
 }
 
-template <int RES, int RSCALE, int QDT>
+template <int RES, int RSCALE, int QDT, bool LOOSE>
 int launch_wide(const KParams& p, cudaStream_t stream, int sms) {
-  auto kern = gdn_dense128_kernel<RES, RSCALE, QDT>;
-  constexpr int smem = Dense128<RES, RSCALE, QDT>::kBytes;
+  auto kern = gdn_dense128_kernel<RES, RSCALE, QDT, LOOSE>;
+  constexpr int smem = Dense128<RES, RSCALE, QDT, LOOSE>::kBytes;
   static thread_local bool configured[64] = {false};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return CARRY_GDN_ERR_NO_DEVICE;
@@ -341,19 +372,32 @@ int launch_wide(const KParams& p, cudaStream_t stream, int sms) {
   return launch_dependent(kern, dim3((unsigned)(tiles < 2LL * sms ? tiles : 2LL * sms)), kWide, smem, stream, p);
 }
 
-template <int RES, int RSCALE>
+template <int RES, int RSCALE, bool LOOSE = false>
 int launch_wide_dtype(const KParams& p, cudaStream_t stream, int sms) {
-  if (p.qkv_dtype == CARRY_F32) return launch_wide<RES, RSCALE, CARRY_F32>(p, stream, sms);
-  if (p.qkv_dtype == CARRY_BF16) return launch_wide<RES, RSCALE, CARRY_BF16>(p, stream, sms);
-  return launch_wide<RES, RSCALE, CARRY_F16>(p, stream, sms);
+  if (p.qkv_dtype == CARRY_F32) return launch_wide<RES, RSCALE, CARRY_F32, LOOSE>(p, stream, sms);
+  if (p.qkv_dtype == CARRY_BF16) return launch_wide<RES, RSCALE, CARRY_BF16, LOOSE>(p, stream, sms);
+  return launch_wide<RES, RSCALE, CARRY_F16, LOOSE>(p, stream, sms);
 }
+
+bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 }  // namespace
 
+// Without a residual: any qmax, any number of heads, either granularity, as long as the codes start on a 16-byte boundary.
+bool noresid128_eligible(const KParams& p) {
+  return !p.packed && p.res_fmt == CARRY_RES_NONE && p.K == kT && p.V == kT && (long long)p.B * p.HV <= 0x7fffffffLL &&
+         aligned16(p.codes_in) && aligned16(p.codes_out);
+}
+
 int launch_dense128(const KParams& p, cudaStream_t stream, int sms) {
-  if (p.res_fmt == CARRY_RES_NONE)
-    return p.sscale_mode == CARRY_SCALE_PER_V ? launch_wide_dtype<CARRY_RES_NONE, CARRY_SCALE_PER_V>(p, stream, sms)
-                                              : launch_wide_dtype<CARRY_RES_NONE, CARRY_SCALE_PER_HEAD>(p, stream, sms);
+  if (p.res_fmt == CARRY_RES_NONE) {
+    const bool per_v = p.sscale_mode == CARRY_SCALE_PER_V;
+    const bool loose = !div_qmax_exact(p.qmax) || !aligned16(p.q) || !aligned16(p.k) || !aligned16(p.v) || (per_v && !aligned16(p.sscale_in));
+    if (loose) return per_v ? launch_wide_dtype<CARRY_RES_NONE, CARRY_SCALE_PER_V, true>(p, stream, sms)
+                            : launch_wide_dtype<CARRY_RES_NONE, CARRY_SCALE_PER_HEAD, true>(p, stream, sms);
+    return per_v ? launch_wide_dtype<CARRY_RES_NONE, CARRY_SCALE_PER_V>(p, stream, sms)
+                 : launch_wide_dtype<CARRY_RES_NONE, CARRY_SCALE_PER_HEAD>(p, stream, sms);
+  }
   const bool i4 = p.res_fmt == CARRY_RES_INT4, pv = p.rscale_mode == CARRY_SCALE_PER_V;
   if (i4) return pv ? launch_wide_dtype<CARRY_RES_INT4, CARRY_SCALE_PER_V>(p, stream, sms)
                     : launch_wide_dtype<CARRY_RES_INT4, CARRY_SCALE_PER_HEAD>(p, stream, sms);

@@ -12,26 +12,22 @@ namespace {
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 }  // namespace
 
-// The streaming kernels need K = V = 128, an integer residual (any residual format, or none, in the statequant
-// layout), a per-V state scale (or none and either granularity), qmax = 2^(bits-1) - 1 for 3..8 bits, and 16-byte
-// aligned, dense rows for every bulk copy.
+// The streaming kernels need K = V = 128, an integer residual (any residual format in the statequant layout; without one:
+// noresid128_eligible), a per-V state scale, qmax = 2^(bits-1) - 1 for 3..8 bits, and 16-byte aligned, dense rows for every
+// bulk copy.
 bool tile128_eligible(const KParams& p) {
   if (p.K != 128 || p.V != 128) return false;
   const bool int_resid = p.res_fmt == CARRY_RES_INT8 || p.res_fmt == CARRY_RES_INT4;
   const bool float_resid = p.res_fmt == CARRY_RES_FP32 || p.res_fmt == CARRY_RES_FP16 || p.res_fmt == CARRY_RES_FP8;
-  const bool no_resid = p.res_fmt == CARRY_RES_NONE;
-  if (!int_resid && !((float_resid || no_resid) && !p.packed)) return false;   // the others: statequant layout only
-  if (p.sscale_mode != CARRY_SCALE_PER_V && !no_resid) return false;
-  // the kernel divides by qmax with a multiply and a correcting fused multiply-add, which equals the
-  // IEEE quotient for these values (the quantisation widths 3..8 bits) and has not been checked for others
-  if (p.qmax != 3.f && p.qmax != 7.f && p.qmax != 15.f && p.qmax != 31.f && p.qmax != 63.f && p.qmax != 127.f)
-    return false;
+  if (!int_resid && !(float_resid && !p.packed)) return false;   // float residuals: statequant layout only
+  if (p.sscale_mode != CARRY_SCALE_PER_V) return false;
+  if (!div_qmax_exact(p.qmax)) return false;
   if (p.HV > 128 || (long long)p.B * p.HV > 0x7fffffffLL) return false;
   const int qes = p.qkv_dtype == CARRY_F32 ? 4 : 2;
   // one residual scale per head: the slot layout copies the 16 bytes around it, the statequant layout reads it as it is
   const bool copied_rscale = int_resid && (p.packed || p.rscale_mode == CARRY_SCALE_PER_V);
-  if (!aligned16(p.codes_in) || !aligned16(p.codes_out) || (!no_resid && (!aligned16(p.resid_in) || !aligned16(p.resid_out))) ||
-      (p.sscale_mode == CARRY_SCALE_PER_V && (!aligned16(p.sscale_in) || !aligned16(p.sscale_out))) ||
+  if (!aligned16(p.codes_in) || !aligned16(p.codes_out) || !aligned16(p.resid_in) || !aligned16(p.resid_out) ||
+      !aligned16(p.sscale_in) || !aligned16(p.sscale_out) ||
       (copied_rscale && (!aligned16(p.rscale_in) || !aligned16(p.rscale_out))) ||
       !aligned16(p.q) || !aligned16(p.k) || !aligned16(p.v) || !aligned16(p.out))
     return false;

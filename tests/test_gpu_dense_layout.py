@@ -90,6 +90,31 @@ def test_int4_residual_scale_of_a_larger_column(edge, rscale):
     assert not got[1].cpu()[..., kind == 4].any()
 
 
+@pytest.mark.parametrize("case", ["2 bits", "129 heads", "activations", "scales"])
+@pytest.mark.parametrize("sscale", ["v", "head"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_step_without_residual_at_any_width_and_alignment(case, sscale, dtype):
+    """128-wide heads without a residual need nothing but codes on a 16-byte boundary: the smallest grid (one level on either
+    side of zero), more heads than the streaming kernel's tables hold, and vectors that start anywhere."""
+    from carrykernel_b200 import _lib
+    from carrykernel_b200.statequant import kernel as sq
+    B, HV, bits = (3, 129, 4) if case == "129 heads" else (20, 16, 2 if case == "2 bits" else 8)
+    h0, q, k, v, alpha, beta = seeded_inputs(B, HV, 128, 128, seed=B, dtype=dtype, alpha_mode="gated")
+    h, scale, _, _ = [None if x is None else x.to(DEV) for x in orc.init_quant_state(h0, bits, orc.RES_NONE, "v", sscale)]
+    acts = [x.to(DEV) for x in (q, k, v, alpha, beta)]
+    if case == "activations":
+        acts = [_off_grid(x) for x in acts]
+    elif case == "scales":
+        scale = _off_grid(scale)
+    kw = dict(bits=bits, res_fmt=sq.RES_NONE, state_scale=sscale)
+    got = sq.gdn_quant_step_fused(h, scale, None, None, *acts, **kw)
+    assert _lib.load_library().carry_gdn_last_kernel() == 5
+    want = sq.gdn_quant_step_fused(_off_grid(h), scale, None, None, *acts, **kw)
+    assert _lib.load_library().carry_gdn_last_kernel() == 1
+    check_quant_step(got, [None if x is None else x.cpu() for x in want], orc.RES_NONE, unpack_int4=orc.unpack_int4,
+                     what=f"{case} {sscale}", max_frac=1e-3)
+
+
 @pytest.mark.parametrize("B,HV", [(1, 1), (2, 3), (40, 31)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 def test_fp32_step_of_narrow_heads(B, HV, dtype):
