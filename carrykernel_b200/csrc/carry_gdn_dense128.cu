@@ -140,6 +140,8 @@ __global__ void __launch_bounds__(kWide, 2) gdn_dense128_kernel(const __grid_con
     if constexpr (LOOSE) return scale_from_amax(m, p.qmax, p.eps_mode);
     return scale_fast(m, p.qmax, p.inv_qmax, p.eps_mode);
   };
+  // ... and as it is written out: the shortcut makes a NaN of an infinite maximum, whose quotient is infinite
+  auto put_scale = [&](float* to, float m, float sn) { *to = D::kNone && m == __int_as_float(0x7f800000) ? m : sn; };
   auto all_heads = [&]() { return warp_max_nonneg(head_max[lane & (kWideWarps - 1)]); };
 
   int s = 0;
@@ -223,7 +225,9 @@ __global__ void __launch_bounds__(kWide, 2) gdn_dense128_kernel(const __grid_con
       const float2 sum = add2(add2(d[0], d[1]), add2(d[2], d[3]));
       const float dv = __fmul_rn(beta, __fadd_rn(vec_at(p.v, D::kV, col), -sum.x));
       delta[col] = dv;
-      store_from_float(p.out, (long long)tile * kT + col, p.o_dtype, fmaf(dv, *kq_sum, sum.y));
+      // (0 * dv: the sum over rows of an infinite write has both signs in it; the folded sum alone would not show that)
+      const float hq = D::kNone ? fmaf(0.f, dv, sum.y) : sum.y;
+      store_from_float(p.out, (long long)tile * kT + col, p.o_dtype, fmaf(dv, *kq_sum, hq));
     }
     __syncthreads();
     // rank-1 write, residual, column maxima
@@ -263,16 +267,16 @@ __global__ void __launch_bounds__(kWide, 2) gdn_dense128_kernel(const __grid_con
     // new state scales
     float2 snA, snB, inA, inB;
     if constexpr (D::kHeadState) {
-      const float sn = new_scale(all_heads());
+      const float top = all_heads(), sn = new_scale(top);
       snA = snB = splat(sn);
       inA = inB = splat(rcp_refined(sn));
-      if (tid == 0) p.sscale_out[tile] = sn;
+      if (tid == 0) put_scale(p.sscale_out + tile, top, sn);
     } else {
       if (finisher) {
-        const float sn = new_scale(col_max());
+        const float top = col_max(), sn = new_scale(top);
         scale_of[col] = sn;
         inv_of[col] = rcp_refined(sn);
-        p.sscale_out[(long long)tile * kT + col] = sn;
+        put_scale(p.sscale_out + (long long)tile * kT + col, top, sn);
       }
       __syncthreads();
       const float4 s4 = *reinterpret_cast<const float4*>(scale_of + c0), i4 = *reinterpret_cast<const float4*>(inv_of + c0);
@@ -336,10 +340,8 @@ __global__ void __launch_bounds__(kWide, 2) gdn_dense128_kernel(const __grid_con
       for (int i = 0; i < kLaneRows; ++i) {
         const float2 rA = fma2(hA[i], inA, magic2), rB = fma2(hB[i], inB, magic2);
         if constexpr (D::kInt4) {
-          // 16 * odd + even (+ 136: both nibbles offset by 8) in one float, whose low byte is the pair
-          const uint32_t p01 = __float_as_uint(fmaf(__fadd_rn(rA.y, -kMagicRound), 16.0f, __fadd_rn(rA.x, 136.0f)));
-          const uint32_t p23 = __float_as_uint(fmaf(__fadd_rn(rB.y, -kMagicRound), 16.0f, __fadd_rn(rB.x, 136.0f)));
-          *reinterpret_cast<uint16_t*>(dst + i * (kT / 2)) = (uint16_t)(__byte_perm(p01, p23, 0x0040) ^ 0x8888u);
+          *reinterpret_cast<uint16_t*>(dst + i * (kT / 2)) =
+              (uint16_t)pack_s4x4(__float_as_uint(rA.x), __float_as_uint(rA.y), __float_as_uint(rB.x), __float_as_uint(rB.y));
         } else {
           *reinterpret_cast<uint32_t*>(dst + i * kT) = pack4(__float_as_uint(rA.x), __float_as_uint(rA.y), __float_as_uint(rB.x), __float_as_uint(rB.y));
         }

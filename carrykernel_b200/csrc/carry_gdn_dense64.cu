@@ -7,8 +7,11 @@
 // registers (a row of a warp is 32 bytes of codes, a whole sector), and results go back the same way.  One CTA of two
 // warps per (request, head), six or eight to an SM, so that one tile's loads run under another's arithmetic.
 //
+// A NaN or an infinity leaves the codes and scales that the generic kernel leaves: a warp whose columns
+// it reaches goes element by element.  (Looking for them takes 4 to 6 %: 15.4 -> 16.0 us at 100 requests x 32 heads, int8 residual.)
+//
 // The generic kernel, which took these shapes, stages a tile as fp32 in shared memory and walks columns with a quarter
-// of its threads: 215 us at 100 requests x 32 heads with an int8 residual; this one 17 us.
+// of its threads: 215 us at 100 requests x 32 heads with an int8 residual; this one 16 us.
 #include "carry_gdn_tile128.cuh"
 
 namespace carry {
@@ -47,6 +50,13 @@ __device__ __forceinline__ float column_max(const float (&x)[4], int g) {
   return fmaxf(keep, __shfl_xor_sync(kAll, send, 8));
 }
 
+// the largest magnitude of three, a NaN if one of them is (fmaxf passes a NaN over)
+__device__ __forceinline__ float max3abs_nan(float a, float b, float c) {
+  float r;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
 // What both kernels start with: k and q of the tile as {k, k, q, q} rows (a copy per warp), <k, q>
 template <int QDT>
 __device__ __forceinline__ float spread_kq(const void* q, const void* k, long long at, float4* rows, int lane) {
@@ -60,6 +70,23 @@ __device__ __forceinline__ float spread_kq(const void* q, const void* k, long lo
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) kq += __shfl_xor_sync(kAll, kq, o);
   return kq;
+}
+
+// The codes of a lane's 16 elements x[0], x[4], ... of a column to bytes `pitch` apart, and their remainders in place, by the
+// true quotient and the clamp as the generic kernel does it: for columns that hold a NaN or an infinity, or whose scale is one
+// (the reciprocal makes NaNs of all its quotients).  nibble: 0 whole bytes, 1 the low half of each, 2 the high half
+// behind it.  Returns the largest remainder.
+__device__ __noinline__ float quantize_column_plainly(float* x, float s, float qmax, int8_t* to, int pitch, int nibble) {
+  float worst = 0.f;
+#pragma unroll 1
+  for (int i = 0; i < 16; ++i, to += pitch) {
+    const float code = quantize_div(x[4 * i], s, qmax);
+    x[4 * i] = fmaf(code, -s, x[4 * i]);
+    worst = fmaxf(worst, fabsf(x[4 * i]));
+    const int c = (int)code;
+    *to = (int8_t)(nibble == 0 ? c : nibble == 1 ? (c & 15) : (*to | (c << 4)));
+  }
+  return worst;
 }
 
 // RSCALE: granularity of the residual's scale, or of the state's where there is no residual
@@ -101,7 +128,10 @@ __global__ void __launch_bounds__(kPair, RES == CARRY_RES_NONE ? 8 : 6) gdn_dens
 
   // dequantise, decay, partial column sums
   const float2 sA = make_float2(scol[0], scol[1]), sB = make_float2(scol[2], scol[3]), alpha2 = splat(alpha);
-  const float2 saA = mul2(sA, alpha2), saB = mul2(sB, alpha2);
+  float2 saA = mul2(sA, alpha2), saB = mul2(sB, alpha2);
+  if constexpr (kFold) {                // an infinite scale makes NaNs, as 0 * scale does; the folded sum alone would not
+    saA = fma2(saA, splat(0.f), saA); saB = fma2(saB, splat(0.f), saB);
+  }
   float2 hA[16], hB[16], dkA = splat(0.f), dkB = dkA, dqA = dkA, dqB = dkA;
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
@@ -125,8 +155,10 @@ __global__ void __launch_bounds__(kPair, RES == CARRY_RES_NONE ? 8 : 6) gdn_dens
     if (g >= 2) {                       // the lanes that hold q totals finish their two columns' output
       const bool up = g & 1;
       const long long at = nh * kN + c0 + (up ? 2 : 0);
-      store_from_float(p.out, at, p.o_dtype, fmaf(up ? dv[2] : dv[0], kq, mine[0]));
-      store_from_float(p.out, at + 1, p.o_dtype, fmaf(up ? dv[3] : dv[1], kq, mine[1]));
+      const float d0 = up ? dv[2] : dv[0], d1 = up ? dv[3] : dv[1];
+      // (0 * d: the sum over rows of an infinite write has both signs in it)
+      store_from_float(p.out, at, p.o_dtype, fmaf(d0, kq, fmaf(0.f, d0, mine[0])));
+      store_from_float(p.out, at + 1, p.o_dtype, fmaf(d1, kq, fmaf(0.f, d1, mine[1])));
     }
   }
   // rank-1 write, residual, column maxima
@@ -148,8 +180,21 @@ __global__ void __launch_bounds__(kPair, RES == CARRY_RES_NONE ? 8 : 6) gdn_dens
       hA[i] = fma2(s8x2_to_float<0, 1>(w), esA, fma2(kr, dvA, hA[i]));
       hB[i] = fma2(s8x2_to_float<2, 3>(w), esB, fma2(kr, dvB, hB[i]));
     }
-    amax[0] = fmaxf(amax[0], fabsf(hA[i].x)); amax[1] = fmaxf(amax[1], fabsf(hA[i].y));
-    amax[2] = fmaxf(amax[2], fabsf(hB[i].x)); amax[3] = fmaxf(amax[3], fabsf(hB[i].y));
+    if (i & 1) {                        // two rows per three-operand maximum; it keeps a NaN
+      amax[0] = max3abs_nan(amax[0], hA[i - 1].x, hA[i].x); amax[1] = max3abs_nan(amax[1], hA[i - 1].y, hA[i].y);
+      amax[2] = max3abs_nan(amax[2], hB[i - 1].x, hB[i].x); amax[3] = max3abs_nan(amax[3], hB[i - 1].y, hB[i].y);
+    }
+  }
+  const float inf = __int_as_float(0x7f800000);
+  const bool finite = max3abs_nan(max3abs_nan(amax[0], amax[1], amax[2]), amax[3], 0.f) < inf;
+  if (!finite) {                        // a scale passes NaNs over
+#pragma unroll
+    for (int b = 0; b < 4; ++b) amax[b] = 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      amax[0] = fmaxf(amax[0], fabsf(hA[i].x)); amax[1] = fmaxf(amax[1], fabsf(hA[i].y));
+      amax[2] = fmaxf(amax[2], fabsf(hB[i].x)); amax[3] = fmaxf(amax[3], fabsf(hB[i].y));
+    }
   }
   // a scale per column (its lane group's g-th lane works it out), or one for the matrix
   auto scales = [&](const float (&m)[4], bool per_head, float qmax, float (&s)[4], float (&inv)[4]) {
@@ -177,13 +222,38 @@ __global__ void __launch_bounds__(kPair, RES == CARRY_RES_NONE ? 8 : 6) gdn_dens
 #pragma unroll
     for (int b = 0; b < 4; ++b) p.sscale_out[nh * kN + c0 + b] = snew[b];
   }
+  int8_t* cout = p.codes_out + nh * kN * kN + g * kN + c0;
+  uint8_t* eout = reinterpret_cast<uint8_t*>(p.resid_out) + nh * kN * kRow + g * kRow + (kInt4 ? c0 / 2 : c0);
+  constexpr float rqmax = kInt4 ? 7.0f : 127.0f;
+  float eamax[4] = {0.f, 0.f, 0.f, 0.f}, es[4], ei[4];
+  auto put_resid_scales = [&]() {
+    if (kHeadResid) {
+      if (tid == 0) p.rscale_out[nh] = es[0];
+    } else if (g == 0) {
+#pragma unroll
+      for (int b = 0; b < 4; ++b) p.rscale_out[nh * kN + c0 + b] = es[b];
+    }
+  };
+  if (__any_sync(kAll, !finite || !(snew[0] + snew[1] + snew[2] + snew[3] < inf))) {      // (one vote per warp: scales() meets)
+    float plain[64];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) { plain[4 * i] = hA[i].x; plain[4 * i + 1] = hA[i].y; plain[4 * i + 2] = hB[i].x; plain[4 * i + 3] = hB[i].y; }
+#pragma unroll
+    for (int b = 0; b < 4; ++b) eamax[b] = quantize_column_plainly(plain + b, snew[b], p.qmax, cout + b, 4 * kN, 0);
+    if constexpr (!kNone) {
+      scales(eamax, kHeadResid, rqmax, es, ei);
+      put_resid_scales();
+#pragma unroll
+      for (int b = 0; b < 4; ++b)
+        quantize_column_plainly(plain + b, es[b], rqmax, reinterpret_cast<int8_t*>(eout) + (kInt4 ? b / 2 : b), 4 * kRow, kInt4 ? 1 + (b & 1) : 0);
+    }
+    return;
+  }
   // codes; remainders in place of the targets
   const float2 invA = make_float2(sinv[0], sinv[1]), invB = make_float2(sinv[2], sinv[3]);
   const float2 nsA = make_float2(-snew[0], -snew[1]), nsB = make_float2(-snew[2], -snew[3]);
   const float2 magic2 = splat(kMagicRound), nmagic2 = splat(-kMagicRound);
   const float thr[4] = {snew[0] * kTieGuard, snew[1] * kTieGuard, snew[2] * kTieGuard, snew[3] * kTieGuard};
-  int8_t* cout = p.codes_out + nh * kN * kN + g * kN + c0;
-  float eamax[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
     float2 yA = fma2(hA[i], invA, magic2), yB = fma2(hB[i], invB, magic2);
@@ -198,26 +268,16 @@ __global__ void __launch_bounds__(kPair, RES == CARRY_RES_NONE ? 8 : 6) gdn_dens
     eamax[2] = fmaxf(eamax[2], fabsf(hB[i].x)); eamax[3] = fmaxf(eamax[3], fabsf(hB[i].y));
   }
   if constexpr (!kNone) {
-    float es[4], ei[4];
-    scales(eamax, kHeadResid, kInt4 ? 7.0f : 127.0f, es, ei);
-    if (kHeadResid) {
-      if (tid == 0) p.rscale_out[nh] = es[0];
-    } else if (g == 0) {
-#pragma unroll
-      for (int b = 0; b < 4; ++b) p.rscale_out[nh * kN + c0 + b] = es[b];
-    }
+    scales(eamax, kHeadResid, rqmax, es, ei);
+    put_resid_scales();
+    if (kHeadResid && !(es[0] < inf)) ei[0] = ei[1] = ei[2] = ei[3] = 0.f;      // from the other warp's columns
     const float2 ieA = make_float2(ei[0], ei[1]), ieB = make_float2(ei[2], ei[3]);
-    uint8_t* eout = reinterpret_cast<uint8_t*>(p.resid_out) + nh * kN * kRow + g * kRow + (kInt4 ? c0 / 2 : c0);
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       const float2 rA = fma2(hA[i], ieA, magic2), rB = fma2(hB[i], ieB, magic2);
-      if constexpr (kInt4) {
-        const uint32_t p01 = __float_as_uint(fmaf(__fadd_rn(rA.y, -kMagicRound), 16.0f, __fadd_rn(rA.x, 136.0f)));
-        const uint32_t p23 = __float_as_uint(fmaf(__fadd_rn(rB.y, -kMagicRound), 16.0f, __fadd_rn(rB.x, 136.0f)));
-        *reinterpret_cast<uint16_t*>(eout + 4 * i * kRow) = (uint16_t)(__byte_perm(p01, p23, 0x0040) ^ 0x8888u);
-      } else {
-        *reinterpret_cast<uint32_t*>(eout + 4 * i * kRow) = pack4(__float_as_uint(rA.x), __float_as_uint(rA.y), __float_as_uint(rB.x), __float_as_uint(rB.y));
-      }
+      const uint32_t r[4] = {__float_as_uint(rA.x), __float_as_uint(rA.y), __float_as_uint(rB.x), __float_as_uint(rB.y)};
+      if constexpr (kInt4) *reinterpret_cast<uint16_t*>(eout + 4 * i * kRow) = (uint16_t)pack_s4x4(r[0], r[1], r[2], r[3]);
+      else *reinterpret_cast<uint32_t*>(eout + 4 * i * kRow) = pack4(r[0], r[1], r[2], r[3]);
     }
   }
 }

@@ -3,7 +3,8 @@
 // A row of the slot layout [V][K] is 64 elements, which one lane can hold: lane = one V row.  Sums and maxima over K
 // are then chains inside a lane, every scale is a lane's own, outputs and scales leave coalesced, and nothing is
 // exchanged between lanes except the per-head residual maximum.  (Every operation is rounded where the generic
-// kernel rounds it and in its order, so the two agree bit for bit.)
+// kernel rounds it and in its order, so the two agree bit for bit;
+// rows with a NaN or an infinity, of which the reciprocal would make other codes, go through the true quotients.)
 //
 // Bound: a tile is 4 KB of codes and 2 or 4 KB of residual, and a batch of 48 requests x 16 heads is 5 tiles per
 // SM -- latency and instruction issue, not bandwidth.  So no ring and no roles: one CTA of two warps per
@@ -110,6 +111,22 @@ __device__ __forceinline__ float quantize_row(float2 (&x)[kN / 2], float s, Put&
       if (KEEP) { x[j + i] = e[i]; x[j + i + 1] = e[i + 1]; }
       put(j + i, y[i], y[i + 1]);
     }
+  }
+  return worst;
+}
+
+// The same for a row that holds a NaN or an infinity, or whose scale is one (the reciprocal makes NaNs of all its quotients):
+// element by element as the generic kernel does it, codes straight into the lane's staged row.
+__device__ __noinline__ float quantize_row_plainly(float* x, float s, float qmax, uint8_t* to, bool nibbles) {
+  float worst = 0.f;
+#pragma unroll 1
+  for (int i = 0; i < kN; ++i) {
+    const float code = quantize_div(x[i], s, qmax);
+    x[i] = __fadd_rn(x[i], -__fmul_rn(code, s));
+    worst = fmaxf(worst, fabsf(x[i]));
+    const uint32_t c = (uint32_t)(int)code;
+    if (!nibbles) to[i] = (uint8_t)c;
+    else to[i / 2] = (uint8_t)((i & 1) ? (to[i / 2] | (c << 4)) : (c & 15u));
   }
   return worst;
 }
@@ -238,11 +255,25 @@ __global__ void __launch_bounds__(kPair, 6) gdn_narrow_kernel(const __grid_const
   // state codes into the stage (a lane's own row), remainders in place of the targets
   const float snew = scale_from_amax(amax, p.qmax, p.eps_mode);
   *sscale = snew;
+  // maxima pass a NaN over; the sum for the output keeps the state's, and those of the residual come from its scale
+  const float inf = __int_as_float(0x7f800000);
+  const bool finite = fabsf(o) < inf && snew < inf && fabsf(es) < inf;
+  float plain[kN];                      // the row of a lane that has to go element by element
+  auto take_plain = [&]() {
+#pragma unroll
+    for (int j = 0; j < kN / 2; ++j) { plain[2 * j] = x[j].x; plain[2 * j + 1] = x[j].y; }
+  };
   uint32_t word[4];
-  const float emax = quantize_row<true>(x, snew, [&](int j, float2 a, float2 b) {
-    word[(j / 2) & 3] = pack4(__float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(b.x), __float_as_uint(b.y));
-    if ((j & 7) == 6) *reinterpret_cast<uint4*>(st_codes + lane * kPitch + (j / 8) * 16) = make_uint4(word[0], word[1], word[2], word[3]);
-  });
+  float emax;
+  if (finite) {
+    emax = quantize_row<true>(x, snew, [&](int j, float2 a, float2 b) {
+      word[(j / 2) & 3] = pack4(__float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(b.x), __float_as_uint(b.y));
+      if ((j & 7) == 6) *reinterpret_cast<uint4*>(st_codes + lane * kPitch + (j / 8) * 16) = make_uint4(word[0], word[1], word[2], word[3]);
+    });
+  } else {
+    take_plain();
+    emax = quantize_row_plainly(plain, snew, p.qmax, st_codes + lane * kPitch, false);
+  }
   // residual scale and codes
   constexpr float rqmax = kInt4 ? 7.0f : 127.0f;
   float top = emax;
@@ -254,7 +285,10 @@ __global__ void __launch_bounds__(kPair, 6) gdn_narrow_kernel(const __grid_const
   }
   const float esn = scale_from_amax(top, rqmax, p.eps_mode);
   if (kPerV || tid == 0) *rscale = esn;
-  if constexpr (kInt4) {
+  if (!finite || !(esn < inf)) {
+    if (finite) take_plain();
+    quantize_row_plainly(plain, esn, rqmax, st_resid + lane * kPitchR, kInt4);
+  } else if constexpr (kInt4) {
     uint32_t by[4];
     quantize_row<false>(x, esn, [&](int j, float2 a, float2 b) {
       // 16 * odd + even in one float whose low byte is the pair, each nibble offset by 8

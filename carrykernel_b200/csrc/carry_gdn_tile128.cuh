@@ -253,6 +253,12 @@ __device__ __forceinline__ void s4x4_pairs(uint32_t w, float2& a, float2& b) {
   a = add2(make_float2(__uint_as_float(__byte_perm(lo, 0x43000000u, 0x7044)), __uint_as_float(__byte_perm(hi, 0x43000000u, 0x7044))), bias);
   b = add2(make_float2(__uint_as_float(__byte_perm(lo, 0x43000000u, 0x7144)), __uint_as_float(__byte_perm(hi, 0x43000000u, 0x7144))), bias);
 }
+// ... and back: the low nibbles of four words -> two bytes.  Each nibble is its word's alone, so a NaN in one column
+// (whose bits say nothing) leaves the column beside it as it is.
+__device__ __forceinline__ uint32_t pack_s4x4(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  const uint32_t even = __byte_perm(a, c, 0x0040), odd = __byte_perm(b, d, 0x0040) << 4;
+  return (even & 0x0F0Fu) | (odd & 0xF0F0u);
+}
 // four fp8-e5m2 values in a word -> floats.  An e5m2 value is the upper byte of the half with the same
 // value, so each pair of bytes becomes a half2 by one byte permute.
 __device__ __forceinline__ void e5m2x4_to_float(uint32_t w, float2& ab, float2& cd) {

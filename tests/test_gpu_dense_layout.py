@@ -9,7 +9,7 @@ import pytest
 import torch
 
 from oracle import gdn_oracle as orc
-from parity import assert_close, check_quant_step, seeded_inputs
+from parity import assert_close, assert_codes, check_quant_step, seeded_inputs
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -113,6 +113,77 @@ def test_step_without_residual_at_any_width_and_alignment(case, sscale, dtype):
     assert _lib.load_library().carry_gdn_last_kernel() == 1
     check_quant_step(got, [None if x is None else x.cpu() for x in want], orc.RES_NONE, unpack_int4=orc.unpack_int4,
                      what=f"{case} {sscale}", max_frac=1e-3)
+
+
+def _spoil(what, state, acts):
+    """Copies with one value of head (1, 1) replaced; column 5 where the tensor has columns."""
+    state, acts = [None if x is None else x.clone() for x in state], [x.clone() for x in acts]
+    name, value = what.rsplit(" ", 1)
+    t = {"v": acts[2], "k": acts[1], "alpha": acts[3], "scale": state[1], "resid scale": state[3]}[name]
+    t.view(t.shape[0], t.shape[1], -1)[1, 1, min(5, t.numel() // (t.shape[0] * t.shape[1]) - 1)] = float(value)
+    return state, acts
+
+
+def _spoiled_case(edge, res_fmt, rscale, sscale, what):
+    h0, q, k, v, alpha, beta = seeded_inputs(2, 3, edge, edge, seed=1, alpha_mode="gated")
+    state = [None if x is None else x.to(DEV) for x in orc.init_quant_state(h0, 8, res_fmt, rscale, sscale)]
+    if state[3] is not None:
+        g = torch.Generator().manual_seed(1)
+        codes = torch.randint(-7, 8, h0.shape, generator=g).to(torch.int8)
+        state[2] = (orc.pack_int4(codes) if res_fmt == 4 else codes).to(DEV)
+        state[3] += 1e-5
+    acts = [x.to(DEV) for x in (q, k, v, alpha, beta)]
+    return (state, acts), _spoil(what, state, acts), dict(bits=8, res_fmt=res_fmt, resid_scale=rscale, state_scale=sscale)
+
+
+@pytest.mark.parametrize("res_fmt,rscale,sscale", [(3, "v", "v"), (3, "head", "v"), (4, "v", "v"), (4, "head", "v"),
+                                                   (5, "v", "v"), (5, "v", "head")])
+@pytest.mark.parametrize("what", ["v nan", "v inf", "k nan", "k inf", "alpha inf", "scale nan", "scale inf",
+                                  "resid scale nan", "resid scale inf"])
+def test_narrow_heads_with_a_value_that_is_not_finite(res_fmt, rscale, sscale, what):
+    """A NaN or an infinity leaves what the generic kernel leaves: maxima that pass a NaN over, clamped codes.  (The
+    kernels sum in different orders: codes elsewhere may differ at a tie, as in the comparison above.)"""
+    from carrykernel_b200 import _lib
+    from carrykernel_b200.statequant import kernel as sq
+    if res_fmt == 5 and what.startswith("resid"):
+        pytest.skip("no residual")
+    _, (state, acts), kw = _spoiled_case(64, res_fmt, rscale, sscale, what)
+    got = [None if x is None else x.cpu() for x in sq.gdn_quant_step_fused(*state, *acts, **kw)]
+    assert _lib.load_library().carry_gdn_last_kernel() == 8
+    want = [None if x is None else x.cpu() for x in sq.gdn_quant_step_fused(_off_grid(state[0]), *state[1:], *acts, **kw)]
+    assert _lib.load_library().carry_gdn_last_kernel() == 1
+    limit = 2e-3 + 8 / got[1].numel()
+    flips, _ = assert_codes(got[1], want[1], "state codes", max_frac=limit)
+    if res_fmt < 5:
+        a, b = (orc.unpack_int4(x) if res_fmt == 4 else x for x in (got[3], want[3]))
+        assert_codes(a, b, "residual codes", max_frac=limit, exclude=flips)
+    assert torch.equal(torch.isfinite(got[0]), torch.isfinite(want[0]))
+    for i in (0, 2, 4):
+        if got[i] is not None:
+            a, b = got[i], want[i]
+            assert torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(torch.isinf(a), torch.isinf(b)), i
+            ok = torch.isfinite(b)
+            assert_close(a[ok], b[ok], f"output {i}", rtol=1e-3, atol=1e-5 if i == 0 else 1e-9)
+
+
+@pytest.mark.parametrize("edge", [128, 64])
+@pytest.mark.parametrize("res_fmt", [3, 4, 5])
+@pytest.mark.parametrize("what", ["v nan", "v inf", "scale nan", "scale inf"])
+def test_columns_beside_one_that_is_not_finite(edge, res_fmt, what):
+    """With scales per column a NaN or an infinity in one stays in it: every other column is left bit for bit as it would be
+    without it, residual codes that share a byte with the lost column's among them."""
+    from carrykernel_b200.statequant import kernel as sq
+    clean, spoiled, kw = _spoiled_case(edge, res_fmt, "v", "v", what)
+    want, got = (sq.gdn_quant_step_fused(*state, *acts, **kw) for state, acts in (clean, spoiled))
+    keep = torch.ones(2, 3, edge, dtype=torch.bool, device=DEV)
+    keep[1, 1, 5] = False
+    assert not torch.isfinite(got[0][1, 1, 5]) and (what != "v inf" or res_fmt != 5 or torch.isinf(got[2][1, 1, 5]))
+    for a, b in zip(got, want):
+        if a is not None:
+            if res_fmt == 4 and a.dim() == 4 and a.shape[-1] == edge // 2:
+                a, b = (orc.unpack_int4(x.cpu()).to(DEV) for x in (a, b))
+            where = keep[:, :, None].expand(a.shape) if a.dim() == 4 else keep
+            assert torch.equal(a[where], b[where])
 
 
 @pytest.mark.parametrize("B,HV", [(1, 1), (2, 3), (40, 31)])
