@@ -130,13 +130,12 @@ ERR_UNSUPPORTED = -5
 
 EXPORTS = ("carry_gdn_quant_step", "carry_gdn_quant_decode", "carry_gdn_fp32_step", "carry_gdn_packed_decode",
            "carry_gdn_packed_decode_multi", "carry_gdn_pool_store", "carry_gdn_pool_load",
-           "carry_gdn_pool_copy", "carry_gdn_pool_copy_layers", "carry_gdn_write_ids", "carry_gdn_strerror",
+           "carry_gdn_pool_copy", "carry_gdn_pool_copy_layers", "carry_gdn_strerror",
            "carry_gdn_abi_version", "carry_gdn_last_kernel")
 # what the native call path is given the addresses of, in the order it expects them (csrc/host_native.cpp, Table)
 _NATIVE_ENTRIES = ("carry_gdn_quant_step", "carry_gdn_fp32_step", "carry_gdn_packed_decode",
                    "carry_gdn_packed_decode_multi", "carry_gdn_pool_store", "carry_gdn_pool_load",
-                   "carry_gdn_pool_copy", "carry_gdn_pool_copy_layers", "carry_gdn_write_ids",
-                   "carry_gdn_quant_decode")
+                   "carry_gdn_pool_copy", "carry_gdn_pool_copy_layers", "carry_gdn_quant_decode")
 
 _lib = None
 _lock = threading.Lock()
@@ -174,10 +173,9 @@ def load_library(path: str | None = None):
         lib.carry_gdn_pool_load.argtypes = [C.POINTER(PoolLoadArgs), C.c_void_p]
         lib.carry_gdn_pool_copy.argtypes = [C.POINTER(PoolCopyArgs), C.c_void_p]
         lib.carry_gdn_pool_copy_layers.argtypes = [C.POINTER(PoolCopyLayersArgs), C.c_void_p]
-        lib.carry_gdn_write_ids.argtypes = [C.c_void_p, C.c_void_p, C.c_int32, C.c_void_p]
         for fn in (lib.carry_gdn_quant_step, lib.carry_gdn_fp32_step, lib.carry_gdn_packed_decode,
                    lib.carry_gdn_packed_decode_multi, lib.carry_gdn_pool_store, lib.carry_gdn_pool_load,
-                   lib.carry_gdn_pool_copy, lib.carry_gdn_pool_copy_layers, lib.carry_gdn_write_ids, lib.carry_gdn_quant_decode):
+                   lib.carry_gdn_pool_copy, lib.carry_gdn_pool_copy_layers, lib.carry_gdn_quant_decode):
             fn.restype = C.c_int
         if lib.carry_gdn_abi_version() != ABI_VERSION:
             raise CudaUnavailable(

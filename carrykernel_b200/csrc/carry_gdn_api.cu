@@ -291,12 +291,4 @@ int carry_gdn_pool_copy_layers(const CarryGdnPoolCopyLayersArgs* a, void* stream
   return rc;
 }
 
-int carry_gdn_write_ids(int32_t* dst, const int32_t* ids, int32_t n, void* stream) {
-  clear_stale_error();
-  if (n < 0) return CARRY_GDN_ERR_SHAPE;
-  if (n == 0) return CARRY_GDN_OK;
-  if (!dst || !ids) return CARRY_GDN_ERR_NULL;
-  return carry::launch_write_ids(dst, ids, n, static_cast<cudaStream_t>(stream));
-}
-
 }  // extern "C"

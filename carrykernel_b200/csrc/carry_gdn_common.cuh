@@ -238,6 +238,5 @@ int launch_pool_store(const CarryGdnPoolStoreArgs& a, cudaStream_t stream);
 int launch_pool_load(const CarryGdnPoolLoadArgs& a, cudaStream_t stream);
 int launch_pool_copy(const CarryGdnPoolCopyArgs& a, cudaStream_t stream);
 int launch_pool_copy_layers(const CarryGdnPoolCopyLayersArgs& a, cudaStream_t stream);
-int launch_write_ids(int32_t* dst, const int32_t* ids, int n, cudaStream_t stream);
 
 }  // namespace carry

@@ -829,17 +829,6 @@ __global__ void __launch_bounds__(kThreads) pool_copy_layers_kernel(const __grid
              left < kPiece ? left : kPiece);
 }
 
-// slot ids from kernel arguments to device memory
-constexpr int kIdsPerLaunch = 960;
-struct IdBlock {
-  int32_t v[kIdsPerLaunch];
-};
-__global__ void __launch_bounds__(kThreads) write_ids_kernel(int32_t* dst, int n, const __grid_constant__ IdBlock ids) {
-  depend_release();
-  depend_wait();
-  for (int i = threadIdx.x; i < n; i += kThreads) dst[i] = ids.v[i];
-}
-
 int grid_for(long long tiles) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -940,17 +929,6 @@ int launch_pool_copy_layers(const CarryGdnPoolCopyLayersArgs& a, cudaStream_t st
       m.src[l][3] = s.resid_scale + from * s.stride_rscale_slot; m.dst[l][3] = d.resid_scale + to * d.stride_rscale_slot;
     }
     const int rc = launch_dependent(pool_copy_layers_kernel, dim3((unsigned)pieces, (unsigned)layers), kThreads, 0, stream, m);
-    if (rc != CARRY_GDN_OK) return rc;
-  }
-  return CARRY_GDN_OK;
-}
-
-int launch_write_ids(int32_t* dst, const int32_t* ids, int n, cudaStream_t stream) {
-  for (int i = 0; i < n; i += kIdsPerLaunch) {
-    const int m = n - i < kIdsPerLaunch ? n - i : kIdsPerLaunch;
-    IdBlock b;
-    for (int j = 0; j < m; ++j) b.v[j] = ids[i + j];
-    const int rc = launch_dependent(write_ids_kernel, dim3(1), kThreads, 0, stream, dst + i, m, b);
     if (rc != CARRY_GDN_OK) return rc;
   }
   return CARRY_GDN_OK;

@@ -35,10 +35,9 @@ struct Table {
   int (*pool_load)(const CarryGdnPoolLoadArgs*, void*);
   int (*pool_copy)(const CarryGdnPoolCopyArgs*, void*);
   int (*pool_copy_layers)(const CarryGdnPoolCopyLayersArgs*, void*);
-  int (*write_ids)(int32_t*, const int32_t*, int32_t, void*);
   int (*quant_decode)(const CarryGdnDecodeArgs*, void*);
 };
-constexpr int kEntries = 10;
+constexpr int kEntries = 9;
 
 const Table* table_of(PyObject* o) { return static_cast<const Table*>(PyLong_AsVoidPtr(o)); }
 
@@ -557,29 +556,6 @@ PyObject* pool_copy_layers(PyObject*, PyObject* const* o, Py_ssize_t n) {
   });
 }
 
-// A fresh int32 tensor on the device from a list of ints.  (table, ids, device index) -> tensor
-PyObject* ids_tensor(PyObject*, PyObject* const* o, Py_ssize_t n) {
-  return guarded([&]() -> PyObject* {
-    if (n != 3) return nullptr;
-    const Table* tab = table_of(o[0]);
-    long dev;
-    if (!tab || !PyList_CheckExact(o[1]) || !as_int(o[2], dev) || dev < 0) return nullptr;
-    const Py_ssize_t N = PyList_GET_SIZE(o[1]);
-    if (!fits32(N)) return nullptr;
-    std::vector<int32_t> ids(static_cast<size_t>(N));
-    for (Py_ssize_t i = 0; i < N; ++i) {
-      long x;
-      if (!as_int(PyList_GET_ITEM(o[1], i), x) || x < INT32_MIN || x > INT32_MAX) return nullptr;
-      ids[static_cast<size_t>(i)] = static_cast<int32_t>(x);
-    }
-    const at::Tensor t = fresh({N}, at::kInt, static_cast<int>(dev));
-    int32_t* to = static_cast<int32_t*>(t.data_ptr());
-    if (!launch(static_cast<int>(dev), [&](void* s) { return tab->write_ids(to, ids.data(), static_cast<int32_t>(N), s); }))
-      return nullptr;
-    return THPVariable_Wrap(t);
-  });
-}
-
 // (address of each entry point, in the order of Table) -> the table's address; it lives as long as the process
 PyObject* make_table(PyObject*, PyObject* const* o, Py_ssize_t n) {
   if (n != kEntries) {
@@ -603,7 +579,7 @@ PyObject* make_table(PyObject*, PyObject* const* o, Py_ssize_t n) {
 #define CARRY_FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {CARRY_FAST(make_table), CARRY_FAST(packed_decode), CARRY_FAST(quant_step), CARRY_FAST(quant_decode), CARRY_FAST(quant_chain),
                          CARRY_FAST(fp32_step), CARRY_FAST(pool_move), CARRY_FAST(pool_copy), CARRY_FAST(pool_copy_layers),
-                         CARRY_FAST(ids_tensor), {nullptr, nullptr, 0, nullptr}};
+                         {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", "Native call path of the Python surfaces.", -1, methods};
 
 }  // namespace

@@ -149,18 +149,13 @@ class SlotCache:
 
     def indices(self, requests: Iterable, pad_to: Optional[int] = None) -> torch.Tensor:
         """``ssm_state_indices`` (int32, on the pools' device) for a batch of running requests;
-        ``None`` entries and the tail up to ``pad_to`` become the padding id 0."""
+        ``None`` entries and the tail up to ``pad_to`` become the padding id 0.  The ids are in place when
+        this returns (any stream may read them), which waits for what is queued on the current stream."""
         ids: List[int] = [NULL_SLOT if r is None else self._slot_of[r] for r in requests]
         if pad_to is not None:
             if pad_to < len(ids):
                 raise ValueError("pad_to is shorter than the batch")
             ids += [NULL_SLOT] * (pad_to - len(ids))
-        if self.device.type == "cuda" and ids:
-            lib = _lib._lib or _lib.load_library()
-            # as kernel arguments: a copy from pageable memory would wait for everything ahead in the stream
-            made = lib.native.ids_tensor(lib.native_table, ids, self.pools[0][0].get_device())
-            if made is not None:
-                return made
         return torch.tensor(ids, dtype=torch.int32, device=self.device)
 
     # ---- moves ------------------------------------------------------------

@@ -319,13 +319,6 @@ typedef struct CarryGdnPoolCopyLayersArgs {
 
 int carry_gdn_pool_copy_layers(const CarryGdnPoolCopyLayersArgs* args, void* stream);
 
-/*
- * Write n int32 values (slot ids) from host memory to device memory in stream
- * order.  They travel as kernel arguments: the call reads `ids` before it
- * returns and neither stages nor synchronises.
- */
-int carry_gdn_write_ids(int32_t* dst, const int32_t* ids, int32_t n, void* stream);
-
 /* Human-readable text for a CARRY_GDN_ERR_* code (static storage). */
 const char* carry_gdn_strerror(int code);
 

@@ -1,5 +1,5 @@
-"""The one-launch move of a slot through a stack of layers and the slot ids written as kernel arguments, at the
-edges of what one launch holds (48 layers, 960 ids) and with runs that are not multiples of 16 bytes."""
+"""The one-launch move of a slot through a stack of layers, at the edges of what one launch holds (48 layers) and with runs
+that are not multiples of 16 bytes; and the slot ids of a batch, whatever its length and on whatever stream they are read."""
 
 from __future__ import annotations
 
@@ -45,3 +45,26 @@ def test_indices_of_any_length(n):
     idx = c.indices(range(n), pad_to=n + 3)
     assert idx.dtype == torch.int32 and idx.is_cuda
     assert idx.tolist() == [c.slot(r) for r in range(n)] + [0, 0, 0]
+
+
+def test_indices_are_in_place_for_any_stream():
+    """Ids asked for on a stream that is busy are read by another one that waits for nothing."""
+    from carrykernel_b200.vllm_integration.state_cache import SlotCache
+    n = 1000
+    c = SlotCache(1, n + 1, 1, 2, 2, DEV)
+    for r in range(n):
+        c.allocate(r)
+    want = [c.slot(r) for r in range(n)]
+    busy, other = torch.cuda.Stream(), torch.cuda.Stream()
+    c.indices(range(n))                              # whatever is set up on first use
+    with torch.cuda.stream(busy):
+        stale = torch.full((n,), -5, dtype=torch.int32, device=DEV)      # what a block of this size holds
+        torch.cuda.synchronize()
+        del stale
+        torch.cuda._sleep(100_000_000)               # 50 ms
+        idx = c.indices(range(n))
+    with torch.cuda.stream(other):
+        seen = idx.clone()
+    other.synchronize()
+    assert seen.tolist() == want
+    busy.synchronize()
