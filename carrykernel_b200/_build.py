@@ -23,7 +23,6 @@ LIB = os.path.join(PKG, "libcarry_gdn.so")
 # that changed under the streaming kernel's feet.  Nothing in the package loads it.
 WAIT_TEST_LIB = os.path.join(PKG, "libcarry_gdn_waittest.so")
 # Native call path of the Python surfaces (CPython extension over torch's C++ tensors; no device code)
-NATIVE = os.path.join(PKG, "_native.so")
 NATIVE_SOURCE = "host_native.cpp"
 SOURCES = ("carry_gdn_api.cu", "carry_gdn_generic.cu", "carry_gdn_tile128.cu",
            "carry_gdn_tile128_vk.cu", "carry_gdn_tile128_kv.cu", "carry_gdn_multi.cu",
@@ -33,6 +32,14 @@ HEADERS = ("carry_gdn_common.cuh", "carry_gdn_tile128.cuh", "carry_gdn_slot_tile
 NVCC_FLAGS = ("-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xptxas", "-v", "-Xcompiler", "-fPIC")
 
+
+def native_path() -> str:
+    """Where the native call path lies.  It is good for one torch and one Python only, so both are in its name: after an
+    update of either there is none, and :func:`build` makes one."""
+    import sysconfig
+
+    import torch
+    return os.path.join(PKG, f"_native.torch-{torch.__version__}{sysconfig.get_config_var('EXT_SUFFIX')}")
 
 
 def _nvcc() -> str:
@@ -57,7 +64,7 @@ def _native_command(out: str):
 
 
 def is_stale() -> bool:
-    products = (LIB, WAIT_TEST_LIB, NATIVE)
+    products = (LIB, WAIT_TEST_LIB, native_path())
     if not all(os.path.exists(p) for p in products):
         return True
     built = min(os.path.getmtime(p) for p in products)
@@ -82,8 +89,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
     def compile_one(job):
         src, twin = job
         if src == NATIVE_SOURCE:
-            cmd = _native_command(NATIVE)
-            return NATIVE, cmd, subprocess.run(cmd, cwd=CSRC, capture_output=True, text=True)
+            cmd = _native_command(native_path())
+            return native_path(), cmd, subprocess.run(cmd, cwd=CSRC, capture_output=True, text=True)
         obj = os.path.join(obj_dir, src.replace(".cu", ".waittest.o" if twin else ".o"))
         cmd = [nvcc, *NVCC_FLAGS, *(("-DCARRY_TEST_WAIT_EXPIRY",) if twin else ()), "-c", "-o", obj, src]
         proc = subprocess.run(cmd, cwd=CSRC, capture_output=True, text=True)

@@ -1,14 +1,18 @@
 """ctypes binding of ``libcarry_gdn.so`` (the C ABI in ``include/carry_gdn.h``).
 
 The structures below mirror the header field for field.  There is no fallback:
-if the shared object is missing or a call fails, an exception is raised.
+if the shared object is missing or a call fails, an exception is raised.  (The
+native call path in front of it only saves host time: without it every call
+takes the Python checks and ctypes.)
 """
 
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import os
 import threading
+import warnings
 
 import torch
 
@@ -141,6 +145,24 @@ _lib = None
 _lock = threading.Lock()
 
 
+class _NoNative:
+    """In the native call path's place where it cannot be loaded: takes no call, so every surface goes its Python way."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
+def _load_native():
+    from . import _build
+    path = _build.native_path()
+    if not os.path.exists(path):
+        raise ImportError(f"{path} is missing")
+    spec = importlib.util.spec_from_file_location(f"{__package__}._native", path)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module
+
+
 def load_library(path: str | None = None):
     """Load (once, thread-safe) and return the ctypes handle of the library."""
     global _lib
@@ -180,15 +202,14 @@ def load_library(path: str | None = None):
         if lib.carry_gdn_abi_version() != ABI_VERSION:
             raise CudaUnavailable(
                 f"ABI mismatch: library {lib.carry_gdn_abi_version()}, binding {ABI_VERSION}")
+        lib.native, lib.native_table = _NoNative(), None
         try:
-            from . import _native
-        except ImportError as exc:
-            raise CudaUnavailable(
-                f"the native call path is missing or cannot be loaded ({exc}): "
-                "build it with `python -m carrykernel_b200._build`") from exc
-        lib.native_table = _native.make_table(
-            *(C.cast(getattr(lib, name), C.c_void_p).value for name in _NATIVE_ENTRIES))
-        lib.native = _native
+            lib.native = _load_native()
+            lib.native_table = lib.native.make_table(
+                *(C.cast(getattr(lib, name), C.c_void_p).value for name in _NATIVE_ENTRIES))
+        except (ImportError, OSError) as exc:
+            warnings.warn(f"the native call path cannot be loaded ({exc}): calls go through ctypes and take some 20 us of host "
+                          "time each; `python -m carrykernel_b200._build` builds it for this torch", RuntimeWarning, stacklevel=2)
         _lib = lib
         return _lib
 

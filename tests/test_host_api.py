@@ -322,3 +322,23 @@ def test_scale_division_shortcut_is_exact(qmax):
         # float64 division then rounding to float32 is the float32 quotient: a double rounding could
         # only bite when the float64 quotient sits exactly on a float32 tie, which a/qmax with a 24-bit
         # a and qmax < 2^7 cannot do unless it is exact
+
+
+def test_native_call_path_is_loaded_and_belongs_to_this_torch(lib):
+    assert lib.native.__file__ == _build.native_path() and torch.__version__ in lib.native.__file__
+    assert lib.native_table
+
+
+def test_another_torch_makes_the_build_stale_and_leaves_the_ctypes_way(lib, monkeypatch):
+    """An update of torch: the extension built for the old one is not loaded, the build knows that it has work to do, and until
+    then every surface works without it."""
+    monkeypatch.setattr(_lib, "_lib", None)
+    monkeypatch.setattr(torch, "__version__", "99.0")
+    assert "99.0" in _build.native_path() and _build.is_stale()
+    with pytest.warns(RuntimeWarning, match="native call path"):
+        bare = _lib.load_library()
+    monkeypatch.undo()
+    monkeypatch.setattr(_lib, "_lib", bare)
+    assert bare.native.quant_step(bare.native_table, None) is None
+    with pytest.raises(_lib.CudaUnavailable):
+        sq.gdn_step_fused_fp32(*(torch.zeros(1, 1, 4, 4), *(torch.zeros(1, 1, 4),) * 3, *(torch.zeros(1, 1),) * 2))
