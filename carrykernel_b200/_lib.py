@@ -18,7 +18,7 @@ import torch
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(PKG, "libcarry_gdn.so")
-ABI_VERSION = 3
+ABI_VERSION = 4
 
 F32, BF16, F16 = 0, 1, 2
 RES_FP32, RES_FP16, RES_FP8, RES_INT8, RES_INT4, RES_NONE = 0, 1, 2, 3, 4, 5
@@ -179,6 +179,9 @@ def load_library(path: str | None = None):
             lib = C.CDLL(path)
         except OSError as exc:
             raise CudaUnavailable(f"cannot load {path}: {exc}") from exc
+        if not hasattr(lib, "carry_gdn_abi_version") or lib.carry_gdn_abi_version() != ABI_VERSION:
+            found = lib.carry_gdn_abi_version() if hasattr(lib, "carry_gdn_abi_version") else "unknown"
+            raise CudaUnavailable(f"ABI mismatch: {path} is version {found}, the binding is version {ABI_VERSION}")
         for name in EXPORTS:
             if not hasattr(lib, name):
                 raise CudaUnavailable(f"{path} does not export {name}")
@@ -199,9 +202,6 @@ def load_library(path: str | None = None):
                    lib.carry_gdn_packed_decode_multi, lib.carry_gdn_pool_store, lib.carry_gdn_pool_load,
                    lib.carry_gdn_pool_copy, lib.carry_gdn_pool_copy_layers, lib.carry_gdn_quant_decode):
             fn.restype = C.c_int
-        if lib.carry_gdn_abi_version() != ABI_VERSION:
-            raise CudaUnavailable(
-                f"ABI mismatch: library {lib.carry_gdn_abi_version()}, binding {ABI_VERSION}")
         lib.native, lib.native_table = _NoNative(), None
         try:
             lib.native = _load_native()

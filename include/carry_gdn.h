@@ -24,7 +24,7 @@
 extern "C" {
 #endif
 
-#define CARRY_GDN_ABI_VERSION 3
+#define CARRY_GDN_ABI_VERSION 4
 
 /* element types of activations / outputs */
 enum { CARRY_F32 = 0, CARRY_BF16 = 1, CARRY_F16 = 2 };

@@ -342,3 +342,14 @@ def test_another_torch_makes_the_build_stale_and_leaves_the_ctypes_way(lib, monk
     assert bare.native.quant_step(bare.native_table, None) is None
     with pytest.raises(_lib.CudaUnavailable):
         sq.gdn_step_fused_fp32(*(torch.zeros(1, 1, 4, 4), *(torch.zeros(1, 1, 4),) * 3, *(torch.zeros(1, 1),) * 2))
+
+
+def test_a_library_of_an_older_abi_is_named_as_such(tmp_path, monkeypatch):
+    """The version stands for the set of entry points: carry_gdn_quant_decode and carry_gdn_pool_copy_layers came with 4."""
+    import subprocess
+    src, old = tmp_path / "old.c", tmp_path / "old.so"
+    src.write_text("int carry_gdn_abi_version(void) { return 3; }\n")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(old), str(src)], check=True)
+    monkeypatch.setattr(_lib, "_lib", None)
+    with pytest.raises(_lib.CudaUnavailable, match="ABI mismatch.*version 3.*version 4"):
+        _lib.load_library(str(old))
