@@ -247,31 +247,60 @@ def test_multi_token_kernel_wait_runs_out():
         assert torch.equal(x_bad[mask], x_good[mask])
 
 
-def test_statequant_layout_kernel_wait_runs_out():
+def _statequant_case(B, HV, res_fmt):
+    """``run(status)`` of one step into outputs that show what was not written, and which kernel took it."""
     from carrykernel_b200 import _lib
     from carrykernel_b200.statequant import kernel as sq
-    B, HV, K, V = 3, 8, 128, 128
-    h0, q, k, v, alpha, beta = seeded_inputs(B, HV, K, V, seed=4, alpha_mode="gated")
-    st = [x.to(DEV) for x in orc.init_quant_state(h0, 8, orc.RES_INT8)]
+    h0, q, k, v, alpha, beta = seeded_inputs(B, HV, 128, 128, seed=4, alpha_mode="gated")
+    st = [None if x is None else x.to(DEV) for x in orc.init_quant_state(h0, 8, res_fmt)]
     acts = [x.to(DEV) for x in (q, k, v, alpha, beta)]
 
     def run(status):
-        outs = (torch.full((B, HV, V), float("nan"), device=DEV), torch.full_like(st[0], 77),
-                torch.full_like(st[1], -1.0), torch.full_like(st[2], 77), torch.full_like(st[3], -1.0))
-        sq.quant_step_into(*st, *acts, outs, 8, orc.RES_INT8, "v", "v", status=status)
+        outs = [torch.full((B, HV, 128), -3.0, device=DEV)]
+        outs += [None if x is None else torch.full_like(x.float(), -3.0).to(x.dtype) for x in st]
+        sq.quant_step_into(*st, *acts, outs, 8, res_fmt, "v", "v", status=status)
+        kernel = _lib.load_library().carry_gdn_last_kernel()
         torch.cuda.synchronize()
-        return outs
+        return [x.float() for x in outs if x is not None], kernel
 
+    return run
+
+
+# the streaming kernel (floating-point residuals) and the kernel with 16 warps per tile (the others)
+@pytest.mark.parametrize("res_fmt,kernel", [(orc.RES_FP32, 2), (orc.RES_FP8, 2), (orc.RES_INT8, 2), (orc.RES_INT4, 2), (orc.RES_NONE, 5)])
+def test_statequant_layout_kernel_wait_runs_out(res_fmt, kernel):
+    from carrykernel_b200 import _lib
+    B, HV = 3, 8
+    run = _statequant_case(B, HV, res_fmt)
     status = torch.zeros(1, dtype=torch.int32, device=DEV)
-    good = run(status)
-    assert int(status.item()) == 0
+    good, took = run(status)
+    assert int(status.item()) == 0 and took == kernel
     with wait_test_library():
-        bad = run(status)
-    assert int(status.item()) == _lib.STATUS_TIMEOUT
+        bad, took = run(status)
+    assert int(status.item()) == _lib.STATUS_TIMEOUT and took == kernel
     n, head = 0, 1
-    assert torch.isnan(bad[0][n, head]).all()
-    assert torch.all(bad[1][n, head] == 77) and torch.all(bad[2][n, head] == -1) and torch.all(bad[3][n, head] == 77)
     keep = torch.ones(B, HV, dtype=torch.bool, device=DEV)
     keep[n, head] = False
     for x_bad, x_good in zip(bad, good):
+        assert torch.all(x_bad[n, head] == -3)
         assert torch.equal(x_bad[keep], x_good[keep])
+
+
+@pytest.mark.parametrize("res_fmt", [orc.RES_INT8, orc.RES_NONE])
+def test_statequant_layout_kernel_wait_runs_out_with_more_tiles_requested(res_fmt):
+    """The CTA whose first tile never arrives has the next ones on their way: it leaves all of its tiles untouched."""
+    from carrykernel_b200 import _lib
+    ctas = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    HV = 8
+    B = 5 * ctas // HV + 1
+    run = _statequant_case(B, HV, res_fmt)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    good, _ = run(status)
+    assert int(status.item()) == 0
+    with wait_test_library():
+        bad, _ = run(status)
+    assert int(status.item()) == _lib.STATUS_TIMEOUT
+    stopped = (torch.arange(B * HV, device=DEV) % ctas == 1).view(B, HV)
+    for x_bad, x_good in zip(bad, good):
+        assert torch.all(x_bad[stopped] == -3)
+        assert torch.equal(x_bad[~stopped], x_good[~stopped])
