@@ -219,6 +219,7 @@ int launch_dependent(void (*kern)(P...), dim3 grid, unsigned threads, size_t sme
 }
 
 // kernels / launchers implemented in the other translation units
+int sm_count();
 int launch_generic(const KParams& p, cudaStream_t stream);
 int launch_fp32(const CarryGdnFp32Args& a, cudaStream_t stream);
 bool tile128_eligible(const KParams& p);

@@ -25,6 +25,7 @@ namespace {
 struct MultiExtra {
   int T;
   long long stride_mixed_t, stride_a_t, stride_b_t;   // elements from one token of a request to the next
+  int first_wave;                                     // CTAs that the device holds at once
 };
 
 template <int RES, int RSCALE, int QDT>
@@ -53,8 +54,7 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_multi_kernel(const __grid_con
   // behind the first wave find the launch ahead finished, and the look at the index is in their way: hints from all
   // of them, 66.4 and 41.9 us.
   depend_release();
-  constexpr int kFirstWave = 2 * 148;                // two CTAs on each SM
-  if (tid == 0 && blockIdx.x < kFirstWave) {
+  if (tid == 0 && (int)blockIdx.x < x.first_wave) {
     const long long guess = __ldcg(p.slot_idx + (long long)n * p.stride_idx);
     if (guess > 0 && guess < p.num_slots) {
       unsigned long long a8[8];
@@ -225,7 +225,9 @@ int launch_multi(const KParams& p_in, int T, long long stride_mixed_t, long long
                  cudaStream_t stream) {
   KParams p = p_in;
   fill_shifts(p);
-  MultiExtra x = {T, stride_mixed_t, stride_a_t, stride_b_t};
+  const int sms = sm_count();
+  if (sms == 0) return CARRY_GDN_ERR_NO_DEVICE;
+  MultiExtra x = {T, stride_mixed_t, stride_a_t, stride_b_t, 2 * sms};
   const bool i4 = p.res_fmt == CARRY_RES_INT4, pv = p.rscale_mode == CARRY_SCALE_PER_V;
   if (i4) return pv ? launch_multi_dtype<CARRY_RES_INT4, CARRY_SCALE_PER_V>(p, x, stream)
                     : launch_multi_dtype<CARRY_RES_INT4, CARRY_SCALE_PER_HEAD>(p, x, stream);

@@ -40,24 +40,27 @@ bool tile128_eligible(const KParams& p) {
   return true;
 }
 
-int launch_tile128(const KParams& p, cudaStream_t stream) {
+// SMs of the current device; 0 when there is none that the launchers can keep a record of
+int sm_count() {
   static thread_local int sms[64] = {0};
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return CARRY_GDN_ERR_NO_DEVICE;
-  if (dev >= 64) return CARRY_GDN_ERR_NO_DEVICE;
-  if (sms[dev] == 0) {
-    if (cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms[dev] <= 0) {
-      cudaGetLastError();
-      sms[dev] = 0;
-      return CARRY_GDN_ERR_NO_DEVICE;
-    }
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return 0;
+  if (sms[dev] == 0 && (cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms[dev] < 0)) {
+    cudaGetLastError();
+    sms[dev] = 0;
   }
+  return sms[dev];
+}
+
+int launch_tile128(const KParams& p, cudaStream_t stream) {
+  const int sms = sm_count();
+  if (sms == 0) return CARRY_GDN_ERR_NO_DEVICE;
   KParams q = p;
   fill_shifts(q);
-  if (q.packed) return launch_tile128_vk(q, stream, sms[dev]);
+  if (q.packed) return launch_tile128_vk(q, stream, sms);
   const bool float_resid = q.res_fmt == CARRY_RES_FP32 || q.res_fmt == CARRY_RES_FP16 || q.res_fmt == CARRY_RES_FP8;
   // A floating-point residual needs a stage of up to 82 KB: no room for two CTAs, so it stays with one of two groups.
-  return float_resid ? launch_tile128_kv(q, stream, sms[dev]) : launch_dense128(q, stream, sms[dev]);
+  return float_resid ? launch_tile128_kv(q, stream, sms) : launch_dense128(q, stream, sms);
 }
 
 }  // namespace carry
