@@ -226,12 +226,12 @@ __global__ void __launch_bounds__(kPair, RES == CARRY_RES_NONE ? 8 : 6) gdn_dens
   uint8_t* eout = reinterpret_cast<uint8_t*>(p.resid_out) + nh * kN * kRow + g * kRow + (kInt4 ? c0 / 2 : c0);
   constexpr float rqmax = kInt4 ? 7.0f : 127.0f;
   float eamax[4] = {0.f, 0.f, 0.f, 0.f}, es[4], ei[4];
-  auto put_resid_scales = [&]() {
+  auto put_resid_scales = [&](const float (&s)[4]) {
     if (kHeadResid) {
-      if (tid == 0) p.rscale_out[nh] = es[0];
+      if (tid == 0) p.rscale_out[nh] = s[0];
     } else if (g == 0) {
 #pragma unroll
-      for (int b = 0; b < 4; ++b) p.rscale_out[nh * kN + c0 + b] = es[b];
+      for (int b = 0; b < 4; ++b) p.rscale_out[nh * kN + c0 + b] = s[b];
     }
   };
   if (__any_sync(kAll, !finite || !(snew[0] + snew[1] + snew[2] + snew[3] < inf))) {      // (one vote per warp: scales() meets)
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(kPair, RES == CARRY_RES_NONE ? 8 : 6) gdn_dens
     for (int b = 0; b < 4; ++b) eamax[b] = quantize_column_plainly(plain + b, snew[b], p.qmax, cout + b, 4 * kN, 0);
     if constexpr (!kNone) {
       scales(eamax, kHeadResid, rqmax, es, ei);
-      put_resid_scales();
+      put_resid_scales(es);
 #pragma unroll
       for (int b = 0; b < 4; ++b)
         quantize_column_plainly(plain + b, es[b], rqmax, reinterpret_cast<int8_t*>(eout) + (kInt4 ? b / 2 : b), 4 * kRow, kInt4 ? 1 + (b & 1) : 0);
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(kPair, RES == CARRY_RES_NONE ? 8 : 6) gdn_dens
   }
   if constexpr (!kNone) {
     scales(eamax, kHeadResid, rqmax, es, ei);
-    put_resid_scales();
+    put_resid_scales(es);
     if (kHeadResid && !(es[0] < inf)) ei[0] = ei[1] = ei[2] = ei[3] = 0.f;      // from the other warp's columns
     const float2 ieA = make_float2(ei[0], ei[1]), ieB = make_float2(ei[2], ei[3]);
 #pragma unroll

@@ -134,7 +134,6 @@ __device__ __noinline__ float quantize_row_plainly(float* x, float s, float qmax
 template <int RES, int RSCALE, int QDT>
 __global__ void __launch_bounds__(kPair, 6) gdn_narrow_kernel(const __grid_constant__ KParams p) {
   constexpr bool kInt4 = RES == CARRY_RES_INT4, kPerV = RSCALE == CARRY_SCALE_PER_V;
-  constexpr int qes = (QDT == CARRY_F32) ? 4 : 2;
   constexpr int kRowR = kInt4 ? kN / 2 : kN, kPitchR = kInt4 ? kPitch4 : kPitch;   // residual: bytes of a row, and staged
   __shared__ __align__(16) uint8_t codes_all[2][kRows * kPitch];
   __shared__ __align__(16) uint8_t resid_all[2][kRows * kPitchR];

@@ -195,9 +195,6 @@ __device__ __forceinline__ uint32_t order_token() {
 __device__ __forceinline__ void stg_b32(unsigned long long addr, uint32_t v) {
   asm volatile("st.global.b32 [%0], %1;" ::"l"(addr), "r"(v) : "memory");
 }
-__device__ __forceinline__ void stg_b16(unsigned long long addr, uint32_t v) {
-  asm volatile("st.global.b16 [%0], %1;" ::"l"(addr), "h"((unsigned short)v) : "memory");
-}
 
 // The 8 warps of a group meet on a hardware named barrier (ids 1..3 for group 0, 4..6 for group 1).
 // Every thread of a group runs the same tiles and reaches the same number of meetings in each of them
@@ -272,15 +269,8 @@ __device__ __forceinline__ uint32_t float4_to_e5m2x4(float2 ab, float2 cd) {
   const uint32_t hi = __nv_cvt_float2_to_fp8x2(cd, __NV_SATFINITE, __NV_E5M2);
   return lo | (hi << 16);
 }
-// bytes A and B of w (each nibble already XOR-ed with 8): {low nibbles}, {16 * high nibbles}
-template <int A, int B>
-__device__ __forceinline__ void s4x4_to_float(uint32_t w, float2& lo, float2& hi16) {
-  const uint32_t a = __byte_perm(w, 0x4B000000u, 0x7440 | A), b = __byte_perm(w, 0x4B000000u, 0x7440 | B);
-  lo = add2(make_float2(__uint_as_float(a & 0xFFFFFF0Fu), __uint_as_float(b & 0xFFFFFF0Fu)), splat(-kMagicNib));
-  hi16 = add2(make_float2(__uint_as_float(a & 0xFFFFFFF0u), __uint_as_float(b & 0xFFFFFFF0u)), splat(-kMagicByte));
-}
-// the same from a word whose low nibbles (wl = w & 0x0F0F0F0F) and high nibbles (wh = w & 0xF0F0F0F0)
-// were separated beforehand: two masks per word instead of four per byte pair
+// bytes A and B of a word whose low nibbles (wl = w & 0x0F0F0F0F) and high nibbles (wh = w & 0xF0F0F0F0) were separated
+// beforehand, each nibble already XOR-ed with 8: {low nibbles}, {16 * high nibbles}
 template <int A, int B>
 __device__ __forceinline__ void s4x4_split_to_float(uint32_t wl, uint32_t wh, float2& lo, float2& hi16) {
   lo = add2(make_float2(__uint_as_float(__byte_perm(wl, 0x4B000000u, 0x7440 | A)),
