@@ -8,7 +8,7 @@
 // delta, the scales and their reciprocals) in shared memory (four lanes per column, over all 16 warps, measured 5 % slower:
 // more instructions in all); a scale per head needs one maximum per warp
 // only.  256 requests x 32 heads, against that shape: no residual, one scale per head 129 -> 98 us, per V 133 -> 105; int8
-// residual 164 -> 147, int4 172 -> 152 (one scale per head); 16 requests, int8 16.7 -> 13.2.
+// residual 164 -> 147, int4 172 -> 150 (one scale per head); 16 requests, int8 16.7 -> 13.2.
 //
 // A CTA is persistent (tile = blockIdx.x + number * gridDim.x) and loads with bulk copies into a ring of up to 4 stages; a
 // stage is requested again after the meeting behind the last read of it.  Addresses follow from the tile's index, the

@@ -240,10 +240,10 @@ __device__ __forceinline__ float2 nib2_biased(uint32_t w) {
                      __uint_as_float(__byte_perm(w, 0x43000000u, 0x7044 | (B << 8))));
 }
 // four int4 codes in two bytes (even index in the low nibble) -> {code 0, code 1}, {code 2, code 3}, exact.  (Leaving the
-// 136 of the biased nibble to a later addend takes an instruction less per pair -- 151.5 us instead of 150.4 with one scale
-// per head, 256 requests x 32 heads of 128 -- but every target then passes through a sum of that size: 136 residual
-// steps, which a residual scale that belongs to a larger column makes as large as one likes against the column's own
-// step: 4.6e-3 of the state codes of a column 1e4 times below the largest came out one off.)
+// 136 of the biased nibble to a later addend takes an instruction less per pair -- 1 us of 150 with one scale per head,
+// 256 requests x 32 heads of 128 -- but every target then passes through a sum of that size: 136 residual steps,
+// which a residual scale that belongs to a larger column makes as large as one likes against the column's own step:
+// 4.6e-3 of the state codes of a column 1e4 times below the largest came out one off.)
 __device__ __forceinline__ void s4x4_pairs(uint32_t w, float2& a, float2& b) {
   const uint32_t lo = (w ^ 0x8888u) & 0x0F0Fu, hi = ((w ^ 0x8888u) >> 4) & 0x0F0Fu;
   const float2 bias = splat(-136.0f);
