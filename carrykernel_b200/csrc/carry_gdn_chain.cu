@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_chain_kernel(const __grid_con
     // new scales, codes, residual
     const float4 s4 = *reinterpret_cast<const float4*>(scale_of + c0), i4 = *reinterpret_cast<const float4*>(inv_of + c0);
     scol[0] = s4.x; scol[1] = s4.y; scol[2] = s4.z; scol[3] = s4.w;
-    const float thr[4] = {s4.x * kTieGuard, s4.y * kTieGuard, s4.z * kTieGuard, s4.w * kTieGuard};
+    const float thr[4] = {s4.x * kTieGuardExact, s4.y * kTieGuardExact, s4.z * kTieGuardExact, s4.w * kTieGuardExact};
     const float2 invA = make_float2(i4.x, i4.y), invB = make_float2(i4.z, i4.w);
     const float2 nsA = make_float2(-scol[0], -scol[1]), nsB = make_float2(-scol[2], -scol[3]);
     float eamax[4] = {0.f, 0.f, 0.f, 0.f};
@@ -254,13 +254,7 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_chain_kernel(const __grid_con
     }
     if (fmaxf(fmaxf(eamax[0] - thr[0], eamax[1] - thr[1]), fmaxf(eamax[2] - thr[2], eamax[3] - thr[3])) > 0.f) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {                      // a quotient within the tie guard
-        float2 yA = add2(s8x2_to_float<0, 1>(cw[i] ^ 0x80808080u), magic2);
-        float2 yB = add2(s8x2_to_float<2, 3>(cw[i] ^ 0x80808080u), magic2);
-        redecide_rec(hA[i].x, yA.x, scol[0], thr[0]); redecide_rec(hA[i].y, yA.y, scol[1], thr[1]);
-        redecide_rec(hB[i].x, yB.x, scol[2], thr[2]); redecide_rec(hB[i].y, yB.y, scol[3], thr[3]);
-        cw[i] = pack4(__float_as_uint(yA.x), __float_as_uint(yA.y), __float_as_uint(yB.x), __float_as_uint(yB.y));
-      }
+      for (int i = 0; i < 16; ++i) redecide_quad(hA[i], hB[i], cw[i], scol, thr);      // a quotient within the tie guard (whole columns: 254 us instead of 241)
     }
     if (t + 1 < x.T) {
 #pragma unroll

@@ -301,15 +301,15 @@ __global__ void __launch_bounds__(kWide, 2) gdn_dense128_kernel(const __grid_con
           m[2] = fmaxf(fmaxf(m[2], fabsf(hB[i - 1].x)), fabsf(hB[i].x)); m[3] = fmaxf(fmaxf(m[3], fabsf(hB[i - 1].y)), fabsf(hB[i].y));
         }
       }
-      const float2 thA = mul2(snA, splat(kTieGuard)), thB = mul2(snB, splat(kTieGuard));
+      const float2 thA = mul2(snA, splat(kTieGuardExact)), thB = mul2(snB, splat(kTieGuardExact));
+      // One warp in 40 has a quotient within the tie guard, and all sixteen wait for it at the next meeting: only the rows with
+      // such an element are gone through again (all eight: 97.6 us instead of 95.8, 256 requests x 32 heads, no residual).
       if (fmaxf(fmaxf(m[0] - thA.x, m[1] - thA.y), fmaxf(m[2] - thB.x, m[3] - thB.y)) > 0.f) {
-        m[0] = m[1] = m[2] = m[3] = 0.f;                 // rare: a quotient within the tie guard
+        const float sn[4] = {snA.x, snA.y, snB.x, snB.y}, thr[4] = {thA.x, thA.y, thB.x, thB.y};
+        m[0] = m[1] = m[2] = m[3] = 0.f;
 #pragma unroll
         for (int i = 0; i < kLaneRows; ++i) {
-          float2 yA = add2(s8x2_to_float<0, 1>(cw[i] ^ 0x80808080u), magic2), yB = add2(s8x2_to_float<2, 3>(cw[i] ^ 0x80808080u), magic2);
-          redecide_rec(hA[i].x, yA.x, snA.x, thA.x); redecide_rec(hA[i].y, yA.y, snA.y, thA.y);
-          redecide_rec(hB[i].x, yB.x, snB.x, thB.x); redecide_rec(hB[i].y, yB.y, snB.y, thB.y);
-          cw[i] = pack4(__float_as_uint(yA.x), __float_as_uint(yA.y), __float_as_uint(yB.x), __float_as_uint(yB.y));
+          redecide_quad(hA[i], hB[i], cw[i], sn, thr);
           m[0] = fmaxf(m[0], fabsf(hA[i].x)); m[1] = fmaxf(m[1], fabsf(hA[i].y));
           m[2] = fmaxf(m[2], fabsf(hB[i].x)); m[3] = fmaxf(m[3], fabsf(hB[i].y));
         }

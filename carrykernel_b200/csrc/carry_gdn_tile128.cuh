@@ -33,7 +33,7 @@
 // remainder = fma(code', -scale', target).  Scales are amax / qmax by an exact
 // shortcut (div_qmax).  round(target / s) is evaluated as rint(target * (1/s)) with a
 // reciprocal good to 2^-24; the two can only differ when the quotient is within ~8e-6
-// of a tie, which shows up as a remainder within 2^-16 of half a step -- rows where
+// of a tie, which shows up as a remainder within 1.2e-5 of half a step -- elements where
 // that happens are re-decided with the true division.  Residual codes use
 // rint(e * (1/es)) as is.  Math runs as packed f32x2 (IEEE round-to-nearest per
 // component).
@@ -216,6 +216,11 @@ constexpr float kMagicRound = 12582912.0f;      // 1.5 * 2^23: x + M rounds x to
 constexpr float kMagicByte = 8388736.0f;        // 2^23 + 128
 constexpr float kMagicNib = 8388616.0f;         // 2^23 + 8
 constexpr float kTieGuard = 0.4999847412109375f;  // 0.5 - 2^-16
+// The same where the remainder target - code * scale is one fused multiply-add, and so exact: in units of the step, the
+// reciprocal moves a quotient of at most 127 by 127 * 2^-24 (1 + 2^-20) = 7.6e-6, rounding the true one to fp32 by half a unit
+// in the last place, 3.9e-6, and the threshold is rounded by 3e-8: 1.2e-5 covers the sum.  (kTieGuard has room for a product
+// that was rounded before it was subtracted.)
+constexpr float kTieGuardExact = 0.499988f;
 
 // bytes A and B of w (each already XOR-ed with 0x80) -> {float(code A), float(code B)}
 template <int A, int B>
@@ -453,6 +458,16 @@ __device__ __forceinline__ void redecide_rec(float& e, float& y, float s, float 
     const float code = exact_code(t, s);
     y = __fadd_rn(code, kMagicRound);
     e = fmaf(code, -s, t);
+  }
+}
+
+// ... of four neighbouring columns of one row, each with its own scale: nothing is done unless one of them is within the guard.
+__device__ __forceinline__ void redecide_quad(float2& a, float2& b, uint32_t& cw, const float (&s)[4], const float (&thr)[4]) {
+  if ((fabsf(a.x) > thr[0]) | (fabsf(a.y) > thr[1]) | (fabsf(b.x) > thr[2]) | (fabsf(b.y) > thr[3])) {
+    float2 yA = add2(s8x2_to_float<0, 1>(cw ^ 0x80808080u), splat(kMagicRound)), yB = add2(s8x2_to_float<2, 3>(cw ^ 0x80808080u), splat(kMagicRound));
+    redecide_rec(a.x, yA.x, s[0], thr[0]); redecide_rec(a.y, yA.y, s[1], thr[1]);
+    redecide_rec(b.x, yB.x, s[2], thr[2]); redecide_rec(b.y, yB.y, s[3], thr[3]);
+    cw = pack4(__float_as_uint(yA.x), __float_as_uint(yA.y), __float_as_uint(yB.x), __float_as_uint(yB.y));
   }
 }
 
@@ -1136,7 +1151,7 @@ gdn_tile128_kernel(const __grid_constant__ KParams p) {
         }
         float snew[4], thr[4];
 #pragma unroll
-        for (int b = 0; b < 4; ++b) { snew[b] = scale_fast(amax[b], p.qmax, rqmax_state, p.eps_mode); thr[b] = snew[b] * kTieGuard; }
+        for (int b = 0; b < 4; ++b) { snew[b] = scale_fast(amax[b], p.qmax, rqmax_state, p.eps_mode); thr[b] = snew[b] * kTieGuardExact; }
         const float2 invA = make_float2(rcp_refined(snew[0]), rcp_refined(snew[1]));
         const float2 invB = make_float2(rcp_refined(snew[2]), rcp_refined(snew[3]));
         const float2 nsA = make_float2(-snew[0], -snew[1]), nsB = make_float2(-snew[2], -snew[3]);
@@ -1154,17 +1169,8 @@ gdn_tile128_kernel(const __grid_constant__ KParams p) {
           }
         }
         if (fmaxf(fmaxf(eamax[0] - thr[0], eamax[1] - thr[1]), fmaxf(eamax[2] - thr[2], eamax[3] - thr[3])) > 0.f) {
-          eamax[0] = eamax[1] = eamax[2] = eamax[3] = 0.f;      // rare: a quotient within the tie guard
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            float2 yA = add2(s8x2_to_float<0, 1>(cw[i] ^ 0x80808080u), magic2);
-            float2 yB = add2(s8x2_to_float<2, 3>(cw[i] ^ 0x80808080u), magic2);
-            redecide_rec(hA[i].x, yA.x, snew[0], thr[0]); redecide_rec(hA[i].y, yA.y, snew[1], thr[1]);
-            redecide_rec(hB[i].x, yB.x, snew[2], thr[2]); redecide_rec(hB[i].y, yB.y, snew[3], thr[3]);
-            cw[i] = pack4(__float_as_uint(yA.x), __float_as_uint(yA.y), __float_as_uint(yB.x), __float_as_uint(yB.y));
-            eamax[0] = fmaxf(eamax[0], fabsf(hA[i].x)); eamax[1] = fmaxf(eamax[1], fabsf(hA[i].y));
-            eamax[2] = fmaxf(eamax[2], fabsf(hB[i].x)); eamax[3] = fmaxf(eamax[3], fabsf(hB[i].y));
-          }
+          for (int i = 0; i < 16; ++i) redecide_quad(hA[i], hB[i], cw[i], snew, thr);      // rare: a quotient within the tie guard
         }
         {
           const unsigned long long dst_codes = dst_of(D_CODES);
