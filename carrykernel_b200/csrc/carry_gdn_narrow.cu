@@ -12,9 +12,15 @@
 // Codes and residual come in by coalesced 16-byte asynchronous copies into rows padded against bank conflicts, while
 // gates and norms are worked out, and go out the same way.
 //
-// Measured (48 requests x 16 heads, int8 residual, 12 layers back to back from DRAM): 7.9 us per launch (8.3 without the hints
-// to the L2 ahead of the dependency wait), the generic kernel 79 us; 512 requests: 56 us (2.5 TB/s) against 540.  168 registers and 6 CTAs per SM, since the row is 64 of them:
-// at 128 registers and 8 CTAs 140 bytes spill and the launch takes 10 us.
+// Measured (48 requests x 16 heads, int8 residual, 12 layers back to back): 7.7 us per launch with the state in the L2, 8.0
+// out of it, 8.3 where inputs that repeat hold the state at a fixed point (ties in every row); the generic kernel 79 us.
+// 512 requests: 58 us (2.4 TB/s) against 540.  168 registers and 6 CTAs per SM, since the row is 64 of them: at 128
+// registers and 8 CTAs 140 bytes spill and the launch takes 10 us.
+//
+// Nothing touches memory ahead of the dependency wait.  Hints to the L2 for the slot that the index names then and for
+// q, k and v take the 8.3 us to 8.0 and the 8.0 to 7.9, but the wait waits for them too: behind a kernel that does not release
+// its dependents, as most of an engine's, a launch takes 0.9 us more (48 requests, 12 layers with another kernel ahead of each:
+// 156 -> 166 us; int4 146 -> 157), and back to back with the state in the L2 0.1 to 0.3 us more.
 #include "carry_gdn_tile128.cuh"
 
 namespace carry {
@@ -132,7 +138,7 @@ __device__ __noinline__ float quantize_row_plainly(float* x, float s, float qmax
 }
 
 template <int RES, int RSCALE, int QDT>
-__global__ void __launch_bounds__(kPair, 6) gdn_narrow_kernel(const __grid_constant__ KParams p, int first_wave) {
+__global__ void __launch_bounds__(kPair, 6) gdn_narrow_kernel(const __grid_constant__ KParams p) {
   constexpr bool kInt4 = RES == CARRY_RES_INT4, kPerV = RSCALE == CARRY_SCALE_PER_V;
   constexpr int kRowR = kInt4 ? kN / 2 : kN, kPitchR = kInt4 ? kPitch4 : kPitch;   // residual: bytes of a row, and staged
   __shared__ __align__(16) uint8_t codes_all[2][kRows * kPitch];
@@ -145,23 +151,6 @@ __global__ void __launch_bounds__(kPair, 6) gdn_narrow_kernel(const __grid_const
   split_tile(p, (int)blockIdx.x, n, hv, h);
 
   depend_release();
-  // While the launch ahead runs out: hints to the L2 for the rows of the slot that the index names now and for this tile's
-  // activations.  (CTAs beyond those the device holds at once start later and find it finished.)
-  if ((int)blockIdx.x < first_wave) {
-    if (lane == 0) {
-      const int guess = __ldcg(p.slot_idx + (long long)n * p.stride_idx);
-      if (guess > 0 && guess < p.num_slots) {
-        l2_prefetch_bulk(p.codes_out + guess * p.stride_state_slot + ((long long)hv * kN + kRows * warp) * kN, kRows * kN);
-        l2_prefetch_bulk(reinterpret_cast<const uint8_t*>(p.resid_out) + guess * p.stride_resid_slot + ((long long)hv * kN + kRows * warp) * kRowR, kRows * kRowR);
-        l2_prefetch_line(p.sscale_out + guess * p.stride_sscale_slot + (long long)hv * kN + kRows * warp);
-        l2_prefetch_line(p.rscale_out + guess * p.stride_rscale_slot + (kPerV ? (long long)hv * kN + kRows * warp : (long long)hv));
-      }
-    } else if (lane < 4) {                               // q, k, v
-      constexpr int qes = QDT == CARRY_F32 ? 4 : 2;
-      const long long at = lane == 1 ? (long long)h * kN : lane == 2 ? ((long long)p.H + h) * kN : 2LL * p.H * kN + (long long)hv * kN;
-      l2_prefetch_line(reinterpret_cast<const uint8_t*>(p.q) + ((long long)n * p.stride_mixed_tok + at) * qes);
-    }
-  }
   depend_wait();
   const int slot_id = p.slot_idx[(long long)n * p.stride_idx];
   const GateRaw raw = gate_loads(p, n, hv, 0, 0);
@@ -327,10 +316,9 @@ __global__ void __launch_bounds__(kPair, 6) gdn_narrow_kernel(const __grid_const
 template <int RES, int RSCALE>
 int launch_dtype64(const KParams& p, cudaStream_t stream) {
   const dim3 grid((unsigned)((long long)p.B * p.HV));
-  const int first_wave = 6 * sm_count();
-  if (p.qkv_dtype == CARRY_F32) return launch_dependent(gdn_narrow_kernel<RES, RSCALE, CARRY_F32>, grid, kPair, 0, stream, p, first_wave);
-  if (p.qkv_dtype == CARRY_BF16) return launch_dependent(gdn_narrow_kernel<RES, RSCALE, CARRY_BF16>, grid, kPair, 0, stream, p, first_wave);
-  return launch_dependent(gdn_narrow_kernel<RES, RSCALE, CARRY_F16>, grid, kPair, 0, stream, p, first_wave);
+  if (p.qkv_dtype == CARRY_F32) return launch_dependent(gdn_narrow_kernel<RES, RSCALE, CARRY_F32>, grid, kPair, 0, stream, p);
+  if (p.qkv_dtype == CARRY_BF16) return launch_dependent(gdn_narrow_kernel<RES, RSCALE, CARRY_BF16>, grid, kPair, 0, stream, p);
+  return launch_dependent(gdn_narrow_kernel<RES, RSCALE, CARRY_F16>, grid, kPair, 0, stream, p);
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
