@@ -324,6 +324,56 @@ def test_scale_division_shortcut_is_exact(qmax):
         # a and qmax < 2^7 cannot do unless it is exact
 
 
+def test_tie_guards_cover_the_reciprocal():
+    """Codes are rint(t * y), y the hardware's reciprocal of the scale s (within an ulp) after one Newton step, and are decided
+    again by rint(t / s) where the remainder is beyond the guard times s (carry_gdn_tile128.cuh: rcp_refined, kTieGuardExact
+    for remainders of one fused multiply-add, kTieGuard for products rounded first).  So: y is as close as the guards assume for
+    every mantissa, and no code differs without its remainder being beyond the guard, on either side of every tie.
+
+    float64 holds the products of two float32 exactly, and the differences of nearly equal numbers taken here."""
+    import re
+
+    import numpy as np
+    from carrykernel_b200 import _build
+    with open(f"{_build.CSRC}/carry_gdn_tile128.cuh") as src:
+        guards = {n: np.float32(v) for n, v in re.findall(r"constexpr float (kTieGuard\w*) = ([\d.]+)f;", src.read())}
+    assert set(guards) == {"kTieGuard", "kTieGuardExact"}
+    f32, f64 = np.float32, np.float64
+
+    def refined(s, ulps):
+        y = f32(1) / s
+        for _ in range(abs(ulps)):
+            y = np.nextafter(y, f32(2 if ulps > 0 else 0), dtype=f32)
+        r = f32(1.0 - s.astype(f64) * y)
+        return f32(y.astype(f64) * r + y)
+
+    s_all = (np.uint32(127 << 23) | np.arange(1 << 23, dtype=np.uint32)).view(f32)
+    for ulps in (-1, 0, 1):
+        y = refined(s_all, ulps)
+        assert np.abs(s_all.astype(f64) * y - 1.0).max() <= 2.0 ** -24 * (1 + 2.0 ** -20)
+
+    rng = np.random.default_rng(0)
+    s = np.concatenate([s_all[rng.integers(0, 1 << 23, 1 << 14)], s_all[:64], s_all[-64:]])[:, None]
+    n = np.arange(127, dtype=f64)[None, :]
+    tie = f32((n + 0.5) * s)
+    differ = beyond = 0
+    for ulps in (-1, 0, 1):
+        y = refined(s, ulps)
+        for off in range(-4, 5):                        # targets: the tie and four float32 on either side
+            t = (tie.view(np.int32) + np.int32(off)).view(f32)
+            fast, true = np.rint(t.astype(f64) * y), np.rint(f32(t / s))
+            wrong = fast != true
+            fused = np.abs(f32(t.astype(f64) - fast * s))
+            apart = np.abs(f32(t - f32(fast * s)))
+            for e, guard in ((fused, guards["kTieGuardExact"]), (apart, guards["kTieGuard"])):
+                assert np.all(e[wrong] > np.broadcast_to(f32(s * guard), e.shape)[wrong])
+                # the form f = fma(-s, guard, e) > 0
+                assert np.all((e.astype(f64) - s.astype(f64) * f64(guard))[wrong] > 0)
+            differ += int(wrong.sum())
+            beyond += int((wrong & (fused <= s * f32(0.5 - 2e-6))).sum())
+    assert differ > 1000 and beyond > 0            # a guard that is much narrower would fail here
+
+
 def test_native_call_path_is_loaded_and_belongs_to_this_torch(lib):
     assert lib.native.__file__ == _build.native_path() and torch.__version__ in lib.native.__file__
     assert lib.native_table
