@@ -40,13 +40,10 @@ def _pool(num_slots, HV, V, K, resid_fmt, rscale, seed):
     return list(orc.init_quantized_pool(num_slots, HV, V, K, h0=pool, resid_fmt=resid_fmt, resid_scale=rscale))
 
 
-@pytest.mark.parametrize("resid_fmt", [orc.RESID_INT4, orc.RESID_INT8])
-@pytest.mark.parametrize("rscale", ["head", "v"])
-@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
-def test_multi_equals_single_token_calls(resid_fmt, rscale, dtype):
+def _check_equals_single_token_calls(T, resid_fmt, rscale, dtype, H=16, HV=32):
     qpd = _qpd()
     from carrykernel_b200 import _lib
-    B, T, H, HV, K, V = 5, 3, 16, 32, 128, 128
+    B, K, V = 5, 128, 128
     num_slots = 9
     st = _pool(num_slots, HV, V, K, resid_fmt, rscale, seed=11)
     mixed, a, b, A_log, dt_bias = _inputs(B, T, H, HV, K, V, 5, dtype)
@@ -73,6 +70,21 @@ def test_multi_equals_single_token_calls(resid_fmt, rscale, dtype):
     for x, y in zip(got, ref):
         assert torch.equal(x, y)
     assert torch.all(out[1] == 0)
+
+
+@pytest.mark.parametrize("resid_fmt", [orc.RESID_INT4, orc.RESID_INT8])
+@pytest.mark.parametrize("rscale", ["head", "v"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_multi_equals_single_token_calls(resid_fmt, rscale, dtype):
+    _check_equals_single_token_calls(3, resid_fmt, rscale, dtype)
+
+
+@pytest.mark.parametrize("T", [1, 7, 8, 9, 17])
+@pytest.mark.parametrize("resid_fmt", [orc.RESID_INT4, orc.RESID_INT8])
+@pytest.mark.parametrize("rscale", ["head", "v"])
+def test_multi_equals_single_token_calls_across_chunks_of_activations(T, resid_fmt, rscale):
+    """The kernel fetches the activations of 8 tokens at a time; the refill is the only block barrier between tokens."""
+    _check_equals_single_token_calls(T, resid_fmt, rscale, torch.float16, H=4, HV=8)
 
 
 def test_multi_against_oracle():
