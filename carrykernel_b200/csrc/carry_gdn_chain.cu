@@ -5,11 +5,11 @@
 //
 // What it saves: 8 tokens of 64 requests x 32 heads with an fp32 residual were nine passes of eager kernels for the
 // initial state (0.4 ms) and 8 launches that each move 10 bytes per element (0.54 ms, at 85 % of the copy rate).  Here the
-// state crosses HBM once, 9 bytes per element in all, and the arithmetic bounds: 1021 -> 254 us.
+// state crosses HBM once, 9 bytes per element in all, and the arithmetic bounds: 1021 -> 241 us.
 //
 // One CTA of 8 warps per tile, two per SM.  Lane = 4 columns x the warp's 16 rows.  A column's sums and its maximum are
 // finished by one lane, through shared memory, and handed to the others the same way: four meetings per token.  (Every
-// warp finishing all 128 columns for itself needs two, but takes 306 us instead of 254.)  Codes stay in registers from
+// warp finishing all 128 columns for itself needs two, but took 306 us where this took 254.)  Codes stay in registers from
 // token to token, the residual in shared memory in its own format; a token's k and q are spread per warp as {k, k, q, q}
 // rows so that packed instructions read them as they are.
 #include "carry_gdn_tile128.cuh"
@@ -253,8 +253,9 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_chain_kernel(const __grid_con
       }
     }
     if (fmaxf(fmaxf(eamax[0] - thr[0], eamax[1] - thr[1]), fmaxf(eamax[2] - thr[2], eamax[3] - thr[3])) > 0.f) {
+      // a quotient within the tie guard: only its quad is gone through again (whole columns: 251 us instead of 241)
 #pragma unroll
-      for (int i = 0; i < 16; ++i) redecide_quad(hA[i], hB[i], cw[i], scol, thr);      // a quotient within the tie guard (whole columns: 254 us instead of 241)
+      for (int i = 0; i < 16; ++i) redecide_quad(hA[i], hB[i], cw[i], scol, thr);
     }
     if (t + 1 < x.T) {
 #pragma unroll

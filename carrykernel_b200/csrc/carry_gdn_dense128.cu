@@ -7,8 +7,8 @@
 // column's reduction is finished once, by its lane of the first four warps, which leaves what the others need (the
 // delta, the scales and their reciprocals) in shared memory (four lanes per column, over all 16 warps, measured 5 % slower:
 // more instructions in all); a scale per head needs one maximum per warp
-// only.  256 requests x 32 heads, against that shape: no residual, one scale per head 129 -> 98 us, per V 133 -> 105; int8
-// residual 164 -> 147, int4 172 -> 150 (one scale per head); 16 requests, int8 16.7 -> 13.2.
+// only.  256 requests x 32 heads, against that shape: no residual, one scale per head 129 -> 96 us, per V 133 -> 101; int8
+// residual 164 -> 138, int4 172 -> 145 (one scale per head); 16 requests, int8 16.7 -> 13.2.
 //
 // A CTA is persistent (tile = blockIdx.x + number * gridDim.x) and loads with bulk copies into a ring of up to 4 stages; a
 // stage is requested again after the meeting behind the last read of it.  Addresses follow from the tile's index, the
@@ -302,8 +302,9 @@ __global__ void __launch_bounds__(kWide, 2) gdn_dense128_kernel(const __grid_con
         }
       }
       const float2 thA = mul2(snA, splat(kTieGuardExact)), thB = mul2(snB, splat(kTieGuardExact));
-      // One warp in 40 has a quotient within the tie guard, and all sixteen wait for it at the next meeting: only the rows with
-      // such an element are gone through again (all eight: 97.6 us instead of 95.8, 256 requests x 32 heads, no residual).
+      // One warp in 40 has a quotient within the tie guard, and all sixteen wait for it at the next meeting: only the quads with
+      // such an element are gone through again (all eight: 97.0 us instead of 95.9 for 256 requests x 32 heads without a
+      // residual, 144.8 instead of 138.1 with int8 and one scale per head).
       if (fmaxf(fmaxf(m[0] - thA.x, m[1] - thA.y), fmaxf(m[2] - thB.x, m[3] - thB.y)) > 0.f) {
         const float sn[4] = {snA.x, snA.y, snB.x, snB.y}, thr[4] = {thA.x, thA.y, thB.x, thB.y};
         m[0] = m[1] = m[2] = m[3] = 0.f;

@@ -9,8 +9,12 @@
 // slot-layout tile body of the streaming kernel (carry_gdn_slot_tile.inc),
 // with its stores pointed at the staged tile instead of global memory; a warp
 // only ever reads and writes its own 16 rows of the tile, so tokens need no
-// ordering between warps beyond the body's own meeting, which only a residual scale per head has (that scale is carried in
-// a register: read back from the staged tile, it cost a block barrier per token, 524 us instead of 512 for 8 layers of 32 requests, 4 tokens).  Activation vectors, gates and norms
+// ordering between warps beyond the body's own meeting, which is empty unless
+// there is one residual scale per head.  That scale is carried in a register:
+// read back from the staged tile, it takes a block barrier per token (8 layers of
+// 32 requests, 4 tokens: 524 us instead of 513; with a scale per V row, where the
+// barrier held warps together that need nothing from one another, 538 instead of
+// 490 for int4, 535 instead of 488 for int8).  Activation vectors, gates and norms
 // of up to 8 tokens are fetched together, one trip to global memory per chunk of
 // tokens instead of one per token.
 #include "carry_gdn_tile128.cuh"

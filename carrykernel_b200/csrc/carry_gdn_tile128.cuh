@@ -215,11 +215,15 @@ __device__ __forceinline__ float max3abs(float m, float2 x) { return fmaxf(fmaxf
 constexpr float kMagicRound = 12582912.0f;      // 1.5 * 2^23: x + M rounds x to an integer (RNE)
 constexpr float kMagicByte = 8388736.0f;        // 2^23 + 128
 constexpr float kMagicNib = 8388616.0f;         // 2^23 + 8
+// Tie guards, in steps: a code whose remainder is beyond the guard is decided again by the true quotient.  In units of the
+// step, the reciprocal moves a quotient of at most 127 by 127 * 2^-24 (1 + 2^-20) = 7.6e-6, rounding the true one to fp32 by
+// half a unit in the last place, 3.9e-6, and the threshold is rounded by 3e-8: 1.2e-5 covers the sum where the remainder
+// target - code * scale is one fused multiply-add, and so exact (kTieGuardExact).  A product that is rounded before it is
+// subtracted may be off by another 7.6e-6, against 7.6e-6 of the reciprocal: 2^-16 covers that (kTieGuard).  Measured: codes
+// that differ have remainders within 3.9e-6 and 1.13e-5 of half a step (tests/test_host_api.py repeats it).  The narrower
+// guard matters where other warps wait for the one that looks again; where none does (64-wide heads, a chain's
+// initial state) kTieGuard serves both kinds of remainder.
 constexpr float kTieGuard = 0.4999847412109375f;  // 0.5 - 2^-16
-// The same where the remainder target - code * scale is one fused multiply-add, and so exact: in units of the step, the
-// reciprocal moves a quotient of at most 127 by 127 * 2^-24 (1 + 2^-20) = 7.6e-6, rounding the true one to fp32 by half a unit
-// in the last place, 3.9e-6, and the threshold is rounded by 3e-8: 1.2e-5 covers the sum.  (kTieGuard has room for a product
-// that was rounded before it was subtracted.)
 constexpr float kTieGuardExact = 0.499988f;
 
 // bytes A and B of w (each already XOR-ed with 0x80) -> {float(code A), float(code B)}
@@ -461,7 +465,8 @@ __device__ __forceinline__ void redecide_rec(float& e, float& y, float s, float 
   }
 }
 
-// ... of four neighbouring columns of one row, each with its own scale: nothing is done unless one of them is within the guard.
+// ... of four neighbouring columns of one row, each with its own scale: nothing is done unless one of them is within the
+// guard.
 __device__ __forceinline__ void redecide_quad(float2& a, float2& b, uint32_t& cw, const float (&s)[4], const float (&thr)[4]) {
   if ((fabsf(a.x) > thr[0]) | (fabsf(a.y) > thr[1]) | (fabsf(b.x) > thr[2]) | (fabsf(b.y) > thr[3])) {
     float2 yA = add2(s8x2_to_float<0, 1>(cw ^ 0x80808080u), splat(kMagicRound)), yB = add2(s8x2_to_float<2, 3>(cw ^ 0x80808080u), splat(kMagicRound));
@@ -1168,9 +1173,12 @@ gdn_tile128_kernel(const __grid_constant__ KParams p) {
             eamax[2] = fmaxf(fmaxf(eamax[2], fabsf(hB[i - 1].x)), fabsf(hB[i].x)); eamax[3] = fmaxf(fmaxf(eamax[3], fabsf(hB[i - 1].y)), fabsf(hB[i].y));
           }
         }
+        // One warp in 20 has a quotient within the tie guard, and the others wait for it at the next meeting: only the quads
+        // with such an element are gone through again (whole columns: 66.8 us instead of 62.0 for 64 requests x 32 heads with
+        // an fp32 residual, 244 instead of 232 for 256).
         if (fmaxf(fmaxf(eamax[0] - thr[0], eamax[1] - thr[1]), fmaxf(eamax[2] - thr[2], eamax[3] - thr[3])) > 0.f) {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) redecide_quad(hA[i], hB[i], cw[i], snew, thr);      // rare: a quotient within the tie guard
+          for (int i = 0; i < 16; ++i) redecide_quad(hA[i], hB[i], cw[i], snew, thr);
         }
         {
           const unsigned long long dst_codes = dst_of(D_CODES);
