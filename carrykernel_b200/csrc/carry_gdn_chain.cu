@@ -23,7 +23,6 @@ struct ChainExtra {
   int first_token;        // tokens already applied by earlier launches (offset into q, k, v, alpha, beta, o)
 };
 
-
 constexpr int kChainChunk = 8;           // tokens whose activations and facts are fetched together
 
 template <int RES, int QDT>

@@ -59,7 +59,6 @@ struct KParams {
   long long stride_idx;
   int num_slots;
   void* out;
-  float floor_amax, floor_scale;   // eps_mode as the two floors it means, one of them 0 (fill_shifts)
 };
 
 // head counts as shifts where they are powers of two (split_tile)
@@ -68,8 +67,6 @@ inline void fill_shifts(KParams& p) {
   p.hv_shift = log2_or_minus1(p.HV);
   p.group = p.HV / p.H;
   p.group_shift = log2_or_minus1(p.group);
-  p.floor_amax = p.eps_mode == CARRY_EPS_ON_AMAX ? kEps : 0.0f;
-  p.floor_scale = p.eps_mode == CARRY_EPS_ON_AMAX ? 0.0f : kEps;
 }
 
 // the values of qmax for which the streaming kernels' way to divide by it (div_qmax) is exact: 3 to 8 bits
@@ -87,22 +84,6 @@ __device__ __forceinline__ void store_from_float(void* p, long long i, int dtype
   if (dtype == CARRY_F32) reinterpret_cast<float*>(p)[i] = x;
   else if (dtype == CARRY_BF16) reinterpret_cast<__nv_bfloat16*>(p)[i] = __float2bfloat16_rn(x);
   else reinterpret_cast<__half*>(p)[i] = __float2half_rn(x);
-}
-
-// The same without a branch on the type, for lanes with `on` set: what is not theirs to write is converted as well.
-__device__ __forceinline__ void store_from_float_if(bool on, uint8_t* p, int i, int dtype, float x) {
-  const bool wide = dtype == CARRY_F32;
-  const unsigned short half = (dtype == CARRY_BF16) ? __bfloat16_as_ushort(__float2bfloat16_rn(x)) : __half_as_ushort(__float2half_rn(x));
-  asm volatile(
-      "{\n"
-      ".reg .pred w, n;\n"
-      "setp.ne.u32 w, %0, 0;\n"
-      "setp.ne.u32 n, %1, 0;\n"
-      "@w st.global.f32 [%2], %3;\n"
-      "@n st.global.u16 [%2], %4;\n"
-      "}\n" ::"r"((int)(on && wide)), "r"((int)(on && !wide)),
-      "l"(p + i * (wide ? 4 : 2)), "f"(x), "h"(half)
-      : "memory");
 }
 
 // scale from an absolute maximum, with the floor applied where the front end's

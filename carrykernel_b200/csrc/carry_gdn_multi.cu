@@ -26,8 +26,6 @@ int launch_multi(const KParams& p, int T, long long stride_mixed_t, long long st
 
 namespace {
 
-constexpr int kSlotThreads = 256;
-
 struct MultiExtra {
   int T;
   long long stride_mixed_t, stride_a_t, stride_b_t;   // elements from one token of a request to the next
@@ -35,18 +33,18 @@ struct MultiExtra {
 };
 
 template <int RES, int RSCALE, int QDT>
-__global__ void __launch_bounds__(kSlotThreads, 2) gdn_multi_kernel(const __grid_constant__ KParams p,
+__global__ void __launch_bounds__(kThreads, 2) gdn_multi_kernel(const __grid_constant__ KParams p,
                                                                const __grid_constant__ MultiExtra x) {
   using L = StageLayout<RES, LAYOUT_VK, QDT, RSCALE>;
   constexpr int qes = (QDT == CARRY_F32) ? 4 : 2;
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ __align__(8) uint64_t full_bar;
   __shared__ int poison_flag;
-  __shared__ uint32_t head_max[4];                    // largest new residual of a token, as bits, by token mod 4
+  __shared__ float head_red[2][kWarps];
   constexpr int kChunk = 8;                           // tokens whose activations and facts are fetched together
   __shared__ TileMeta meta_t[kChunk];
   __shared__ __align__(16) uint8_t vec_t[kChunk][3 * L::kVecBytes];   // raw q | k | v per token
-  __shared__ DotBuf dots_t[kChunk];
+  __shared__ __align__(16) float q_warp[kWarps * kT];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gw = warp, gtid = tid;
   uint8_t* sb = smem;
@@ -78,7 +76,7 @@ __global__ void __launch_bounds__(kSlotThreads, 2) gdn_multi_kernel(const __grid
   const long long out_tok0 = ((long long)n * x.T * p.HV + hv) * kT;      // out is [B, T, HV, V]
   const long long out_tok_stride = (long long)p.HV * kT;
   if (slot <= 0) {                                   // padding request: zeros for every token, pool untouched
-    for (int i = tid; i < x.T * kT; i += kSlotThreads)
+    for (int i = tid; i < x.T * kT; i += kThreads)
       store_from_float(p.out, out_tok0 + (long long)(i / kT) * out_tok_stride + (i % kT), p.o_dtype, 0.f);
     return;
   }
@@ -90,7 +88,6 @@ __global__ void __launch_bounds__(kSlotThreads, 2) gdn_multi_kernel(const __grid
 #pragma unroll
     for (int i = 0; i < 8; ++i) addr[i] = a8[i];
     poison_flag = 0;
-    head_max[0] = head_max[1] = head_max[2] = head_max[3] = 0u;
     mbar_init(&full_bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     // the state of the tile: codes, residual, state scales, residual scale(s)
@@ -105,7 +102,6 @@ __global__ void __launch_bounds__(kSlotThreads, 2) gdn_multi_kernel(const __grid
   const float rqmax_state = p.inv_qmax;
   bool healthy = true;
 
-  const SlotLane at = slot_lane(gw, lane);
   float es_head = 0.f;                               // one residual scale per head: carried from token to token
   for (int t = 0; t < x.T; ++t) {
     const int tc = t % kChunk;
@@ -115,7 +111,7 @@ __global__ void __launch_bounds__(kSlotThreads, 2) gdn_multi_kernel(const __grid
       // norms by one warp per token
       const int nt = (x.T - t < kChunk) ? (x.T - t) : kChunk;
       constexpr int kVecChunks = 3 * L::kVecBytes / 16;
-      for (int i = tid; i < nt * kVecChunks; i += kSlotThreads) {
+      for (int i = tid; i < nt * kVecChunks; i += kThreads) {
         const int tt = i / kVecChunks, c = i - tt * kVecChunks;
         const int which = c / (L::kVecBytes / 16), cc = c - which * (L::kVecBytes / 16);
         const uint8_t* src = reinterpret_cast<const uint8_t*>(addr[D_Q + which]) + (long long)(t + tt) * x.stride_mixed_t * qes;
@@ -125,8 +121,6 @@ __global__ void __launch_bounds__(kSlotThreads, 2) gdn_multi_kernel(const __grid
         tile_meta<RES, RSCALE, QDT, 32>(p, tile, lane, true, &meta_t[warp], nullptr,
                                      (long long)(t + warp) * x.stride_mixed_t, (long long)(t + warp) * x.stride_a_t,
                                      (long long)(t + warp) * x.stride_b_t);
-      __syncthreads();
-      if (warp < nt) prepare_dots<QDT>(&vec_t[warp][L::kVecBytes], &vec_t[warp][0], lane, &meta_t[warp], &dots_t[warp]);
       __syncthreads();
     }
     if (t == 0) {                                    // the tile has to be there; the verdict is the CTA's, not a warp's
@@ -140,49 +134,49 @@ __global__ void __launch_bounds__(kSlotThreads, 2) gdn_multi_kernel(const __grid
     const uint4 tm0 = lds_v4(&meta_t[tc]), tm1 = lds_v4(reinterpret_cast<const uint8_t*>(&meta_t[tc]) + 16);
     const float alpha = __uint_as_float(tm0.w), beta = __uint_as_float(tm1.x), k_mul = __uint_as_float(tm1.y),
                 q_mul = __uint_as_float(tm1.z), kq = __uint_as_float(tm1.w);
-    const uint4 tm2 = lds_v4(reinterpret_cast<const uint8_t*>(&meta_t[tc]) + 32);
-    const bool dot_fixed = __uint_as_float(tm2.x) != 0.0f;
-    const float dot_mul = __uint_as_float((lane & 2) ? tm2.w : tm2.z);
     const float* sscale = reinterpret_cast<const float*>(sb + L::kSScale);
     const float* rscale = reinterpret_cast<const float*>(sb + L::kRScale);
     const float2 alpha2 = splat(alpha);
     const float2 magic2 = splat(kMagicRound), nmagic2 = splat(-kMagicRound);
-    uint8_t* out_to = reinterpret_cast<uint8_t*>(p.out) + (out_tok0 + (long long)t * out_tok_stride) * (p.o_dtype == CARRY_F32 ? 4 : 2);
+    const long long out_tok = out_tok0 + (long long)t * out_tok_stride;
 
-#define CARRY_SLOT_DOTS dots_t[tc]
 #define CARRY_SLOT_VEC_Q (&vec_t[tc][0])
 #define CARRY_SLOT_VEC_K (&vec_t[tc][L::kVecBytes])
 #define CARRY_SLOT_VEC_V (&vec_t[tc][2 * L::kVecBytes])
-#define CARRY_SLOT_OUT(on, idx, value) store_from_float_if(on, out_to, (idx), p.o_dtype, (value))
-#define CARRY_SLOT_PUT_SSCALE(on, row_, bits_) if (on) *reinterpret_cast<uint32_t*>(sb + L::kSScale + (row_) * 4) = (bits_)
-#define CARRY_SLOT_CODES_TO (sb + L::kCodes)
-#define CARRY_SLOT_RESID_TO (sb + L::kResid)
-#define CARRY_SLOT_PUT16(base, offset, v) *reinterpret_cast<uint4*>((base) + (offset)) = (v)
-#define CARRY_SLOT_PUT8(base, offset, v) *reinterpret_cast<uint2*>((base) + (offset)) = (v)
-#define CARRY_SLOT_HEAD_MAX head_max[t & 3]
-#define CARRY_SLOT_MEET(statement)                                           \
-  if constexpr (RSCALE == CARRY_SCALE_PER_HEAD) {                            \
-    statement;                                                               \
-    if (tid == 0) head_max[(t + 2) & 3] = 0u;  /* last read two meetings ago */ \
-    __syncthreads();                                                          \
+#define CARRY_SLOT_OUT(idx, value) store_from_float(p.out, out_tok + (idx), p.o_dtype, (value))
+#define CARRY_SLOT_PUT_SSCALE(r0_, v4_) *reinterpret_cast<uint4*>(sb + L::kSScale + (r0_) * 4) = (v4_)
+#define CARRY_SLOT_PUT_CODES(r0_, c0_, cw_)                                                                        \
+  {                                                                                                                \
+    _Pragma("unroll") for (int i_ = 0; i_ < 4; ++i_)                                                               \
+        *reinterpret_cast<uint4*>(sb + L::kCodes + ((r0_) + i_) * kT + (c0_)) =                                    \
+        make_uint4(cw_[i_][0], cw_[i_][1], cw_[i_][2], cw_[i_][3]);                                                \
   }
-#define CARRY_SLOT_PUT_RSCALE_V(on, row_, bits_) if (on) *reinterpret_cast<uint32_t*>(sb + L::kRScale + (row_) * 4) = (bits_)
+#define CARRY_SLOT_HEAD_RED head_red[t & 1]
+#define CARRY_SLOT_MEET(statement)                \
+  if constexpr (RSCALE == CARRY_SCALE_PER_HEAD) { \
+    if (lane == 0) { statement; }                 \
+    warps_meet(3);                                \
+  }
+#define CARRY_SLOT_RESID_BEGIN()
+#define CARRY_SLOT_PUT_RESID4(i_, r0_, c0_, w_) \
+  *reinterpret_cast<uint2*>(sb + L::kResid + ((r0_) + (i_)) * (kT / 2) + (c0_) / 2) = (w_)
+#define CARRY_SLOT_PUT_RESID8(i_, r0_, c0_, w_) *reinterpret_cast<uint4*>(sb + L::kResid + ((r0_) + (i_)) * kT + (c0_)) = (w_)
+#define CARRY_SLOT_PUT_RSCALE_V(r0_, v4_) *reinterpret_cast<uint4*>(sb + L::kRScale + (r0_) * 4) = (v4_)
 #define CARRY_SLOT_PUT_RSCALE_HEAD(bits_) reinterpret_cast<uint32_t*>(sb + L::kRScale)[hv & 3] = (bits_)
 #include "carry_gdn_slot_tile.inc"
     if constexpr (RSCALE == CARRY_SCALE_PER_HEAD) es_head = esn[0];
     __syncwarp();                                    // a warp's rows are its own: written by one lane, read by another
-#undef CARRY_SLOT_DOTS
 #undef CARRY_SLOT_VEC_Q
 #undef CARRY_SLOT_VEC_K
 #undef CARRY_SLOT_VEC_V
 #undef CARRY_SLOT_OUT
 #undef CARRY_SLOT_PUT_SSCALE
-#undef CARRY_SLOT_CODES_TO
-#undef CARRY_SLOT_RESID_TO
-#undef CARRY_SLOT_PUT16
-#undef CARRY_SLOT_PUT8
-#undef CARRY_SLOT_HEAD_MAX
+#undef CARRY_SLOT_PUT_CODES
+#undef CARRY_SLOT_HEAD_RED
 #undef CARRY_SLOT_MEET
+#undef CARRY_SLOT_RESID_BEGIN
+#undef CARRY_SLOT_PUT_RESID4
+#undef CARRY_SLOT_PUT_RESID8
 #undef CARRY_SLOT_PUT_RSCALE_V
 #undef CARRY_SLOT_PUT_RSCALE_HEAD
   }
@@ -194,9 +188,9 @@ __global__ void __launch_bounds__(kSlotThreads, 2) gdn_multi_kernel(const __grid
     return;
   }
   // the tile goes back to the pool: 16 bytes per thread and step, whole lines
-  for (int i = tid; i < kT * kT / 16; i += kSlotThreads)
+  for (int i = tid; i < kT * kT / 16; i += kThreads)
     stg_v4(addr[D_CODES] + 16ull * i, *reinterpret_cast<const uint4*>(sb + L::kCodes + 16 * i));
-  for (int i = tid; i < L::kResidBytes / 16; i += kSlotThreads)
+  for (int i = tid; i < L::kResidBytes / 16; i += kThreads)
     stg_v4(addr[D_RESID] + 16ull * i, *reinterpret_cast<const uint4*>(sb + L::kResid + 16 * i));
   if (tid < 32) stg_v4(addr[D_SSCALE] + 16ull * tid, *reinterpret_cast<const uint4*>(sb + L::kSScale + 16 * tid));
   if (RSCALE == CARRY_SCALE_PER_V) {
@@ -222,7 +216,7 @@ int launch_multi_variant(const KParams& p, const MultiExtra& x, cudaStream_t str
     }
     configured[dev] = true;
   }
-  return launch_dependent(kern, dim3((unsigned)((long long)p.B * p.HV)), kSlotThreads, smem, stream, p, x);
+  return launch_dependent(kern, dim3((unsigned)((long long)p.B * p.HV)), kThreads, smem, stream, p, x);
 }
 
 template <int RES, int RSCALE>

@@ -1,7 +1,8 @@
-// Streaming kernels for the serving shape, K = V = 128: the helpers that they share, and the one of the statequant layout
-// [K][V] with a floating-point residual (the layout's other formats: carry_gdn_dense128.cu; the slot layout [V][K]:
-// carry_gdn_tile128_vk.cu).  One (request, head) tile is 16 KB of codes + its residual; all of it is contiguous in
-// memory in both layouts, so every tile moves with a handful of 1-D bulk async copies (TMA, no tensor map):
+// Streaming kernel for the serving shape: K = V = 128, int8 state, int8 or packed
+// int4 residual in the slot layout, a floating-point residual in the statequant
+// layout (carry_gdn_dense128.cu has that layout's other formats).  One (request, head) tile is 16 KB of codes + 8/16 KB of
+// residual; all of it is contiguous in memory in both layouts, so every tile
+// moves with a handful of 1-D bulk async copies (TMA, no tensor map):
 //
 //   global --cp.async.bulk--> shared stage --> registers --16-byte stores--> global
 //
@@ -15,8 +16,16 @@
 // results leave straight from registers as 16-byte vector stores that cover whole
 // 128-byte lines.  The state is read from HBM once and written once.
 //
-// Work split inside a group (256 threads = 8 warps): warp w owns rows 16w..16w+15 of the tile, lane = 4 contiguous columns
-// x those rows; column sums are finished across the 8 warps through shared memory (three meetings per tile).
+// Work split inside a group (256 threads = 8 warps): warp w owns memory rows
+// 16w..16w+15 of the tile.
+//   * slot layout [V][K] (scale per row): lane = (row group rg, column group
+//     cg): 4 rows x 16 contiguous columns.  Everything the math reduces over
+//     (K) lies along the row, so reductions are shuffles inside 8 lanes; the
+//     warps meet once per tile (for the per-head residual scale, and to agree on
+//     the next tile).
+//   * statequant layout [K][V] (scale per column): lane = 4 contiguous columns
+//     x the warp's 16 rows; column sums are finished across the 8 warps through
+//     shared memory (three meetings per tile).
 //
 // Arithmetic.  Everything that feeds a state code keeps the reference's operation
 // order, with the contractions written out as explicit fused multiply-adds:
@@ -29,8 +38,6 @@
 // rint(e * (1/es)) as is.  Math runs as packed f32x2 (IEEE round-to-nearest per
 // component).
 #pragma once
-#include <stddef.h>
-
 #include "carry_gdn_common.cuh"
 
 namespace carry {
@@ -39,7 +46,6 @@ namespace {
 constexpr int kT = 128;                 // tile edge
 constexpr int kThreads = 256;          // threads of one group: the 8 warps that share a tile
 constexpr int kWarps = 8;
-enum { LAYOUT_VK = 0, LAYOUT_KV = 1 };  // slot layout [V][K]; statequant layout [K][V]
 // Polls of a stage barrier before a wait gives up.  CARRY_TEST_WAIT_EXPIRY builds a test-only library in
 // which the copies of global tile 1 announce 16 bytes more than they bring, so that its barrier never
 // completes, and the limit is short: the expiry path (status bit, poisoned CTA, pool left untouched) then
@@ -64,6 +70,8 @@ __device__ __forceinline__ bool test_inputs_changed(int) { return false; }
 __device__ __forceinline__ void test_note_changed(int*, bool) {}
 #endif
 constexpr int kTileCache = 64;         // per group: cached slot ids and gates of the CTA's first tiles
+
+enum { LAYOUT_VK = 0, LAYOUT_KV = 1 };  // slot layout [V][K]; statequant layout [K][V]
 
 // ---------------------------------------------------------------------------
 // PTX wrappers
@@ -184,12 +192,6 @@ __device__ __forceinline__ uint32_t order_token() {
   asm volatile("mov.u32 %0, 0;" : "=r"(t) : : "memory");
   return t;
 }
-__device__ __forceinline__ void stg_b32_if(bool on, unsigned long long addr, uint32_t v) {
-  asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %0, 0;\n@p st.global.b32 [%1], %2;\n}\n" ::"r"((int)on), "l"(addr), "r"(v) : "memory");
-}
-__device__ __forceinline__ void shared_max_if(bool on, uint32_t* word, uint32_t v) {
-  asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %0, 0;\n@p red.shared.max.u32 [%1], %2;\n}\n" ::"r"((int)on), "r"(smem_u32(word)), "r"(v) : "memory");
-}
 __device__ __forceinline__ void stg_b32(unsigned long long addr, uint32_t v) {
   asm volatile("st.global.b32 [%0], %1;" ::"l"(addr), "r"(v) : "memory");
 }
@@ -239,9 +241,6 @@ template <int A, int B>
 __device__ __forceinline__ float2 s8x2_cvt(uint32_t w) {
   return make_float2((float)(signed char)((w >> (8 * A)) & 0xffu), (float)(signed char)((w >> (8 * B)) & 0xffu));
 }
-// the codes of a quad's even and odd columns
-__device__ __forceinline__ float2 slot_codes_even(uint32_t w) { return s8x2_cvt<0, 2>(w); }
-__device__ __forceinline__ float2 slot_codes_odd(uint32_t w) { return s8x2_to_float<1, 3>(w ^ 0x80808080u); }
 // bytes A and B of w, each a nibble in offset binary (0..15 = code + 8) -> {136 + code A, 136 + code B}:
 // the byte is placed right above the low half-word of a float whose exponent byte says 128
 template <int A, int B>
@@ -300,10 +299,19 @@ __device__ __forceinline__ float warp_max_nonneg(float x) {
   return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(x)));
 }
 
-// max over the 4 lanes of a row, in each of them
-__device__ __forceinline__ float row_max(float x) {
-  x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 1));
-  return fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 2));
+// Four values per lane, each to be maximised over the 8 lanes of a row group.  Halving exchange: lane g
+// of the group ends up with the maximum of x[(g >> 1) & 3], at 4 shuffles instead of 12.
+__device__ __forceinline__ float group_max4_transposed(const float (&x)[4], int g) {
+  const bool up4 = g & 4, up2 = g & 2;
+  float a[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const float keep = up4 ? x[2 + i] : x[i], send = up4 ? x[i] : x[2 + i];
+    a[i] = fmaxf(keep, __shfl_xor_sync(0xffffffffu, send, 4));
+  }
+  const float keep = up2 ? a[1] : a[0], send = up2 ? a[0] : a[1];
+  const float b = fmaxf(keep, __shfl_xor_sync(0xffffffffu, send, 2));
+  return fmaxf(b, __shfl_xor_sync(0xffffffffu, b, 1));
 }
 
 // 1/s to within 2^-24 (1 + 2^-20) relative: the hardware approximation (1 ulp) and one Newton step.  The
@@ -316,6 +324,27 @@ __device__ __forceinline__ float rcp_refined(float s) {
   return fmaf(y, fmaf(-s, y, 1.0f), y);
 }
 
+// Eight values per lane (x[0..3], y[0..3]), each to be summed over the 8 lanes of a row group.
+// Halving exchange: after three rounds lane g of the group holds one total -- x[g] for g < 4,
+// y[g - 4] otherwise -- at 7 shuffles instead of 24.
+__device__ __forceinline__ float group_sum8_transposed(const float (&x)[4], const float (&y)[4], int g) {
+  const bool up4 = g & 4, up2 = g & 2, up1 = g & 1;
+  float a[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float keep = up4 ? y[i] : x[i], send = up4 ? x[i] : y[i];
+    a[i] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+  }
+  float b[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const float keep = up2 ? a[2 + i] : a[i], send = up2 ? a[i] : a[2 + i];
+    b[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
+  }
+  const float keep = up1 ? b[1] : b[0], send = up1 ? b[0] : b[1];
+  return keep + __shfl_xor_sync(0xffffffffu, send, 1);
+}
+
 // amax / qmax, correctly rounded, without the division routine.  `rq` is 1/qmax rounded to nearest;
 // a * rq is within an ulp of the quotient, the remainder a - qmax * q0 is exact in one fused
 // multiply-add and corrects it.  Equal to IEEE division for every float a >= 2^-100 when qmax is one of
@@ -324,10 +353,6 @@ __device__ __forceinline__ float rcp_refined(float s) {
 __device__ __forceinline__ float div_qmax(float a, float qmax, float rq) {
   const float q0 = __fmul_rn(a, rq);
   return fmaf(fmaf(-qmax, q0, a), rq, q0);
-}
-// ... with the floors of KParams: max(amax, 1e-12) / qmax or max(amax / qmax, 1e-12)
-__device__ __forceinline__ float scale_floors(const KParams& p, float amax, float qmax, float rq) {
-  return fmaxf(div_qmax(fmaxf(amax, p.floor_amax), qmax, rq), p.floor_scale);
 }
 __device__ __forceinline__ float scale_fast(float amax, float qmax, float rq, int eps_mode) {
   if (eps_mode == CARRY_EPS_ON_AMAX) return div_qmax(fmaxf(amax, kEps), qmax, rq);
@@ -341,7 +366,9 @@ __device__ __forceinline__ float scale_fast(float amax, float qmax, float rq, in
 // Static shared memory next to the stage ring: barriers, the per-CTA tile caches,
 // the per-warp q scratch (slot layout) or the column-reduction space (statequant
 // layout).  Upper bounds, used to size the ring.
-constexpr int kStaticKV = 23808;        // per group
+constexpr int kStaticVK = 11776;        // per group
+constexpr int kStaticKV = 22528;
+constexpr int kStaticOf(int layout) { return layout == 0 ? kStaticVK : kStaticKV; }
 constexpr int kSmemPerCta = 231424;     // one CTA per SM: 227 KB less 1 KB
 
 template <int RES, int LAYOUT, int QDT, int RSCALE>
@@ -365,8 +392,8 @@ struct StageLayout {
   // Two groups of 8 warps share one CTA (and one SM) when at least 2 stages per group fit (every
   // variant today; 128 registers per thread then), else the CTA is a single group.
   static constexpr int kGroups =
-      ((4 * kBytes + 2 * kStaticKV <= kSmemPerCta) ? 2 : 1);
-  static constexpr int kStatic = kGroups * kStaticKV;
+      ((4 * kBytes + 2 * kStaticOf(LAYOUT) <= kSmemPerCta) ? 2 : 1);
+  static constexpr int kStatic = kGroups * kStaticOf(LAYOUT);
   static constexpr int kBudget = kSmemPerCta - kStatic;
   static constexpr int kFit = kBudget / kBytes;
   // a deeper ring does not help (a tile takes several times longer to compute than to load) and makes the
@@ -438,18 +465,6 @@ __device__ __forceinline__ void redecide_rec(float& e, float& y, float s, float 
   }
 }
 
-// ... of the elements of a quad that share a scale.  A call: it is rarely needed, and written out at every quad it is a third of
-// a kernel's code.
-struct QuadCodes { float2 E, O; uint32_t cw; };
-__device__ __noinline__ QuadCodes redecide_shared(QuadCodes x, float s, float thr) {
-  float2 yE = add2(s8x2_to_float<0, 2>(x.cw ^ 0x80808080u), splat(kMagicRound));
-  float2 yO = add2(s8x2_to_float<1, 3>(x.cw ^ 0x80808080u), splat(kMagicRound));
-  redecide_rec(x.E.x, yE.x, s, thr); redecide_rec(x.E.y, yE.y, s, thr);
-  redecide_rec(x.O.x, yO.x, s, thr); redecide_rec(x.O.y, yO.y, s, thr);
-  x.cw = pack4(__float_as_uint(yE.x), __float_as_uint(yO.x), __float_as_uint(yE.y), __float_as_uint(yO.y));
-  return x;
-}
-
 // ... of four neighbouring columns of one row, each with its own scale: nothing is done unless one of them is within the
 // guard.
 __device__ __forceinline__ void redecide_quad(float2& a, float2& b, uint32_t& cw, const float (&s)[4], const float (&thr)[4]) {
@@ -515,10 +530,8 @@ struct __align__(16) TileMeta {
   float alpha, beta;
   float k_mul, q_mul;   // 1/|k| and scale/|q| (1 when the L2 norm is off; statequant path: 1)
   float kq;             // <k, q> after those factors
-  float k_fix, q_fix;   // slot layout: the powers of two that take k and q to 31-bit integers (both 0: see slot_dots_plain)
-  float k_dot, q_dot;   // ... and what takes a dot product with those integers back: k_mul / k_fix, q_mul / q_fix
 };
-static_assert(sizeof(TileMeta) == 48, "TileMeta is read as 16-byte words");
+static_assert(sizeof(TileMeta) == 32, "TileMeta is read as two 16-byte words");
 
 // Where a tile's data lives: the four places its results go (codes, residual, state scales, residual
 // scale(s)), then the sources that are not one of those (residual scales as read, q, k, v).  Codes,
@@ -655,16 +668,7 @@ __device__ __forceinline__ bool meta_unchanged(const KParams& p, int n, int hv, 
   d |= (uint32_t)(slot ^ x.slot) | (g.a ^ x.g.a) | (g.b ^ x.g.b) | (g.A_log ^ x.g.A_log) | (g.dt_bias ^ x.g.dt_bias);
   return d == 0u;
 }
-// Fixed point for the slot layout's dot products: a vector whose largest magnitude is below 2^e becomes the integers
-// rint(x * 2^(30-e)).  `bits` is that largest magnitude's pattern.  Exact for 16-bit types down to 2^-20 (fp16) and 2^-23
-// (bf16) of the largest element; what is lost below is at most 2^-32 of it.
-__device__ __forceinline__ bool fix_fits(uint32_t bits) { return bits == 0u || (bits >= (30u << 23) && bits < 0x7f800000u); }
-__device__ __forceinline__ float fix_scale(uint32_t bits) {
-  const uint32_t e = max(bits >> 23, 30u);            // biased exponent
-  return __uint_as_float((283u - e) << 23);           // 2^(30 - (e - 126))
-}
-__device__ __forceinline__ float fix_inverse(float scale) { return __uint_as_float(0x7f000000u - __float_as_uint(scale)); }
-// fills m.alpha, beta, k_mul, q_mul, kq and the fixed-point factors (all 32 lanes of a warp together: the sums go over lanes)
+// fills m.alpha, beta, k_mul, q_mul, kq (all 32 lanes of a warp together: the sums go over lanes)
 template <int QDT, int LPT>
 __device__ __forceinline__ void meta_math(const KParams& p, const MetaRaw<QDT, LPT>& r, TileMeta& m) {
   constexpr int kGroups4 = MetaRaw<QDT, LPT>::kElems / 4;   // groups of four elements per lane
@@ -700,38 +704,12 @@ __device__ __forceinline__ void meta_math(const KParams& p, const MetaRaw<QDT, L
     kqsum += __shfl_xor_sync(0xffffffffu, kqsum, o);
   }
   m.k_mul = 1.0f; m.q_mul = 1.0f;
-  m.k_fix = m.q_fix = m.k_dot = m.q_dot = 0.0f;
   if (p.packed) {
     if (p.l2norm) {
       m.k_mul = __frcp_rn(sqrtf(ksum + 1e-6f));
       m.q_mul = __frcp_rn(sqrtf(qsum + 1e-6f));
     }
     m.q_mul *= p.qscale;
-    // largest magnitudes, as bit patterns (infinities and NaNs are above all finite ones)
-    uint32_t kb = 0u, qb = 0u;
-#pragma unroll
-    for (int i = 0; i < MetaRaw<QDT, LPT>::kWords; ++i) {
-      if (QDT == CARRY_F32) {
-        kb = max(kb, r.kw[i] & 0x7fffffffu);
-        qb = max(qb, r.qw[i] & 0x7fffffffu);
-      } else {
-        kb = __vmaxu2(kb, r.kw[i] & 0x7fff7fffu);
-        qb = __vmaxu2(qb, r.qw[i] & 0x7fff7fffu);
-      }
-    }
-    if (QDT != CARRY_F32) {
-      kb = __float_as_uint(act_pair<QDT>(max(kb >> 16, kb & 0xffffu)).x);
-      qb = __float_as_uint(act_pair<QDT>(max(qb >> 16, qb & 0xffffu)).x);
-    }
-#pragma unroll
-    for (int o = 1; o < LPT; o <<= 1) {
-      kb = max(kb, __shfl_xor_sync(0xffffffffu, kb, o));
-      qb = max(qb, __shfl_xor_sync(0xffffffffu, qb, o));
-    }
-    if (fix_fits(kb) && fix_fits(qb)) {
-      m.k_fix = fix_scale(kb); m.q_fix = fix_scale(qb);
-      m.k_dot = m.k_mul * fix_inverse(m.k_fix); m.q_dot = m.q_mul * fix_inverse(m.q_fix);
-    }
   }
   m.kq = kqsum * (m.k_mul * m.q_mul);
 }
@@ -774,136 +752,6 @@ __device__ __noinline__ void tile_meta(const KParams& p, int tile, int sub, bool
   unsigned long long a[8];
   const bool bad = meta_addresses<RES, RSCALE, QDT>(p, m, hv, h, a);
   if (store) meta_put(p, m, a, bad, sub, dst, ddst);
-}
-
-// ---------------------------------------------------------------------------
-// slot layout: the two dot products of a row on the integer tensor cores
-// ---------------------------------------------------------------------------
-// <codes row, k> and <codes row, q> are sums of int8 codes times numbers that every row shares.  k and q are turned into
-// 31-bit integers once per tile (prepare_quad) and cut into four signed base-256 digits each; the digits of k and q are the
-// eight columns of B in mma.m16n8k32 (s8), the codes as they lie in the stage are A.  Four instructions give a warp all its
-// 16 rows' sums, exact, with the codes not decoded yet; one rounding per total follows.  Against packed fp32 multiply-adds
-// over decoded codes (64 instructions of up to 6 register operands each, plus the exchange of partial sums over 8 lanes)
-// this is what makes room in a kernel that is bound by its register operands; against mma in bf16 (A packed from decoded
-// codes, 10.8 cycles per 16 x 16 codes against 9.1 per 16 x 32) it needs no packing and does not round inside the sum.
-struct __align__(16) DotBuf {
-  uint32_t digits[8][36];   // [k digit 0..3, q digit 0..3][8 * t + quad m of lane t]; 36: lanes of rows g, g + 1 in other banks
-  float4 k[32];             // [4 * m + t]: k * k_mul of the quad's columns as {0, 2, 1, 3}
-};
-// quad `Q` (columns 4Q..4Q+3) is quad m = 4 * (Q / 16) + Q % 4 of lane t = Q / 4 % 4: lane t of a row holds columns
-// 16t..16t+15 (m < 4) and 64+16t..64+16t+15
-// A lane's place in a tile: the offset of its codes (first row * 128 + first column) and of its B fragments
-struct SlotLane {
-  int codes, digits;
-  __device__ __forceinline__ int row() const { return codes >> 7; }
-  __device__ __forceinline__ int k() const { return (int)offsetof(DotBuf, k) + (codes & 127); }   // first k in DotBuf
-};
-__device__ __forceinline__ SlotLane slot_lane(int gw, int lane) {
-  const int rg = lane >> 2, cl = lane & 3;
-  SlotLane at = {(16 * gw + rg) * kT + 16 * cl, rg * 144 + 32 * cl};
-  // kept in registers: worked out again from the thread index wherever they are used they cost 40 instructions per tile
-  asm volatile("" : "+r"(at.codes), "+r"(at.digits));
-  return at;
-}
-// quad m of k from shared memory, read again for each of a lane's rows on purpose: k must not stay in registers
-__device__ __forceinline__ float4 slot_k_quad(uint32_t addr, int row, int m) {
-#define CARRY_K_ROW(R)                                                                                           \
-  ((m == 0) ? lds_f4_at<0, R>(addr) : (m == 1) ? lds_f4_at<64, R>(addr) : (m == 2) ? lds_f4_at<128, R>(addr)      \
-   : (m == 3) ? lds_f4_at<192, R>(addr) : (m == 4) ? lds_f4_at<256, R>(addr) : (m == 5) ? lds_f4_at<320, R>(addr) \
-   : (m == 6) ? lds_f4_at<384, R>(addr) : lds_f4_at<448, R>(addr))
-  return row == 0 ? CARRY_K_ROW(0) : CARRY_K_ROW(1);
-#undef CARRY_K_ROW
-}
-template <int QDT>
-struct RawQuad { uint32_t k[QDT == CARRY_F32 ? 4 : 2], q[QDT == CARRY_F32 ? 4 : 2]; };
-template <int QDT>
-__device__ __forceinline__ void raw_floats(const uint32_t* w, float (&x)[4]) {
-  if (QDT == CARRY_F32) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) x[i] = __uint_as_float(w[i]);
-  } else {
-    const float2 a = act_pair<QDT>(w[0]), b = act_pair<QDT>(w[1]);
-    x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
-  }
-}
-// four integers -> their four digits, each a word with one byte per integer
-__device__ __forceinline__ void put_digits(const float (&x)[4], float fix, uint32_t* to) {
-  uint32_t d[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) d[i] = ((uint32_t)__float2int_rn(x[i] * fix) + 0x00808080u) ^ 0x00808080u;
-  const uint32_t a = __byte_perm(d[0], d[1], 0x5140), b = __byte_perm(d[2], d[3], 0x5140);   // {0.0, 1.0, 0.1, 1.1}
-  const uint32_t c = __byte_perm(d[0], d[1], 0x7362), e = __byte_perm(d[2], d[3], 0x7362);
-  to[0 * 36] = __byte_perm(a, b, 0x5410);
-  to[1 * 36] = __byte_perm(a, b, 0x7632);
-  to[2 * 36] = __byte_perm(c, e, 0x5410);
-  to[3 * 36] = __byte_perm(c, e, 0x7632);
-}
-template <int QDT>
-__device__ __forceinline__ void prepare_quad(const RawQuad<QDT>& r, int Q, const TileMeta& m, DotBuf& buf) {
-  float k[4], q[4];
-  raw_floats<QDT>(r.k, k);
-  raw_floats<QDT>(r.q, q);
-  const int t = (Q >> 2) & 3, mm = 4 * (Q >> 4) + (Q & 3);
-  buf.k[4 * mm + t] = make_float4(k[0] * m.k_mul, k[2] * m.k_mul, k[1] * m.k_mul, k[3] * m.k_mul);
-  if (m.k_fix != 0.0f) {
-    put_digits(k, m.k_fix, &buf.digits[0][8 * t + mm]);
-    put_digits(q, m.q_fix, &buf.digits[4][8 * t + mm]);
-  }
-}
-// ... from vectors in shared or global memory (16-byte aligned), lane = quad
-template <int QDT>
-__device__ __forceinline__ RawQuad<QDT> raw_quad(const uint8_t* k, const uint8_t* q, int Q) {
-  RawQuad<QDT> r;
-  if constexpr (QDT == CARRY_F32) {
-    const uint4 a = reinterpret_cast<const uint4*>(k)[Q], b = reinterpret_cast<const uint4*>(q)[Q];
-    r.k[0] = a.x; r.k[1] = a.y; r.k[2] = a.z; r.k[3] = a.w; r.q[0] = b.x; r.q[1] = b.y; r.q[2] = b.z; r.q[3] = b.w;
-  } else {
-    const uint2 a = reinterpret_cast<const uint2*>(k)[Q], b = reinterpret_cast<const uint2*>(q)[Q];
-    r.k[0] = a.x; r.k[1] = a.y; r.q[0] = b.x; r.q[1] = b.y;
-  }
-  return r;
-}
-// ... of one vector, k or q, by one warp, lane = quad
-template <int QDT, bool IS_K>
-__device__ __forceinline__ void prepare_vector(const uint8_t* vec, int Q, const TileMeta& m, DotBuf& buf) {
-  const float4 x4 = act4<QDT>(vec, 4 * Q);
-  const float x[4] = {x4.x, x4.y, x4.z, x4.w};
-  const int t = (Q >> 2) & 3, mm = 4 * (Q >> 4) + (Q & 3);
-  if (IS_K) buf.k[4 * mm + t] = make_float4(x[0] * m.k_mul, x[2] * m.k_mul, x[1] * m.k_mul, x[3] * m.k_mul);
-  put_digits(x, IS_K ? m.k_fix : m.q_fix, &buf.digits[IS_K ? 0 : 4][8 * t + mm]);
-}
-template <int QDT>
-__device__ __noinline__ void prepare_dots(const uint8_t* k, const uint8_t* q, int lane, const TileMeta* m, DotBuf* buf) {
-  const TileMeta mm = *m;
-  prepare_quad<QDT>(raw_quad<QDT>(k, q, lane), lane, mm, *buf);
-}
-// c += a * b; a = {row g: columns 4t.., row g+8, row g: columns 16+4t.., row g+8}, b = {column g of B: rows 4t.., 16+4t..}
-__device__ __forceinline__ void mma_s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-      : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void mma_s8_first(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
-      : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
-}
-// The same totals by plain multiply-adds, for k or q that are not finite or below 2^-97: lane t of a row pair's four ends up with
-// <row, k> (t = 0), <row + 8, k> (1), <row, q> (2), <row + 8, q> (3), factors included.
-template <int QDT>
-__device__ __noinline__ float slot_dots_plain(const uint8_t* codes_row, const uint8_t* k, const uint8_t* q, float k_mul, float q_mul, int t) {
-  float s[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 1
-  for (int i = 0; i < 32; ++i) {
-    const int c = 16 * t + (i & 15) + 64 * (i >> 4);
-    const float a = (float)(signed char)codes_row[c], b = (float)(signed char)codes_row[8 * kT + c];
-    const float kc = act<QDT>(k, c) * k_mul, qc = act<QDT>(q, c) * q_mul;
-    s[0] = fmaf(a, kc, s[0]); s[1] = fmaf(b, kc, s[1]); s[2] = fmaf(a, qc, s[2]); s[3] = fmaf(b, qc, s[3]);
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    s[i] += __shfl_xor_sync(0xffffffffu, s[i], 1);
-    s[i] += __shfl_xor_sync(0xffffffffu, s[i], 2);
-  }
-  return (t == 0) ? s[0] : (t == 1) ? s[1] : (t == 2) ? s[2] : s[3];
 }
 
 // Request one tile into the stage at `sb` (called by one thread): the stage barrier's single arrival
@@ -966,12 +814,14 @@ gdn_tile128_kernel(const __grid_constant__ KParams p) {
   __shared__ int first_cnt[G][2];                    // arrivals at the last meeting of a tile, by the same parity
   __shared__ int poison_flag;
   __shared__ int stage_tile[S];                      // number of the tile last requested into each stage
+  __shared__ float head_red[G][2][kWarps];
   __shared__ TileMeta meta_cache[kCache + G * kWarps];   // this CTA's first tiles; one spare entry per warp
   __shared__ TileDesc desc_cache[kCache + G * kWarps];   // their addresses
+  __shared__ __align__(16) float q_warp[(LAYOUT == LAYOUT_VK) ? G * kWarps * kT : 4];   // per warp: q, scaled, as pairs
   __shared__ __align__(16) float col_red_all[(LAYOUT == LAYOUT_KV) ? G * kWarps * kT * 3 : 4];
   __shared__ __align__(16) float4 kq_rows[(LAYOUT == LAYOUT_KV) ? G * kWarps * 16 : 1];   // per warp: {k, k, q, q} of its rows
-  static_assert(sizeof(full_bar) + sizeof(claimed) + sizeof(first_cnt) + sizeof(stage_tile) + sizeof(meta_cache) + sizeof(desc_cache) +
-                        sizeof(col_red_all) + sizeof(kq_rows) + 64 <= L::kStatic,
+  static_assert(sizeof(full_bar) + sizeof(claimed) + sizeof(first_cnt) + sizeof(stage_tile) + sizeof(head_red) + sizeof(meta_cache) + sizeof(desc_cache) +
+                        sizeof(q_warp) + sizeof(col_red_all) + sizeof(kq_rows) + 64 <= L::kStatic,
                 "static shared memory exceeds what the stage ring was sized for");
   static_assert(S >= 2 * G, "every group needs a stage in use and one on the way");
 
@@ -1162,7 +1012,60 @@ gdn_tile128_kernel(const __grid_constant__ KParams p) {
       const float2 alpha2 = splat(alpha);
       const float2 magic2 = splat(kMagicRound), nmagic2 = splat(-kMagicRound);
 
-      {
+      if constexpr (LAYOUT == LAYOUT_VK) {
+#define CARRY_SLOT_VEC_Q (sb + L::kQ)
+#define CARRY_SLOT_VEC_K (sb + L::kK)
+#define CARRY_SLOT_VEC_V (sb + L::kV)
+#define CARRY_SLOT_OUT(idx, value) store_from_float(p.out, (long long)out_row * kT + (idx), p.o_dtype, (value))
+#define CARRY_SLOT_PUT_SSCALE(r0_, v4_) stg_v4(dst_of(D_SSCALE) + (r0_) * 4, (v4_))
+#define CARRY_SLOT_PUT_CODES(r0_, c0_, cw_)                                                   \
+  {                                                                                           \
+    const unsigned long long base = dst_of(D_CODES) + (r0_) * kT + (c0_);                     \
+    stg_v4_at<0 * kT>(base, make_uint4(cw_[0][0], cw_[0][1], cw_[0][2], cw_[0][3]));          \
+    stg_v4_at<1 * kT>(base, make_uint4(cw_[1][0], cw_[1][1], cw_[1][2], cw_[1][3]));          \
+    stg_v4_at<2 * kT>(base, make_uint4(cw_[2][0], cw_[2][1], cw_[2][2], cw_[2][3]));          \
+    stg_v4_at<3 * kT>(base, make_uint4(cw_[3][0], cw_[3][1], cw_[3][2], cw_[3][3]));          \
+  }
+#define CARRY_SLOT_HEAD_RED head_red[grp][cnt & 1]
+#define CARRY_SLOT_MEET(statement)                \
+  if (lane == 0) { statement; claim_next(cnt); }  \
+  warps_meet(bar0 + 3);                           \
+  refill_stage(it)
+#define CARRY_SLOT_RESID_BEGIN() const unsigned long long dst_resid = dst_of(D_RESID)
+#define CARRY_SLOT_PUT_RESID4(i_, r0_, c0_, w_)                                    \
+  {                                                                                \
+    const unsigned long long base = dst_resid + (r0_) * (kT / 2) + (c0_) / 2;      \
+    if (i_ == 0) stg_v2_at<0 * (kT / 2)>(base, w_);                                \
+    if (i_ == 1) stg_v2_at<1 * (kT / 2)>(base, w_);                                \
+    if (i_ == 2) stg_v2_at<2 * (kT / 2)>(base, w_);                                \
+    if (i_ == 3) stg_v2_at<3 * (kT / 2)>(base, w_);                                \
+  }
+#define CARRY_SLOT_PUT_RESID8(i_, r0_, c0_, w_)                                    \
+  {                                                                                \
+    const unsigned long long base = dst_resid + (r0_) * kT + (c0_);                \
+    const uint4 pw = w_;                                                           \
+    if (i_ == 0) stg_v4_at<0 * kT>(base, pw);                                      \
+    if (i_ == 1) stg_v4_at<1 * kT>(base, pw);                                      \
+    if (i_ == 2) stg_v4_at<2 * kT>(base, pw);                                      \
+    if (i_ == 3) stg_v4_at<3 * kT>(base, pw);                                      \
+  }
+#define CARRY_SLOT_PUT_RSCALE_V(r0_, v4_) stg_v4(dst_of(D_RSCALE) + (r0_) * 4, (v4_))
+#define CARRY_SLOT_PUT_RSCALE_HEAD(bits_) stg_b32(dst_of(D_RSCALE), (bits_))
+#include "carry_gdn_slot_tile.inc"
+#undef CARRY_SLOT_VEC_Q
+#undef CARRY_SLOT_VEC_K
+#undef CARRY_SLOT_VEC_V
+#undef CARRY_SLOT_OUT
+#undef CARRY_SLOT_PUT_SSCALE
+#undef CARRY_SLOT_PUT_CODES
+#undef CARRY_SLOT_HEAD_RED
+#undef CARRY_SLOT_MEET
+#undef CARRY_SLOT_RESID_BEGIN
+#undef CARRY_SLOT_PUT_RESID4
+#undef CARRY_SLOT_PUT_RESID8
+#undef CARRY_SLOT_PUT_RSCALE_V
+#undef CARRY_SLOT_PUT_RSCALE_HEAD
+      } else {
         // ---------------- statequant layout [K][V]: lane = 4 columns x 16 rows ----
         // columns {c0, c0+1} are held as pair A, {c0+2, c0+3} as pair B
         const int r0 = 16 * gw, c0 = 4 * lane;
