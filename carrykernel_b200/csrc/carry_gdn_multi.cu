@@ -5,9 +5,15 @@
 // included, exactly as T single-token launches would do it -- and goes back to
 // the pool once.  State traffic per token is 1/T of the single-token kernel's.
 //
-// One CTA (8 warps) per tile, two CTAs per SM.  The per-token arithmetic is the
-// slot-layout tile body of the streaming kernel (carry_gdn_slot_tile.inc),
-// with its stores pointed at the staged tile instead of global memory; a warp
+// One CTA (8 warps) per tile, two CTAs per SM.  The per-token arithmetic is that of the streaming kernel
+// (carry_gdn_slot_tile.inc), operation for operation and sum for sum, over another split: a lane holds 32 columns (two runs of 16)
+// of 2 rows, 8 apart, where it holds 16 columns of 4 rows there.  Sums and maxima then go over 4 lanes instead of 8 and every
+// lane has two rows' scalars to work out instead of four.  k and q of a token, scaled, are laid out once for all warps instead
+// of once per warp, and the output's store has no branches.  Bound: the FMA and ALU pipes, whose busy cycles do not overlap; what is
+// taken off either is the gain.  8 layers of 32 requests, 4 tokens: 495 us, 513 before; a launch of 64 requests, 6 tokens: 167, 172
+// before (fp32 activations 168, 191).
+// (The streaming kernel has no register left for this split: 60 bytes spill in its loop, 843 us for 24 layers of 64 requests
+// instead of 740.)  A warp
 // only ever reads and writes its own 16 rows of the tile, so tokens need no
 // ordering between warps beyond the body's own meeting, which is empty unless
 // there is one residual scale per head.  That scale is carried in a register:
@@ -26,6 +32,86 @@ int launch_multi(const KParams& p, int T, long long stride_mixed_t, long long st
 
 namespace {
 
+// k and q of a tile as every warp reads them: fp32, times k_mul and q_mul, each quad of columns as {0, 2, 1, 3}.  Quad `Q`
+// (columns 4Q..4Q+3) is quad m = 4 * (Q / 16) + Q % 4 of lane t = Q / 4 % 4, since lane t of a row holds columns 16t..16t+15
+// (m < 4) and 64+16t..64+16t+15, and lies at 4 * m + t.
+struct __align__(16) KqBuf { float4 k[32], q[32]; };
+// A lane's place in a tile: the offset of its codes (first row * 128 + first column)
+struct SlotLane {
+  int codes;
+  __device__ __forceinline__ int row() const { return codes >> 7; }
+  __device__ __forceinline__ int k() const { return codes & 127; }                   // offset of its first quad of k
+};
+__device__ __forceinline__ SlotLane slot_lane(int gw, int lane) {
+  SlotLane at = {(16 * gw + (lane >> 2)) * kT + 16 * (lane & 3)};
+  // kept in a register: worked out again from the thread index wherever it is used it costs 40 instructions per tile
+  asm volatile("" : "+r"(at.codes));
+  return at;
+}
+// quad m of k (q: 512 bytes on) from shared memory, read again for each use on purpose: they must not stay in registers
+template <int TAG, int VEC>
+__device__ __forceinline__ float4 slot_quad(uint32_t addr, int m) {
+  constexpr int B = 512 * VEC;
+  return (m == 0) ? lds_f4_at<B, TAG>(addr) : (m == 1) ? lds_f4_at<B + 64, TAG>(addr) : (m == 2) ? lds_f4_at<B + 128, TAG>(addr)
+         : (m == 3) ? lds_f4_at<B + 192, TAG>(addr) : (m == 4) ? lds_f4_at<B + 256, TAG>(addr) : (m == 5) ? lds_f4_at<B + 320, TAG>(addr)
+         : (m == 6) ? lds_f4_at<B + 384, TAG>(addr) : lds_f4_at<B + 448, TAG>(addr);
+}
+// one vector, k or q, by one warp, lane = quad
+__device__ __forceinline__ void put_quad(float4 x, int Q, float mul, float4* to) {
+  to[4 * (4 * (Q >> 4) + (Q & 3)) + ((Q >> 2) & 3)] = make_float4(x.x * mul, x.z * mul, x.y * mul, x.w * mul);
+}
+template <int QDT>
+__device__ __forceinline__ void prepare_vector(const uint8_t* vec, int Q, float mul, float4* to) { put_quad(act4<QDT>(vec, 4 * Q), Q, mul, to); }
+// Four sums over a row's 4 lanes: lane t ends up with x[t]'s
+__device__ __forceinline__ float row_sums4(const float (&x)[4], int t) {
+  const bool up2 = t & 2, up1 = t & 1;
+  float a[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) a[i] = (up2 ? x[2 + i] : x[i]) + __shfl_xor_sync(0xffffffffu, up2 ? x[i] : x[2 + i], 2);
+  return (up1 ? a[1] : a[0]) + __shfl_xor_sync(0xffffffffu, up1 ? a[0] : a[1], 1);
+}
+
+// max over the 4 lanes of a row, in each of them
+__device__ __forceinline__ float row_max(float x) {
+  x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 1));
+  return fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 2));
+}
+
+__device__ __forceinline__ void shared_max_if(bool on, uint32_t* word, uint32_t v) {
+  asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %0, 0;\n@p red.shared.max.u32 [%1], %2;\n}\n" ::"r"((int)on), "r"(smem_u32(word)), "r"(v) : "memory");
+}
+// redecide_rec for the elements of a quad.  A call: it is rarely needed, and written out at every quad it is a third of the
+// kernel's code (501 us instead of 488 for 8 layers of 32 requests, 4 tokens).
+struct QuadCodes { float2 E, O; uint32_t cw; };
+__device__ __noinline__ QuadCodes redecide_shared(QuadCodes x, float s, float thr) {
+  float2 yE = add2(s8x2_to_float<0, 2>(x.cw ^ 0x80808080u), splat(kMagicRound));
+  float2 yO = add2(s8x2_to_float<1, 3>(x.cw ^ 0x80808080u), splat(kMagicRound));
+  redecide_rec(x.E.x, yE.x, s, thr); redecide_rec(x.E.y, yE.y, s, thr);
+  redecide_rec(x.O.x, yO.x, s, thr); redecide_rec(x.O.y, yO.y, s, thr);
+  x.cw = pack4(__float_as_uint(yE.x), __float_as_uint(yO.x), __float_as_uint(yE.y), __float_as_uint(yO.y));
+  return x;
+}
+
+// the codes of a quad's even and odd columns
+__device__ __forceinline__ float2 slot_codes_even(uint32_t w) { return s8x2_cvt<0, 2>(w); }
+__device__ __forceinline__ float2 slot_codes_odd(uint32_t w) { return s8x2_to_float<1, 3>(w ^ 0x80808080u); }
+// store_from_float without a branch on the type, for lanes with `on` set: what is not theirs to write is converted as well.
+__device__ __forceinline__ void store_from_float_if(bool on, uint8_t* p, int i, int dtype, float x) {
+  const bool wide = dtype == CARRY_F32;
+  const unsigned short half = (dtype == CARRY_BF16) ? __bfloat16_as_ushort(__float2bfloat16_rn(x)) : __half_as_ushort(__float2half_rn(x));
+  asm volatile(
+      "{\n"
+      ".reg .pred w, n;\n"
+      "setp.ne.u32 w, %0, 0;\n"
+      "setp.ne.u32 n, %1, 0;\n"
+      "@w st.global.f32 [%2], %3;\n"
+      "@n st.global.u16 [%2], %4;\n"
+      "}\n" ::"r"((int)(on && wide)), "r"((int)(on && !wide)),
+      "l"(p + i * (wide ? 4 : 2)), "f"(x), "h"(half)
+      : "memory");
+}
+
+
 struct MultiExtra {
   int T;
   long long stride_mixed_t, stride_a_t, stride_b_t;   // elements from one token of a request to the next
@@ -40,11 +126,11 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_multi_kernel(const __grid_con
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ __align__(8) uint64_t full_bar;
   __shared__ int poison_flag;
-  __shared__ float head_red[2][kWarps];
+  __shared__ uint32_t head_max[4];                    // largest new residual of a token, as bits, by token mod 4
   constexpr int kChunk = 8;                           // tokens whose activations and facts are fetched together
   __shared__ TileMeta meta_t[kChunk];
   __shared__ __align__(16) uint8_t vec_t[kChunk][3 * L::kVecBytes];   // raw q | k | v per token
-  __shared__ __align__(16) float q_warp[kWarps * kT];
+  __shared__ KqBuf kq_t[kChunk];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gw = warp, gtid = tid;
   uint8_t* sb = smem;
@@ -88,6 +174,7 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_multi_kernel(const __grid_con
 #pragma unroll
     for (int i = 0; i < 8; ++i) addr[i] = a8[i];
     poison_flag = 0;
+    head_max[0] = head_max[1] = head_max[2] = head_max[3] = 0u;
     mbar_init(&full_bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     // the state of the tile: codes, residual, state scales, residual scale(s)
@@ -102,6 +189,7 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_multi_kernel(const __grid_con
   const float rqmax_state = p.inv_qmax;
   bool healthy = true;
 
+  const SlotLane at = slot_lane(gw, lane);
   float es_head = 0.f;                               // one residual scale per head: carried from token to token
   for (int t = 0; t < x.T; ++t) {
     const int tc = t % kChunk;
@@ -122,6 +210,11 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_multi_kernel(const __grid_con
                                      (long long)(t + warp) * x.stride_mixed_t, (long long)(t + warp) * x.stride_a_t,
                                      (long long)(t + warp) * x.stride_b_t);
       __syncthreads();
+      if (warp < nt) {
+        prepare_vector<QDT>(&vec_t[warp][0], lane, meta_t[warp].q_mul, kq_t[warp].q);
+        prepare_vector<QDT>(&vec_t[warp][L::kVecBytes], lane, meta_t[warp].k_mul, kq_t[warp].k);
+      }
+      __syncthreads();
     }
     if (t == 0) {                                    // the tile has to be there; the verdict is the CTA's, not a warp's
       mbar_wait(&full_bar, 0u, poison, p.status);
@@ -132,53 +225,213 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_multi_kernel(const __grid_con
     if (!healthy) break;
 
     const uint4 tm0 = lds_v4(&meta_t[tc]), tm1 = lds_v4(reinterpret_cast<const uint8_t*>(&meta_t[tc]) + 16);
-    const float alpha = __uint_as_float(tm0.w), beta = __uint_as_float(tm1.x), k_mul = __uint_as_float(tm1.y),
-                q_mul = __uint_as_float(tm1.z), kq = __uint_as_float(tm1.w);
+    const float alpha = __uint_as_float(tm0.w), beta = __uint_as_float(tm1.x), kq = __uint_as_float(tm1.w);
     const float* sscale = reinterpret_cast<const float*>(sb + L::kSScale);
     const float* rscale = reinterpret_cast<const float*>(sb + L::kRScale);
     const float2 alpha2 = splat(alpha);
     const float2 magic2 = splat(kMagicRound), nmagic2 = splat(-kMagicRound);
-    const long long out_tok = out_tok0 + (long long)t * out_tok_stride;
+    uint8_t* out_to = reinterpret_cast<uint8_t*>(p.out) + (out_tok0 + (long long)t * out_tok_stride) * (p.o_dtype == CARRY_F32 ? 4 : 2);
 
-#define CARRY_SLOT_VEC_Q (&vec_t[tc][0])
-#define CARRY_SLOT_VEC_K (&vec_t[tc][L::kVecBytes])
-#define CARRY_SLOT_VEC_V (&vec_t[tc][2 * L::kVecBytes])
-#define CARRY_SLOT_OUT(idx, value) store_from_float(p.out, out_tok + (idx), p.o_dtype, (value))
-#define CARRY_SLOT_PUT_SSCALE(r0_, v4_) *reinterpret_cast<uint4*>(sb + L::kSScale + (r0_) * 4) = (v4_)
-#define CARRY_SLOT_PUT_CODES(r0_, c0_, cw_)                                                                        \
-  {                                                                                                                \
-    _Pragma("unroll") for (int i_ = 0; i_ < 4; ++i_)                                                               \
-        *reinterpret_cast<uint4*>(sb + L::kCodes + ((r0_) + i_) * kT + (c0_)) =                                    \
-        make_uint4(cw_[i_][0], cw_[i_][1], cw_[i_][2], cw_[i_][3]);                                                \
-  }
-#define CARRY_SLOT_HEAD_RED head_red[t & 1]
-#define CARRY_SLOT_MEET(statement)                \
-  if constexpr (RSCALE == CARRY_SCALE_PER_HEAD) { \
-    if (lane == 0) { statement; }                 \
-    warps_meet(3);                                \
-  }
-#define CARRY_SLOT_RESID_BEGIN()
-#define CARRY_SLOT_PUT_RESID4(i_, r0_, c0_, w_) \
-  *reinterpret_cast<uint2*>(sb + L::kResid + ((r0_) + (i_)) * (kT / 2) + (c0_) / 2) = (w_)
-#define CARRY_SLOT_PUT_RESID8(i_, r0_, c0_, w_) *reinterpret_cast<uint4*>(sb + L::kResid + ((r0_) + (i_)) * kT + (c0_)) = (w_)
-#define CARRY_SLOT_PUT_RSCALE_V(r0_, v4_) *reinterpret_cast<uint4*>(sb + L::kRScale + (r0_) * 4) = (v4_)
-#define CARRY_SLOT_PUT_RSCALE_HEAD(bits_) reinterpret_cast<uint32_t*>(sb + L::kRScale)[hv & 3] = (bits_)
-#include "carry_gdn_slot_tile.inc"
+    auto put_out = [&](bool on, int idx, float value) { store_from_float_if(on, out_to, idx, p.o_dtype, value); };
+    auto put_sscale = [&](bool on, int r, uint32_t bits) { if (on) *reinterpret_cast<uint32_t*>(sb + L::kSScale + r * 4) = bits; };
+    auto put_rscale = [&](bool on, int r, uint32_t bits) { if (on) *reinterpret_cast<uint32_t*>(sb + L::kRScale + r * 4) = bits; };
+    auto put16 = [](uint8_t* to, int offset, uint4 v) { *reinterpret_cast<uint4*>(to + offset) = v; };
+    auto put8 = [](uint8_t* to, int offset, uint2 v) { *reinterpret_cast<uint2*>(to + offset) = v; };
+    // A quad of columns (one 32-bit word of codes) is held as two pairs: E = {col 0, col 2}, O = {col 1, col 3}.
+    // Int4 residual: the dot products run over the bare codes (the row's scale * decay goes on the
+    // totals) and the target is three fused multiply-adds per pair (phase 2).  Against the int8-residual
+    // form below, which keeps the reference's order of roundings, a target moves by a few units in the
+    // last place: measured 2e-6 of the state codes and 3e-5 of the int4 residual codes differ from the
+    // oracle's, each by one step (limit 1e-3).  An int8 residual code is 18 times finer and already
+    // differs in 3e-4 of the elements from reduction order alone, so that format keeps the exact order.
+    constexpr bool kFold = (RES == CARRY_RES_INT4);
+    const bool odd = lane & 1;
+    const uint8_t* codes_at = sb + L::kCodes + at.codes;
+    const uint8_t* resid_at = sb + L::kResid + (RES == CARRY_RES_INT4 ? at.codes / 2 : at.codes);
+    const float* sscale_at = reinterpret_cast<const float*>(sb + L::kSScale) + at.row();
+    const uint32_t k_addr = smem_u32(&kq_t[tc]) + at.k() + order_token();
+    float2 hE[2][8], hO[2][8];            // [row][quad]
+    // phase 1: dequantise, decay, dot products: per 16 columns one chain for each half of a pair, then over the 8 runs of 16
+    const float srow[2] = {sscale_at[0], sscale_at[8]};
+    float dot_mine;      // lanes 0..3 of a row pair: <row, k>, <row + 8, k>, <row, q>, <row + 8, q>
+    {
+      float part[4];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        uint32_t w[2][4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const uint4 x = *reinterpret_cast<const uint4*>(codes_at + 8 * kT * i + 64 * j);
+          w[i][0] = x.x; w[i][1] = x.y; w[i][2] = x.z; w[i][3] = x.w;
+        }
+        float2 acc[4] = {};
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+          const int m = 4 * j + n;
+          const float4 kk = slot_quad<2, 0>(k_addr, m), qq = slot_quad<2, 1>(k_addr, m);
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            // half of the bytes through the conversion pipe, half through byte permutes (all through either: no gain
+            // for int4, 5 % slower for int8)
+            float2 e = slot_codes_even(w[i][n]), o = slot_codes_odd(w[i][n]);
+            if constexpr (!kFold) { e = mul2(mul2(e, splat(srow[i])), alpha2); o = mul2(mul2(o, splat(srow[i])), alpha2); }
+            hE[i][m] = e; hO[i][m] = o;
+            acc[i] = fma2(o, make_float2(kk.z, kk.w), fma2(e, make_float2(kk.x, kk.y), acc[i]));
+            acc[2 + i] = fma2(o, make_float2(qq.z, qq.w), fma2(e, make_float2(qq.x, qq.y), acc[2 + i]));
+          }
+        }
+#pragma unroll
+        for (int v = 0; v < 4; ++v) part[v] = j ? part[v] + (acc[v].x + acc[v].y) : acc[v].x + acc[v].y;
+      }
+      dot_mine = row_sums4(part, lane & 3);
+      // folded form: the sums ran over the bare codes; the row's scale * decay goes on the total
+      if constexpr (kFold) dot_mine *= (odd ? srow[1] : srow[0]) * alpha;
+    }
+    float dv[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      dv[i] = __fmul_rn(beta, __fadd_rn(act<QDT>(&vec_t[tc][2 * L::kVecBytes], at.row() + 8 * i), -__shfl_sync(0xffffffffu, dot_mine, (lane & 28) + i)));
+    // the lanes that hold a q total finish that row's output
+    put_out(lane & 2, at.row() + (odd ? 8 : 0), fmaf(odd ? dv[1] : dv[0], kq, dot_mine));
+    // The two rows one after the other, so that the first one's exchange of maxima hides behind the second one's arithmetic.
+    float snew[2], emax[2];
+    uint32_t cw[2][8];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      // phase 2: dequantise, decay, rank-1 write and residual, each one fused multiply-add; row maximum
+      const float es = (RSCALE == CARRY_SCALE_PER_V) ? reinterpret_cast<const float*>(sb + L::kRScale)[at.row() + 8 * i] : es_head;
+      const float2 dv2 = splat(dv[i]), es2 = splat(es);
+      float amax = 0.f;
+      if constexpr (kFold) {
+        // target = code * (scale * decay) + k * dv + nibble * es, as three fused multiply-adds.  A
+        // nibble (offset binary, 0..15) lands in the byte above a float's low half-word under the
+        // exponent of 128, which reads 136 + code; the 136 * es goes into the innermost addend, so the
+        // decode costs no arithmetic beyond the byte permute.
+        const float2 nb2 = splat(-136.0f * es), sa2 = splat(srow[i] * alpha);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const uint2 rw = *reinterpret_cast<const uint2*>(resid_at + 8 * (kT / 2) * i + 32 * j);
+          const uint32_t wl[2] = {(rw.x ^ 0x88888888u) & 0x0F0F0F0Fu, (rw.y ^ 0x88888888u) & 0x0F0F0F0Fu};
+          const uint32_t wh[2] = {((rw.x ^ 0x88888888u) >> 4) & 0x0F0F0F0Fu, ((rw.y ^ 0x88888888u) >> 4) & 0x0F0F0F0Fu};
+#pragma unroll
+          for (int n = 0; n < 4; ++n) {
+            const int m = 4 * j + n;
+            const float2 lo = (n & 1) ? nib2_biased<2, 3>(wl[n >> 1]) : nib2_biased<0, 1>(wl[n >> 1]);
+            const float2 hi = (n & 1) ? nib2_biased<2, 3>(wh[n >> 1]) : nib2_biased<0, 1>(wh[n >> 1]);
+            const float4 kk = i ? slot_quad<1, 0>(k_addr, m) : slot_quad<0, 0>(k_addr, m);
+            hE[i][m] = fma2(lo, es2, fma2(hE[i][m], sa2, fma2(make_float2(kk.x, kk.y), dv2, nb2)));
+            hO[i][m] = fma2(hi, es2, fma2(hO[i][m], sa2, fma2(make_float2(kk.z, kk.w), dv2, nb2)));
+            amax = max3abs(max3abs(amax, hE[i][m]), hO[i][m]);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const uint4 rw = *reinterpret_cast<const uint4*>(resid_at + 8 * kT * i + 64 * j);
+          const uint32_t r[4] = {rw.x, rw.y, rw.z, rw.w};
+#pragma unroll
+          for (int n = 0; n < 4; ++n) {
+            const int m = 4 * j + n;
+            const float4 kk = i ? slot_quad<1, 0>(k_addr, m) : slot_quad<0, 0>(k_addr, m);
+            hE[i][m] = fma2(slot_codes_even(r[n]), es2, fma2(make_float2(kk.x, kk.y), dv2, hE[i][m]));
+            hO[i][m] = fma2(slot_codes_odd(r[n]), es2, fma2(make_float2(kk.z, kk.w), dv2, hO[i][m]));
+            amax = max3abs(max3abs(amax, hE[i][m]), hO[i][m]);
+          }
+        }
+      }
+      // phase 3: state scale and codes, new residual.  target - code * scale is one fused multiply-add, which is
+      // exact here (the difference of two nearly equal numbers), so the target can be rebuilt from the
+      // remainder when an element has to be re-decided.  No branch until both rows are done.
+      snew[i] = scale_fast(row_max(amax), p.qmax, rqmax_state, p.eps_mode);
+      const float2 inv2 = splat(rcp_refined(snew[i])), ns2 = splat(-snew[i]);
+      float em = 0.f;
+#pragma unroll
+      for (int m = 0; m < 8; ++m) {
+        const float2 yE = fma2(hE[i][m], inv2, magic2);
+        const float2 yO = fma2(hO[i][m], inv2, magic2);
+        hE[i][m] = fma2(add2(yE, nmagic2), ns2, hE[i][m]);
+        hO[i][m] = fma2(add2(yO, nmagic2), ns2, hO[i][m]);
+        em = max3abs(max3abs(em, hE[i][m]), hO[i][m]);
+        cw[i][m] = pack4(__float_as_uint(yE.x), __float_as_uint(yO.x), __float_as_uint(yE.y), __float_as_uint(yO.y));
+      }
+      emax[i] = em;
+    }
+    put_sscale((lane & 2) == 0, at.row() + (odd ? 8 : 0), __float_as_uint(odd ? snew[1] : snew[0]));
+    // Some quotient within the tie guard: on activations that change, one warp in 20 per tile; on ones that repeat for 100
+    // steps and more an int8 residual settles where a third to half of the warps have one.  The others wait for that warp at
+    // the meeting.  Only the quads with such an element are gone through again.
+    if (fmaxf(fmaf(-snew[0], kTieGuardExact, emax[0]), fmaf(-snew[1], kTieGuardExact, emax[1])) > 0.f) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const float thr = snew[i] * kTieGuardExact;
+        if (emax[i] > thr) {
+          float em = 0.f;
+#pragma unroll
+          for (int m = 0; m < 8; ++m) {
+            if (max3abs(max3abs(0.f, hE[i][m]), hO[i][m]) > thr) {
+              const QuadCodes x = redecide_shared({hE[i][m], hO[i][m], cw[i][m]}, snew[i], thr);
+              hE[i][m] = x.E; hO[i][m] = x.O; cw[i][m] = x.cw;
+            }
+            em = max3abs(max3abs(em, hE[i][m]), hO[i][m]);
+          }
+          emax[i] = em;
+        }
+      }
+    }
+    {
+      const auto to = (sb + L::kCodes) + at.codes;
+      put16(to, 0, make_uint4(cw[0][0], cw[0][1], cw[0][2], cw[0][3]));
+      put16(to, 64, make_uint4(cw[0][4], cw[0][5], cw[0][6], cw[0][7]));
+      put16(to, 8 * kT, make_uint4(cw[1][0], cw[1][1], cw[1][2], cw[1][3]));
+      put16(to, 8 * kT + 64, make_uint4(cw[1][4], cw[1][5], cw[1][6], cw[1][7]));
+    }
+    // phase 4: residual scale and codes
+    float esn[2];
+    if constexpr (RSCALE == CARRY_SCALE_PER_V) {
+      // no data crosses warps here
+#pragma unroll
+      for (int i = 0; i < 2; ++i) esn[i] = scale_fast(row_max(emax[i]), rqmax, rrqmax, p.eps_mode);
+    } else {
+      const uint32_t warp_max = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(emax[0], emax[1])));
+      shared_max_if(lane == 0, &head_max[t & 3], warp_max);
+      if (tid == 0) head_max[(t + 2) & 3] = 0u;        // last read two meetings ago
+      __syncthreads();
+      esn[0] = esn[1] = scale_fast(__uint_as_float(*const_cast<volatile uint32_t*>(&head_max[t & 3])), rqmax, rrqmax, p.eps_mode);
+    }
+    const auto resid_to = (sb + L::kResid) + (RES == CARRY_RES_INT4 ? at.codes / 2 : at.codes);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float2 inv2 = splat(rcp_refined(esn[i]));
+      if constexpr (RES == CARRY_RES_INT4) {
+        // even columns: rint(e/es) + 8 + 128 lands in the low mantissa bits; 16 * rint(e/es) of the odd
+        // column is added on top, so the low byte of the sum is (odd + 8) << 4 | (even + 8); the final
+        // XOR removes the bias of both nibbles.
+        const float2 mE = splat(kMagicRound + 136.0f), sixteen = splat(16.0f);
+        uint32_t word[4];
+#pragma unroll
+        for (int m = 0; m < 8; m += 2) {
+          const float2 a = fma2(add2(fma2(hO[i][m], inv2, magic2), nmagic2), sixteen, fma2(hE[i][m], inv2, mE));
+          const float2 b = fma2(add2(fma2(hO[i][m + 1], inv2, magic2), nmagic2), sixteen, fma2(hE[i][m + 1], inv2, mE));
+          word[m / 2] = pack4(__float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(b.x), __float_as_uint(b.y)) ^ 0x88888888u;
+        }
+        put8(resid_to, 8 * (kT / 2) * i, make_uint2(word[0], word[1]));
+        put8(resid_to, 8 * (kT / 2) * i + 32, make_uint2(word[2], word[3]));
+      } else {
+        uint32_t word[8];
+#pragma unroll
+        for (int m = 0; m < 8; ++m) {
+          const float2 ye = fma2(hE[i][m], inv2, magic2), yo = fma2(hO[i][m], inv2, magic2);
+          word[m] = pack4(__float_as_uint(ye.x), __float_as_uint(yo.x), __float_as_uint(ye.y), __float_as_uint(yo.y));
+        }
+        put16(resid_to, 8 * kT * i, make_uint4(word[0], word[1], word[2], word[3]));
+        put16(resid_to, 8 * kT * i + 64, make_uint4(word[4], word[5], word[6], word[7]));
+      }
+    }
+    if (RSCALE == CARRY_SCALE_PER_V)
+      put_rscale((lane & 2) == 0, at.row() + (odd ? 8 : 0), __float_as_uint(odd ? esn[1] : esn[0]));
+    if (RSCALE == CARRY_SCALE_PER_HEAD && gtid == 0) reinterpret_cast<uint32_t*>(sb + L::kRScale)[hv & 3] = __float_as_uint(esn[0]);
     if constexpr (RSCALE == CARRY_SCALE_PER_HEAD) es_head = esn[0];
     __syncwarp();                                    // a warp's rows are its own: written by one lane, read by another
-#undef CARRY_SLOT_VEC_Q
-#undef CARRY_SLOT_VEC_K
-#undef CARRY_SLOT_VEC_V
-#undef CARRY_SLOT_OUT
-#undef CARRY_SLOT_PUT_SSCALE
-#undef CARRY_SLOT_PUT_CODES
-#undef CARRY_SLOT_HEAD_RED
-#undef CARRY_SLOT_MEET
-#undef CARRY_SLOT_RESID_BEGIN
-#undef CARRY_SLOT_PUT_RESID4
-#undef CARRY_SLOT_PUT_RESID8
-#undef CARRY_SLOT_PUT_RSCALE_V
-#undef CARRY_SLOT_PUT_RSCALE_HEAD
   }
 
   __syncthreads();
