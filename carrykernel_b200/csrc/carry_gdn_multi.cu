@@ -80,10 +80,13 @@ __device__ __forceinline__ float row_max(float x) {
 __device__ __forceinline__ void shared_max_if(bool on, uint32_t* word, uint32_t v) {
   asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %0, 0;\n@p red.shared.max.u32 [%1], %2;\n}\n" ::"r"((int)on), "r"(smem_u32(word)), "r"(v) : "memory");
 }
-// redecide_rec for the elements of a quad.  A call: it is rarely needed, and written out at every quad it is a third of the
-// kernel's code (2.6 % of the time of 8 layers of 32 requests, 4 tokens).
+// redecide_rec for the elements of a quad.  It is rarely needed, and written out at every quad it is a third of the kernel's code,
+// so that it is a call -- except with an int8 residual and a scale per V row, where the compiler's code around the call costs more
+// than the call saves.  Call / in line, us a launch of 32 requests x 32 heads, 4 tokens: int4, one scale per head 62.4 / 63.0;
+// int4, per V row 56.2 / 57.3; int8, one scale per head 63.5 / 63.9; int8, per V row 59.7 / 57.8 (fp32 activations 61.3 / 59.5;
+// 8 requests of 2 tokens 12.7 / 12.4).  New activations at every token or the same ones: alike.
 struct QuadCodes { float2 E, O; uint32_t cw; };
-__device__ __noinline__ QuadCodes redecide_shared(QuadCodes x, float s, float thr) {
+__device__ __forceinline__ QuadCodes redecide_here(QuadCodes x, float s, float thr) {
   float2 yE = add2(s8x2_to_float<0, 2>(x.cw ^ 0x80808080u), splat(kMagicRound));
   float2 yO = add2(s8x2_to_float<1, 3>(x.cw ^ 0x80808080u), splat(kMagicRound));
   redecide_rec(x.E.x, yE.x, s, thr); redecide_rec(x.E.y, yE.y, s, thr);
@@ -91,6 +94,7 @@ __device__ __noinline__ QuadCodes redecide_shared(QuadCodes x, float s, float th
   x.cw = pack4(__float_as_uint(yE.x), __float_as_uint(yO.x), __float_as_uint(yE.y), __float_as_uint(yO.y));
   return x;
 }
+__device__ __noinline__ QuadCodes redecide_shared(QuadCodes x, float s, float thr) { return redecide_here(x, s, thr); }
 
 // the codes of a quad's even and odd columns
 __device__ __forceinline__ float2 slot_codes_even(uint32_t w) { return s8x2_cvt<0, 2>(w); }
@@ -360,6 +364,7 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_multi_kernel(const __grid_con
     // Some quotient within the tie guard: on activations that change, one warp in 20 per tile; on ones that repeat for 100
     // steps and more an int8 residual settles where a third to half of the warps have one.  The others wait for that warp at
     // the meeting.  Only the quads with such an element are gone through again.
+    constexpr bool kInLine = RES == CARRY_RES_INT8 && RSCALE == CARRY_SCALE_PER_V;
     if (fmaxf(fmaf(-snew[0], kTieGuardExact, emax[0]), fmaf(-snew[1], kTieGuardExact, emax[1])) > 0.f) {
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
@@ -369,7 +374,8 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_multi_kernel(const __grid_con
 #pragma unroll
           for (int m = 0; m < 8; ++m) {
             if (max3abs(max3abs(0.f, hE[i][m]), hO[i][m]) > thr) {
-              const QuadCodes x = redecide_shared({hE[i][m], hO[i][m], cw[i][m]}, snew[i], thr);
+              const QuadCodes q = {hE[i][m], hO[i][m], cw[i][m]};
+              const QuadCodes x = kInLine ? redecide_here(q, snew[i], thr) : redecide_shared(q, snew[i], thr);
               hE[i][m] = x.E; hO[i][m] = x.O; cw[i][m] = x.cw;
             }
             em = max3abs(max3abs(em, hE[i][m]), hO[i][m]);
