@@ -9,19 +9,22 @@
 // (carry_gdn_slot_tile.inc), operation for operation and sum for sum, over another split: a lane holds 32 columns (two runs of 16)
 // of 2 rows, 8 apart, where it holds 16 columns of 4 rows there.  Sums and maxima then go over 4 lanes instead of 8 and every
 // lane has two rows' scalars to work out instead of four.  k and q of a token, scaled, are laid out once for all warps instead
-// of once per warp, and the output's store has no branches.  Bound: the FMA and ALU pipes, whose busy cycles do not overlap; what is
-// taken off either is the gain.  8 layers of 32 requests, 4 tokens: 495 us, 513 before; a launch of 64 requests, 6 tokens: 167, 172
-// before (fp32 activations 168, 191).
+// of once per warp, and the output's store has no branches.  32 requests x 32 heads, us a launch of 4 tokens with the other split
+// and with this one: int4, one residual scale per head 64.5 / 62.4, per V row 61.5 / 56.2, int8 per V row 61.0 / 57.8; fp32 activations
+// 71.4 / 63.3, 67.3 / 59.5 (int8).  One token, 16-bit activations: 30.9 / 30.8, 31.0 / 30.3, 32.9 / 32.4; up to 16 requests
+// level to 1.5 % or ahead.
+// Bound: the FMA and ALU pipes, busy for 37 and 38 % of the cycles -- their times add up for most of these instructions, which read
+// more than two or three registers -- and, with one scale per head, the meeting of the 8 warps at every token.
+// The split's price: rows lie 128 bytes apart (64 for int4), so that the lanes of a 16-byte phase meet on half of the banks: 50 conflicts
+// per warp and token, 1.65 M of 6.6 M shared-memory wavefronts of a launch.
 // (The streaming kernel has no register left for this split: 60 bytes spill in its loop, 843 us for 24 layers of 64 requests
-// instead of 740.)  A warp
-// only ever reads and writes its own 16 rows of the tile, so tokens need no
-// ordering between warps beyond the body's own meeting, which is empty unless
-// there is one residual scale per head.  That scale is carried in a register:
-// read back from the staged tile, it takes a block barrier per token (8 layers of
-// 32 requests, 4 tokens: 524 us instead of 513; with a scale per V row, where the
-// barrier held warps together that need nothing from one another, 538 instead of
-// 490 for int4, 535 instead of 488 for int8).  Activation vectors, gates and norms
-// of up to 8 tokens are fetched together, one trip to global memory per chunk of
+// instead of 740.)
+//
+// A warp only ever reads and writes its own 16 rows of the tile, so tokens need no ordering between warps beyond that meeting, which
+// is there only with one residual scale per head.  That scale is carried in a register; read back from the staged tile it takes a block
+// barrier per token, which is 62.4 us just the same.  With a scale per V row a barrier would hold warps together that need
+// nothing from one another: 60.6 instead of 56.2 us for int4, 64.2 instead of 59.7 for int8 (whose re-decision was a call then).
+// Activation vectors, gates and norms of up to 8 tokens are fetched together, one trip to global memory per chunk of
 // tokens instead of one per token.
 #include "carry_gdn_tile128.cuh"
 
@@ -42,8 +45,8 @@ struct SlotLane {
   __device__ __forceinline__ int row() const { return codes >> 7; }
   __device__ __forceinline__ int k() const { return codes & 127; }                   // offset of its first quad of k
 };
-__device__ __forceinline__ SlotLane slot_lane(int gw, int lane) {
-  SlotLane at = {(16 * gw + (lane >> 2)) * kT + 16 * (lane & 3)};
+__device__ __forceinline__ SlotLane slot_lane(int warp, int lane) {
+  SlotLane at = {(16 * warp + (lane >> 2)) * kT + 16 * (lane & 3)};
   // kept in a register: worked out again from the thread index wherever it is used it costs 40 instructions per tile
   asm volatile("" : "+r"(at.codes));
   return at;
@@ -115,7 +118,6 @@ __device__ __forceinline__ void store_from_float_if(bool on, uint8_t* p, int i, 
       : "memory");
 }
 
-
 struct MultiExtra {
   int T;
   long long stride_mixed_t, stride_a_t, stride_b_t;   // elements from one token of a request to the next
@@ -136,17 +138,17 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_multi_kernel(const __grid_con
   __shared__ __align__(16) uint8_t vec_t[kChunk][3 * L::kVecBytes];   // raw q | k | v per token
   __shared__ KqBuf kq_t[kChunk];
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gw = warp, gtid = tid;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   uint8_t* sb = smem;
   volatile int* poison = &poison_flag;
   const int tile = (int)blockIdx.x;
   int n, hv, h;
   split_tile(p, tile, n, hv, h);
   // CTAs that the launch ahead leaves room for start while its last ones run.  What they may do before it has finished
-  // is ask the L2 for the state of the slot that the index names now.  Against a launch that starts when the one ahead
-  // has ended: 3 us less per launch (32 requests x 32 heads, 4 tokens: 69.1 -> 65.9 us; 2 tokens: 43.4 -> 41.3).  The CTAs
+  // is ask the L2 for the state of the slot that the index names now.  32 requests x 32 heads, 4 tokens (1 token): 62.4 us a launch
+  // (30.7); launches that start when the one ahead has ended 63.3 (31.3), an early start without hints 63.1 (31.1).  The CTAs
   // behind the first wave find the launch ahead finished, and the look at the index is in their way: hints from all
-  // of them, 66.4 and 41.9 us.
+  // of them, 62.9 (31.0).
   depend_release();
   if (tid == 0 && (int)blockIdx.x < x.first_wave) {
     const long long guess = __ldcg(p.slot_idx + (long long)n * p.stride_idx);
@@ -193,7 +195,7 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_multi_kernel(const __grid_con
   const float rqmax_state = p.inv_qmax;
   bool healthy = true;
 
-  const SlotLane at = slot_lane(gw, lane);
+  const SlotLane at = slot_lane(warp, lane);
   float es_head = 0.f;                               // one residual scale per head: carried from token to token
   for (int t = 0; t < x.T; ++t) {
     const int tc = t % kChunk;
@@ -230,8 +232,6 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_multi_kernel(const __grid_con
 
     const uint4 tm0 = lds_v4(&meta_t[tc]), tm1 = lds_v4(reinterpret_cast<const uint8_t*>(&meta_t[tc]) + 16);
     const float alpha = __uint_as_float(tm0.w), beta = __uint_as_float(tm1.x), kq = __uint_as_float(tm1.w);
-    const float* sscale = reinterpret_cast<const float*>(sb + L::kSScale);
-    const float* rscale = reinterpret_cast<const float*>(sb + L::kRScale);
     const float2 alpha2 = splat(alpha);
     const float2 magic2 = splat(kMagicRound), nmagic2 = splat(-kMagicRound);
     uint8_t* out_to = reinterpret_cast<uint8_t*>(p.out) + (out_tok0 + (long long)t * out_tok_stride) * (p.o_dtype == CARRY_F32 ? 4 : 2);
@@ -435,7 +435,7 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_multi_kernel(const __grid_con
     }
     if (RSCALE == CARRY_SCALE_PER_V)
       put_rscale((lane & 2) == 0, at.row() + (odd ? 8 : 0), __float_as_uint(odd ? esn[1] : esn[0]));
-    if (RSCALE == CARRY_SCALE_PER_HEAD && gtid == 0) reinterpret_cast<uint32_t*>(sb + L::kRScale)[hv & 3] = __float_as_uint(esn[0]);
+    if (RSCALE == CARRY_SCALE_PER_HEAD && tid == 0) reinterpret_cast<uint32_t*>(sb + L::kRScale)[hv & 3] = __float_as_uint(esn[0]);
     if constexpr (RSCALE == CARRY_SCALE_PER_HEAD) es_head = esn[0];
     __syncwarp();                                    // a warp's rows are its own: written by one lane, read by another
   }

@@ -278,15 +278,6 @@ __device__ __forceinline__ uint32_t float4_to_e5m2x4(float2 ab, float2 cd) {
   const uint32_t hi = __nv_cvt_float2_to_fp8x2(cd, __NV_SATFINITE, __NV_E5M2);
   return lo | (hi << 16);
 }
-// bytes A and B of a word whose low nibbles (wl = w & 0x0F0F0F0F) and high nibbles (wh = w & 0xF0F0F0F0) were separated
-// beforehand, each nibble already XOR-ed with 8: {low nibbles}, {16 * high nibbles}
-template <int A, int B>
-__device__ __forceinline__ void s4x4_split_to_float(uint32_t wl, uint32_t wh, float2& lo, float2& hi16) {
-  lo = add2(make_float2(__uint_as_float(__byte_perm(wl, 0x4B000000u, 0x7440 | A)),
-                        __uint_as_float(__byte_perm(wl, 0x4B000000u, 0x7440 | B))), splat(-kMagicNib));
-  hi16 = add2(make_float2(__uint_as_float(__byte_perm(wh, 0x4B000000u, 0x7440 | A)),
-                          __uint_as_float(__byte_perm(wh, 0x4B000000u, 0x7440 | B))), splat(-kMagicByte));
-}
 // low bytes of four words -> one word (a | b<<8 | c<<16 | d<<24)
 __device__ __forceinline__ uint32_t pack4(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   return __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
@@ -1013,58 +1004,7 @@ gdn_tile128_kernel(const __grid_constant__ KParams p) {
       const float2 magic2 = splat(kMagicRound), nmagic2 = splat(-kMagicRound);
 
       if constexpr (LAYOUT == LAYOUT_VK) {
-#define CARRY_SLOT_VEC_Q (sb + L::kQ)
-#define CARRY_SLOT_VEC_K (sb + L::kK)
-#define CARRY_SLOT_VEC_V (sb + L::kV)
-#define CARRY_SLOT_OUT(idx, value) store_from_float(p.out, (long long)out_row * kT + (idx), p.o_dtype, (value))
-#define CARRY_SLOT_PUT_SSCALE(r0_, v4_) stg_v4(dst_of(D_SSCALE) + (r0_) * 4, (v4_))
-#define CARRY_SLOT_PUT_CODES(r0_, c0_, cw_)                                                   \
-  {                                                                                           \
-    const unsigned long long base = dst_of(D_CODES) + (r0_) * kT + (c0_);                     \
-    stg_v4_at<0 * kT>(base, make_uint4(cw_[0][0], cw_[0][1], cw_[0][2], cw_[0][3]));          \
-    stg_v4_at<1 * kT>(base, make_uint4(cw_[1][0], cw_[1][1], cw_[1][2], cw_[1][3]));          \
-    stg_v4_at<2 * kT>(base, make_uint4(cw_[2][0], cw_[2][1], cw_[2][2], cw_[2][3]));          \
-    stg_v4_at<3 * kT>(base, make_uint4(cw_[3][0], cw_[3][1], cw_[3][2], cw_[3][3]));          \
-  }
-#define CARRY_SLOT_HEAD_RED head_red[grp][cnt & 1]
-#define CARRY_SLOT_MEET(statement)                \
-  if (lane == 0) { statement; claim_next(cnt); }  \
-  warps_meet(bar0 + 3);                           \
-  refill_stage(it)
-#define CARRY_SLOT_RESID_BEGIN() const unsigned long long dst_resid = dst_of(D_RESID)
-#define CARRY_SLOT_PUT_RESID4(i_, r0_, c0_, w_)                                    \
-  {                                                                                \
-    const unsigned long long base = dst_resid + (r0_) * (kT / 2) + (c0_) / 2;      \
-    if (i_ == 0) stg_v2_at<0 * (kT / 2)>(base, w_);                                \
-    if (i_ == 1) stg_v2_at<1 * (kT / 2)>(base, w_);                                \
-    if (i_ == 2) stg_v2_at<2 * (kT / 2)>(base, w_);                                \
-    if (i_ == 3) stg_v2_at<3 * (kT / 2)>(base, w_);                                \
-  }
-#define CARRY_SLOT_PUT_RESID8(i_, r0_, c0_, w_)                                    \
-  {                                                                                \
-    const unsigned long long base = dst_resid + (r0_) * kT + (c0_);                \
-    const uint4 pw = w_;                                                           \
-    if (i_ == 0) stg_v4_at<0 * kT>(base, pw);                                      \
-    if (i_ == 1) stg_v4_at<1 * kT>(base, pw);                                      \
-    if (i_ == 2) stg_v4_at<2 * kT>(base, pw);                                      \
-    if (i_ == 3) stg_v4_at<3 * kT>(base, pw);                                      \
-  }
-#define CARRY_SLOT_PUT_RSCALE_V(r0_, v4_) stg_v4(dst_of(D_RSCALE) + (r0_) * 4, (v4_))
-#define CARRY_SLOT_PUT_RSCALE_HEAD(bits_) stg_b32(dst_of(D_RSCALE), (bits_))
 #include "carry_gdn_slot_tile.inc"
-#undef CARRY_SLOT_VEC_Q
-#undef CARRY_SLOT_VEC_K
-#undef CARRY_SLOT_VEC_V
-#undef CARRY_SLOT_OUT
-#undef CARRY_SLOT_PUT_SSCALE
-#undef CARRY_SLOT_PUT_CODES
-#undef CARRY_SLOT_HEAD_RED
-#undef CARRY_SLOT_MEET
-#undef CARRY_SLOT_RESID_BEGIN
-#undef CARRY_SLOT_PUT_RESID4
-#undef CARRY_SLOT_PUT_RESID8
-#undef CARRY_SLOT_PUT_RSCALE_V
-#undef CARRY_SLOT_PUT_RSCALE_HEAD
       } else {
         // ---------------- statequant layout [K][V]: lane = 4 columns x 16 rows ----
         // columns {c0, c0+1} are held as pair A, {c0+2, c0+3} as pair B
