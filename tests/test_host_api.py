@@ -403,3 +403,14 @@ def test_a_library_of_an_older_abi_is_named_as_such(tmp_path, monkeypatch):
     monkeypatch.setattr(_lib, "_lib", None)
     with pytest.raises(_lib.CudaUnavailable, match="ABI mismatch.*version 3.*version 4"):
         _lib.load_library(str(old))
+
+
+def test_the_name_of_the_kernel_sources_is_that_of_their_code():
+    """The benchmark looks the profiled traffic up by it: comments and line breaks do not change it, code does."""
+    import bench
+    code = 'int a = 1;  asm("mov.u32 %0, 0; // kept  as is"); int b;'
+    noted = '// what a is\nint a = 1; /* one\n more */ asm("mov.u32 %0, 0; // kept  as is");\n  int b;  // and b\n'
+    assert bench.code_only(noted) == bench.code_only(code)
+    assert bench.code_only(code.replace("= 1", "= 2")) != bench.code_only(code)
+    assert bench.code_only(code.replace("kept  as", "kept as")) != bench.code_only(code)
+    assert len(bench.kernel_source_hash()) == 16
