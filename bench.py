@@ -378,7 +378,7 @@ def e2e_run(wl, steps, warmup, groups, kernels=True, repeats=1):
 
 
 # ---------------------------------------------------------------------------
-# CPU arm: the oracle port, timed on the host cores; doubles as the checker
+# CPU arm: the oracle port, timed on the host cores; doubles as the parity check
 # ---------------------------------------------------------------------------
 
 def cpu_sample_inputs(batch, layers, resid, seed=1234, resid_scale="head"):

@@ -1,6 +1,6 @@
 """CPU oracle for the fused Gated-DeltaNet decode step on a quantized state.
 
-TEST INFRASTRUCTURE ONLY.  This module is the checker the CUDA kernels are
+TEST INFRASTRUCTURE ONLY.  This module is the oracle the CUDA kernels are
 compared against; the shipped package never imports it.  It restates, with
 plain torch CPU ops, the arithmetic that tomalmog/carrykernel defines for the
 path (paths below are relative to that project):
