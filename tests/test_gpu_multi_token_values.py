@@ -1,6 +1,6 @@
 """Multi-token call against single-token calls, bit for bit, on activations that are zero, far apart in size, not finite or the
-same for 96 tokens (codes settle at rounding ties then, and most tiles have some to decide again): the two kernels split a tile
-differently, and must still take every sum and maximum alike."""
+same for 96 tokens (the state under an int8 residual settles at rounding ties then, which have to be decided again): the two kernels
+split a tile differently, and must still take every sum and maximum alike."""
 
 from __future__ import annotations
 
